@@ -9,21 +9,28 @@
 // Weights: C^-1 transposed times [1, t, t^2, t^3] (the Hermite basis),
 // csrc/gradient_aware_upscaler.cu:137-154.
 //
-// Forward (HBM-bound: 48 B per source pixel + 12 B per output pixel): a CTA
-// owns an 8 x 64 output tile.  It stages the source window of all four planes
-// in shared memory with coalesced row loads, forms for every (output row,
-// source column) the column products F*cy of the reference
-// (csrc/gradient_aware_upscaler.cu:172-175), and finishes each pixel with the
-// four cx products.  The expressions match the reference's, so results match
-// to rounding.  Windows too large for shared memory (down-scaling) fall back to
-// a direct per-pixel gather.
+// Forward (48 B per source pixel + 12 B per output pixel): a thread owns one
+// value (column, channel) of an output row and walks down up to 64 rows.  It
+// reduces each source row along x once (8 values, read through L1; the next
+// row's are on their way meanwhile) and keeps the two rows of the current
+// cell in registers, so an output costs one shared weight vector, four
+// products and one coalesced store, at any scale and without a staged window.
+// x first, then y: the sum of csrc/gradient_aware_upscaler.cu:172-175 in
+// another order.  2048^2 -> 8192^2: 796 us (8x64 tiles staged in shared
+// memory, y first) -> 260; 2047x1535 -> 3070x2302: 221 -> 64.  Bound by
+// instruction issue (75% of the slots) and the rows' load latency.
 //
-// Backward: a gather.  A CTA owns an 8 x 16 block of source texels, finds the
-// output rows/columns whose cell corners touch it (monotone maps -> binary
-// search), stages that patch of the incoming gradient in shared memory, reduces
-// along x then y with the separable weights, and writes each texel's four
-// gradients once.  The reference scatters 48 float atomics per output pixel
-// (csrc/gradient_aware_upscaler.cu:313-370).
+// Backward: a gather.  A thread owns one value of a texel row and walks the
+// output rows that touch its CTA's texel rows: per row it reduces its column's
+// cotangents along x (weights in registers, up to 8 columns loaded together),
+// adds the two sums to the accumulators of the row's two texel rows, and
+// writes a texel row once when the walk passes it.  No atomics, every texel
+// written; the reference scatters 48 float atomics per output pixel
+// (csrc/gradient_aware_upscaler.cu:313-370).  2047x1535 -> 3070x2302: 328 us
+// (8x16 texels per CTA, patch staged in shared memory) -> 89; 512^2 -> 1024^2:
+// 39 -> 12.  Bound by load latency (half the warps resident at 64 registers).
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace lig {
@@ -87,285 +94,295 @@ __device__ __forceinline__ void coord_idx(const UpMap &m, int d, int &i0, int &i
 }
 
 // ---------------------------------------------------------------- forward
-constexpr int kFwdRows = 8, kFwdCols = 64, kFwdThreads = 256;
-constexpr int kFwdMaxSW = kFwdCols + 4;   // staged source columns (scale <= 1 fits)
-constexpr int kFwdMaxSH = kFwdRows + 4;   // staged source rows
+constexpr int kUpThreads = 256;
+constexpr int kFwdMaxRows = 64;  // 2048^2 -> 8192^2: 268 us with 64 rows a CTA, 292 with 32, 266 with 128
+template <typename T> struct alignas(4 * sizeof(T)) W4 { T w[4]; };
 
-template <typename T, int C>
-struct FwdSmem {
-    int x0[kFwdCols], x1[kFwdCols];
-    T cx[kFwdCols][4];
-    int y0[kFwdRows], y1[kFwdRows];
-    T cy[kFwdRows][4];
-    T src[4][kFwdMaxSH][kFwdMaxSW * C];   // f, fx, fy, fxy
-    T vf[kFwdRows][kFwdMaxSW * C];        // F*cy columns 0/1 (value)
-    T vd[kFwdRows][kFwdMaxSW * C];        // F*cy columns 2/3 (x-derivative)
-};
-
-template <typename T, int C>
-__global__ void __launch_bounds__(kFwdThreads)
-upscale_fwd_kernel(UpMap mx, UpMap my, int src_w, const T *__restrict__ f,
+template <typename T, int C, typename Off>
+__global__ void __launch_bounds__(kUpThreads)
+upscale_fwd_kernel(UpMap mx, UpMap my, int src_w, int rows, const T *__restrict__ f,
                    const T *__restrict__ fx, const T *__restrict__ fy,
                    const T *__restrict__ fxy, T *__restrict__ out) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    FwdSmem<T, C> &S = *reinterpret_cast<FwdSmem<T, C> *>(smem_raw);
-    const int dst_w = mx.dst_n, dst_h = my.dst_n;
-    const int c0 = blockIdx.x * kFwdCols, r0 = blockIdx.y * kFwdRows;
-    const int ncol = min(kFwdCols, dst_w - c0), nrow = min(kFwdRows, dst_h - r0);
-    const int tid = threadIdx.x;
-    if (tid < ncol) coord<T>(mx, c0 + tid, S.x0[tid], S.x1[tid], S.cx[tid]);
-    if (tid >= 128 && tid - 128 < nrow) {
-        int r = tid - 128;
-        coord<T>(my, r0 + r, S.y0[r], S.y1[r], S.cy[r]);
+    __shared__ int2 s_y[kFwdMaxRows];
+    __shared__ int s_end[kFwdMaxRows];
+    __shared__ W4<T> s_cy[kFwdMaxRows];
+    const int dst_w = mx.dst_n;
+    const int r0 = blockIdx.y * rows, nrow = min(rows, my.dst_n - r0);
+    if (threadIdx.x < nrow)
+        coord<T>(my, r0 + threadIdx.x, s_y[threadIdx.x].x, s_y[threadIdx.x].y,
+                 s_cy[threadIdx.x].w);
+    const int64_t q = (int64_t)blockIdx.x * kUpThreads + threadIdx.x;
+    const int c = (int)(q / C), ch = (int)(q - (int64_t)c * C);
+    int x0, x1;
+    T cx[4];
+    coord<T>(mx, min(c, dst_w - 1), x0, x1, cx);
+    __syncthreads();
+    if (threadIdx.x < nrow) {  // the output rows of one source cell follow each other
+        const int2 y = s_y[threadIdx.x];
+        int e = threadIdx.x + 1;
+        while (e < nrow && s_y[e].x == y.x && s_y[e].y == y.y) ++e;
+        s_end[threadIdx.x] = e;
     }
     __syncthreads();
-    const int xs_lo = S.x0[0], xs_hi = S.x1[ncol - 1];
-    const int ys_lo = S.y0[0], ys_hi = S.y1[nrow - 1];
-    const int SW = xs_hi - xs_lo + 1, SH = ys_hi - ys_lo + 1;
-    const T *planes[4] = {f, fx, fy, fxy};
-    if (SW >= 1 && SH >= 1 && SW <= kFwdMaxSW && SH <= kFwdMaxSH) {
-        // stage source window (coalesced: one contiguous 3*SW segment per row)
-        const int seg = C * SW;
-        for (int idx = tid; idx < 4 * SH * seg; idx += kFwdThreads) {
-            int p = idx / (SH * seg), rem = idx % (SH * seg);
-            int r = rem / seg, q = rem % seg;
-            S.src[p][r][q] = planes[p][((int64_t)(ys_lo + r) * src_w + xs_lo) * C + q];
+    if (c >= dst_w) return;
+    // byte offsets in a plane: with 32 bits the four planes' loads share one
+    // offset register (uniform base + offset), without 64-bit sums per load
+    const Off pitch = (Off)src_w * (Off)(C * sizeof(T));
+    const Off oa = (Off)(x0 * C + ch) * (Off)sizeof(T), ob = (Off)(x1 * C + ch) * (Off)sizeof(T);
+    auto at = [](const T *p, Off o) {
+        return *reinterpret_cast<const T *>(reinterpret_cast<const char *>(p) + o);
+    };
+    // the eight source values of row y at this output column, and from them
+    // the row's value and y-derivative there
+    auto fetch = [&](int y, T (&t)[8]) {
+        const Off a = (Off)y * pitch + oa, b = (Off)y * pitch + ob;
+        t[0] = at(f, a); t[1] = at(f, b); t[2] = at(fx, a); t[3] = at(fx, b);
+        t[4] = at(fy, a); t[5] = at(fy, b); t[6] = at(fxy, a); t[7] = at(fxy, b);
+    };
+    auto reduce = [&](const T (&t)[8], T &v, T &d) {
+        v = t[0] * cx[0] + t[1] * cx[1] + t[2] * cx[2] + t[3] * cx[3];
+        d = t[4] * cx[0] + t[5] * cx[1] + t[6] * cx[2] + t[7] * cx[3];
+    };
+    int yb = -1;  // source row held in (vb, db)
+    T va, da, vb = 0, db = 0;
+    int yn = s_y[0].x;  // source row on its way in nx
+    T nx[8];
+    fetch(yn, nx);
+    const int y_last = s_y[nrow - 1].y;
+    auto at_row = [&](int y, T &v, T &d) {
+        if (y != yn) fetch(y, nx);
+        reduce(nx, v, d);
+        yn = min(y + 1, y_last);
+        fetch(yn, nx);
+    };
+    const int64_t o_pitch = (int64_t)dst_w * C;
+    T *o = out + r0 * o_pitch + q;
+    for (int r = 0; r < nrow;) {  // cell rows; s_y is the same for every thread
+        const int2 y = s_y[r];
+        if (y.x == yb) {
+            va = vb;
+            da = db;
+        } else {
+            at_row(y.x, va, da);
         }
-        __syncthreads();
-        // column products per (output row, source column): the reference's
-        // Fcy0/Fcy1 (value planes) and Fcy2/Fcy3 (x-derivative planes)
-        for (int idx = tid; idx < nrow * SW; idx += kFwdThreads) {
-            int r = idx / SW, x = idx % SW;
-            int ya = min(max(S.y0[r] - ys_lo, 0), SH - 1);
-            int yb = min(max(S.y1[r] - ys_lo, 0), SH - 1);
-            const T *cy = S.cy[r];
-#pragma unroll
-            for (int ch = 0; ch < C; ++ch) {
-                int q = C * x + ch;
-                S.vf[r][q] = S.src[0][ya][q] * cy[0] + S.src[0][yb][q] * cy[1] +
-                             S.src[2][ya][q] * cy[2] + S.src[2][yb][q] * cy[3];
-                S.vd[r][q] = S.src[1][ya][q] * cy[0] + S.src[1][yb][q] * cy[1] +
-                             S.src[3][ya][q] * cy[2] + S.src[3][yb][q] * cy[3];
-            }
+        if (y.y == y.x) {
+            vb = va;
+            db = da;
+        } else if (y.y != yb) {
+            at_row(y.y, vb, db);
         }
-        __syncthreads();
-        for (int idx = tid; idx < nrow * kFwdCols; idx += kFwdThreads) {
-            int r = idx / kFwdCols, c = idx % kFwdCols;
-            if (c >= ncol) continue;
-            int xa = min(max(S.x0[c] - xs_lo, 0), SW - 1);
-            int xb = min(max(S.x1[c] - xs_lo, 0), SW - 1);
-            const T *cx = S.cx[c];
-            T *o = out + ((int64_t)(r0 + r) * dst_w + c0 + c) * C;
-#pragma unroll
-            for (int ch = 0; ch < C; ++ch)
-                o[ch] = cx[0] * S.vf[r][C * xa + ch] + cx[1] * S.vf[r][C * xb + ch] +
-                        cx[2] * S.vd[r][C * xa + ch] + cx[3] * S.vd[r][C * xb + ch];
-        }
-        return;
-    }
-    // direct gather (large source windows)
-    for (int idx = tid; idx < nrow * kFwdCols; idx += kFwdThreads) {
-        int r = idx / kFwdCols, c = idx % kFwdCols;
-        if (c >= ncol) continue;
-        const T *cx = S.cx[c], *cy = S.cy[r];
-        int64_t i00 = (int64_t)S.y0[r] * src_w + S.x0[c], i01 = (int64_t)S.y0[r] * src_w + S.x1[c];
-        int64_t i10 = (int64_t)S.y1[r] * src_w + S.x0[c], i11 = (int64_t)S.y1[r] * src_w + S.x1[c];
-        T *o = out + ((int64_t)(r0 + r) * dst_w + c0 + c) * C;
-#pragma unroll
-        for (int ch = 0; ch < C; ++ch) {
-            T F0 = f[C * i00 + ch] * cy[0] + f[C * i10 + ch] * cy[1] + fy[C * i00 + ch] * cy[2] + fy[C * i10 + ch] * cy[3];
-            T F1 = f[C * i01 + ch] * cy[0] + f[C * i11 + ch] * cy[1] + fy[C * i01 + ch] * cy[2] + fy[C * i11 + ch] * cy[3];
-            T F2 = fx[C * i00 + ch] * cy[0] + fx[C * i10 + ch] * cy[1] + fxy[C * i00 + ch] * cy[2] + fxy[C * i10 + ch] * cy[3];
-            T F3 = fx[C * i01 + ch] * cy[0] + fx[C * i11 + ch] * cy[1] + fxy[C * i01 + ch] * cy[2] + fxy[C * i11 + ch] * cy[3];
-            o[ch] = cx[0] * F0 + cx[1] * F1 + cx[2] * F2 + cx[3] * F3;
+        yb = y.y;
+        const int end = s_end[r];
+#pragma unroll 4
+        for (; r < end; ++r, o += o_pitch) {
+            const W4<T> cy = s_cy[r];
+            *o = va * cy.w[0] + vb * cy.w[1] + da * cy.w[2] + db * cy.w[3];
         }
     }
 }
 
 // --------------------------------------------------------------- backward
-constexpr int kBwdTexH = 8, kBwdTexW = 16, kBwdThreads = 256;
-constexpr int kBwdMaxDW = 72, kBwdMaxDH = 40;   // staged output patch (scale <= 4 fits)
+constexpr int kBwdRowChunk = 32;  // output rows whose weights are staged at a time
+constexpr int kBwdMaxRows = 32;   // texel rows a CTA walks (32 to 128 measured alike)
 
-template <typename T, int C>
-struct BwdSmem {
-    int i_lo, i_hi, j_lo, j_hi;
-    int x0[kBwdMaxDW], x1[kBwdMaxDW];
-    T cx[kBwdMaxDW][4];
-    int y0[kBwdMaxDH], y1[kBwdMaxDH];
-    T cy[kBwdMaxDH][4];
-    int ia[kBwdTexW], ib[kBwdTexW], ja[kBwdTexH], jb[kBwdTexH];
-    T g[kBwdMaxDH][kBwdMaxDW * C];
-    T uv[kBwdMaxDH][kBwdTexW * C];   // x-reduced with value weights
-    T ud[kBwdMaxDH][kBwdTexW * C];   // x-reduced with derivative weights
+// First output index in [0, dst_n] whose left (RIGHT: right) corner is >= s.
+// The map is monotone: from the inverse map's estimate a few steps find the
+// index; a degenerate map, or an estimate further off, takes the binary search.
+template <typename T, bool RIGHT>
+__device__ __forceinline__ int first_ge(const UpMap &m, int s) {
+    auto ge = [&](int d) {
+        int a, b;
+        coord_idx<T>(m, d, a, b);
+        return (RIGHT ? b : a) >= s;
+    };
+    const int n = m.dst_n;
+    const T x = (T)(RIGHT ? s - 1 : s);
+    const T est = m.mode == 0 ? (x - (T)m.lo + (T)0.5) * (T)n / (T)m.roi_n - (T)0.5
+                              : x * (T)(n - 1) / (T)max(m.src_n - 1, 1);
+    if (m.mode != 0 || m.roi_n > 0) {
+        int d = (int)max((T)0, min(est, (T)n));
+        d = min(d, n);
+#pragma unroll 1
+        for (int k = 0; k < 4; ++k) {
+            if (d < n && !ge(d)) ++d;
+            else if (d > 0 && ge(d - 1)) --d;
+            else return d;
+        }
+    }
+    int lo = 0, hi = n;  // answer in [lo, hi]
+#pragma unroll 1
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (ge(mid)) hi = mid; else lo = mid + 1;
+    }
+    return lo;
+}
+
+// Weights of output index d, with a clamped cell (both corners the same
+// texel) folded into its first corner.
+template <typename T>
+__device__ __forceinline__ void folded(const UpMap &m, int d, int &i0, int &i1, T (&w)[4]) {
+    coord<T>(m, d, i0, i1, w);
+    if (i0 == i1) {
+        w[0] += w[1];
+        w[2] += w[3];
+        w[1] = w[3] = (T)0;
+    }
+}
+
+// One thread's walk over the output rows that touch its CTA's texel rows
+// [sy0, sy1]: per row the x-reduction of its texel column (uv with the value
+// weights, ud with the derivative weights, output columns ascending), added
+// to the accumulators of the row's two texel rows; a texel row is written
+// when the walk passes it.  NT > 0: the column has at most NT output columns,
+// whose weights are kept in registers and whose values are loaded together,
+// two rows at a time (a loop over a weight table that waits for every load
+// took 140 us at 2047x1535 -> 3070x2302, against 89).
+template <typename T>
+struct BwdWalk {
+    const T *g;          // this thread's first output column, output row 0
+    int64_t g_pitch;
+    T *gf, *gfx, *gfy, *gfxy;
+    int64_t o_pitch;     // values of a texel row
+    bool active;
+    int sy0, sy1, cur;   // texel rows of the CTA; acc0 belongs to row cur, acc1 to cur + 1
+    T acc0[4], acc1[4];
+    __device__ __forceinline__ void flush(int64_t q) {
+        if (cur >= sy0 && cur <= sy1 && active) {
+            const int64_t o = cur * o_pitch + q;
+            gf[o] = acc0[0];
+            gfx[o] = acc0[1];
+            gfy[o] = acc0[2];
+            gfxy[o] = acc0[3];
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            acc0[k] = acc1[k];
+            acc1[k] = (T)0;
+        }
+        ++cur;
+    }
+    __device__ __forceinline__ void row(int64_t q, int2 y, const W4<T> &cy, T uv, T ud) {
+        while (cur < y.x) flush(q);  // y is the same for every thread
+        acc0[0] += uv * cy.w[0];
+        acc0[1] += ud * cy.w[0];
+        acc0[2] += uv * cy.w[2];
+        acc0[3] += ud * cy.w[2];
+        if (y.y != y.x) {
+            acc1[0] += uv * cy.w[1];
+            acc1[1] += ud * cy.w[1];
+            acc1[2] += uv * cy.w[3];
+            acc1[3] += ud * cy.w[3];
+        }
+    }
 };
 
-// first index in [0, n) whose map (i0 or i1) satisfies pred, binary search
-template <typename T>
-__device__ int first_x1_ge(const UpMap &m, int s) {
-    int lo = 0, hi = m.dst_n;  // answer in [lo, hi]
-    while (lo < hi) {
-        int mid = (lo + hi) >> 1, a, b;
-        coord_idx<T>(m, mid, a, b);
-        if (b >= s) hi = mid; else lo = mid + 1;
-    }
-    return lo;
-}
-template <typename T>
-__device__ int last_x0_le(const UpMap &m, int s) {
-    int lo = -1, hi = m.dst_n - 1;  // answer in [lo, hi]
-    while (lo < hi) {
-        int mid = (lo + hi + 1) >> 1, a, b;
-        coord_idx<T>(m, mid, a, b);
-        if (a <= s) lo = mid; else hi = mid - 1;
-    }
-    return lo;
-}
-
-template <typename T>
-__device__ __forceinline__ void wx_of(int s, int a, int b, const T *w, T &wv, T &wd) {
-    wv = (a == s ? w[0] : (T)0) + (b == s ? w[1] : (T)0);
-    wd = (a == s ? w[2] : (T)0) + (b == s ? w[3] : (T)0);
-}
-
 template <typename T, int C>
-__global__ void __launch_bounds__(kBwdThreads)
-upscale_bwd_kernel(UpMap mx, UpMap my, int src_w, int src_h, const T *__restrict__ g,
+__global__ void __launch_bounds__(kUpThreads)
+upscale_bwd_kernel(UpMap mx, UpMap my, int src_w, int src_h, int rows, const T *__restrict__ g,
                    T *__restrict__ gf, T *__restrict__ gfx, T *__restrict__ gfy,
                    T *__restrict__ gfxy) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    BwdSmem<T, C> &S = *reinterpret_cast<BwdSmem<T, C> *>(smem_raw);
-    const int dst_w = mx.dst_n;
-    const int sx0 = blockIdx.x * kBwdTexW, sy0 = blockIdx.y * kBwdTexH;
-    const int nsx = min(kBwdTexW, src_w - sx0), nsy = min(kBwdTexH, src_h - sy0);
-    const int tid = threadIdx.x;
-    if (tid == 0) {
-        S.i_lo = first_x1_ge<T>(mx, sx0);
-        S.i_hi = last_x0_le<T>(mx, sx0 + nsx - 1);
-    } else if (tid == 32) {
-        S.j_lo = first_x1_ge<T>(my, sy0);
-        S.j_hi = last_x0_le<T>(my, sy0 + nsy - 1);
-    }
+    __shared__ int s_rng[4];
+    __shared__ int2 s_y[kBwdRowChunk];
+    __shared__ W4<T> s_cy[kBwdRowChunk];
+    const int tid = threadIdx.x, dst_w = mx.dst_n;
+    const int64_t q = (int64_t)blockIdx.x * kUpThreads + tid;
+    const int sy0 = blockIdx.y * rows, sy1 = min(sy0 + rows, src_h) - 1;
+    if (tid == 0) s_rng[0] = first_ge<T, true>(my, sy0);
+    else if (tid == 32) s_rng[1] = first_ge<T, false>(my, sy1 + 1) - 1;
+    // this thread's texel column x: output columns [ia, im) have it as their
+    // right corner, [im, ib) as their left one
+    const int x = (int)min(q / C, (int64_t)src_w - 1), ch = (int)(q % C);
+    const int ia = first_ge<T, true>(mx, x), im = first_ge<T, false>(mx, x),
+              ib = first_ge<T, false>(mx, x + 1);
+    const int n = ib - ia;
     __syncthreads();
-    const int i_lo = S.i_lo, i_hi = S.i_hi, j_lo = S.j_lo, j_hi = S.j_hi;
-    const int DW = i_hi - i_lo + 1, DH = j_hi - j_lo + 1;
-    const bool staged = DW <= kBwdMaxDW && DH <= kBwdMaxDH;
-    if (DW <= 0 || DH <= 0) {
-        for (int idx = tid; idx < nsy * nsx * C; idx += kBwdThreads) {
-            int r = idx / (nsx * C), q = idx % (nsx * C);
-            int64_t o = ((int64_t)(sy0 + r) * src_w + sx0) * C + q;
-            gf[o] = 0; gfx[o] = 0; gfy[o] = 0; gfxy[o] = 0;
-        }
-        return;
-    }
-    if (staged) {
-        for (int i = tid; i < DW; i += kBwdThreads) coord<T>(mx, i_lo + i, S.x0[i], S.x1[i], S.cx[i]);
-        for (int j = tid; j < DH; j += kBwdThreads) coord<T>(my, j_lo + j, S.y0[j], S.y1[j], S.cy[j]);
-        const int seg = C * DW;
-        for (int idx = tid; idx < DH * seg; idx += kBwdThreads) {
-            int r = idx / seg, q = idx % seg;
-            S.g[r][q] = g[((int64_t)(j_lo + r) * dst_w + i_lo) * C + q];
-        }
-        __syncthreads();
-        // candidate output ranges per source column / row (monotone maps)
-        if (tid < nsx) {
-            int s = sx0 + tid, a = DW, b = -1;
-            for (int i = 0; i < DW; ++i)
-                if (S.x0[i] == s || S.x1[i] == s) { a = min(a, i); b = max(b, i); }
-            S.ia[tid] = a; S.ib[tid] = b;
-        } else if (tid >= 64 && tid - 64 < nsy) {
-            int r = tid - 64, s = sy0 + r, a = DH, b = -1;
-            for (int j = 0; j < DH; ++j)
-                if (S.y0[j] == s || S.y1[j] == s) { a = min(a, j); b = max(b, j); }
-            S.ja[r] = a; S.jb[r] = b;
-        }
-        __syncthreads();
-        // x-reduction: for each staged output row and source column
-        for (int idx = tid; idx < DH * nsx; idx += kBwdThreads) {
-            int r = idx / nsx, sc = idx % nsx, s = sx0 + sc;
-            T av[C] = {}, ad[C] = {};
-            for (int i = S.ia[sc]; i <= S.ib[sc]; ++i) {
-                T wv, wd;
-                wx_of<T>(s, S.x0[i], S.x1[i], S.cx[i], wv, wd);
+    const int j_lo = s_rng[0], j_hi = s_rng[1];
+    BwdWalk<T> B{g + (int64_t)ia * C + ch, (int64_t)dst_w * C, gf, gfx, gfy, gfxy,
+                 (int64_t)src_w * C, q < (int64_t)src_w * C, sy0, sy1, sy0 - 1, {}, {}};
+    auto weights = [&](int i, T &wv, T &wd) {  // of output column ia + i
+        int x0, x1;
+        T w[4];
+        folded<T>(mx, ia + i, x0, x1, w);
+        wv = ia + i < im ? w[1] : w[0];
+        wd = ia + i < im ? w[3] : w[2];
+    };
+    // FULL: every texel column of the CTA has exactly NT output columns
+    auto walk = [&](auto nt_tag, auto full_tag) {
+        constexpr int NT = decltype(nt_tag)::value;
+        [[maybe_unused]] constexpr bool FULL = decltype(full_tag)::value;
+        T wv[NT > 0 ? NT : 1], wd[NT > 0 ? NT : 1];
+        if constexpr (NT > 0) {
 #pragma unroll
-                for (int ch = 0; ch < C; ++ch) {
-                    T gv = S.g[r][C * i + ch];
-                    av[ch] += gv * wv;
-                    ad[ch] += gv * wd;
+            for (int k = 0; k < NT; ++k) {
+                wv[k] = wd[k] = (T)0;
+                if (k < n) weights(k, wv[k], wd[k]);
+            }
+        }
+        for (int jb = j_lo; jb <= j_hi; jb += kBwdRowChunk) {
+            const int nj = min(kBwdRowChunk, j_hi - jb + 1);
+            __syncthreads();
+            if (tid < nj) folded<T>(my, jb + tid, s_y[tid].x, s_y[tid].y, s_cy[tid].w);
+            __syncthreads();
+            const T *gp = B.g + jb * B.g_pitch;
+            if constexpr (NT > 0) {
+                for (int j = 0; j < nj; j += 2, gp += 2 * B.g_pitch) {
+                    const bool two = j + 1 < nj;
+                    T v[2][NT];
+#pragma unroll
+                    for (int k = 0; k < NT; ++k) {
+                        v[0][k] = FULL || k < n ? gp[k * C] : (T)0;
+                        v[1][k] = (FULL || k < n) && two ? gp[B.g_pitch + k * C] : (T)0;
+                    }
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        if (h == 1 && !two) break;
+                        T uv = 0, ud = 0;
+#pragma unroll
+                        for (int k = 0; k < NT; ++k) {
+                            uv += v[h][k] * wv[k];
+                            ud += v[h][k] * wd[k];
+                        }
+                        B.row(q, s_y[j + h], s_cy[j + h], uv, ud);
+                    }
                 }
-            }
-#pragma unroll
-            for (int ch = 0; ch < C; ++ch) {
-                S.uv[r][C * sc + ch] = av[ch];
-                S.ud[r][C * sc + ch] = ad[ch];
-            }
-        }
-        __syncthreads();
-        // y-reduction and write-out
-        for (int idx = tid; idx < nsy * nsx; idx += kBwdThreads) {
-            int rr = idx / nsx, sc = idx % nsx, s = sy0 + rr;
-            T a0[C] = {}, a1[C] = {}, a2[C] = {}, a3[C] = {};
-            for (int j = S.ja[rr]; j <= S.jb[rr]; ++j) {
-                T wv, wd;
-                wx_of<T>(s, S.y0[j], S.y1[j], S.cy[j], wv, wd);
-#pragma unroll
-                for (int ch = 0; ch < C; ++ch) {
-                    T uv = S.uv[j][C * sc + ch], ud = S.ud[j][C * sc + ch];
-                    a0[ch] += uv * wv;   // value plane
-                    a1[ch] += ud * wv;   // x-derivative plane
-                    a2[ch] += uv * wd;   // y-derivative plane
-                    a3[ch] += ud * wd;   // mixed plane
-                }
-            }
-            int64_t o = ((int64_t)s * src_w + sx0 + sc) * C;
-#pragma unroll
-            for (int ch = 0; ch < C; ++ch) {
-                gf[o + ch] = a0[ch]; gfx[o + ch] = a1[ch]; gfy[o + ch] = a2[ch]; gfxy[o + ch] = a3[ch];
-            }
-        }
-        return;
-    }
-    // large patches (strong down-scaling): per texel, straight from global memory
-    for (int idx = tid; idx < nsy * nsx; idx += kBwdThreads) {
-        int rr = idx / nsx, sc = idx % nsx, sy = sy0 + rr, sx = sx0 + sc;
-        T a0[C] = {}, a1[C] = {}, a2[C] = {}, a3[C] = {};
-        int jl = first_x1_ge<T>(my, sy), jh = last_x0_le<T>(my, sy);
-        int il = first_x1_ge<T>(mx, sx), ih = last_x0_le<T>(mx, sx);
-        for (int j = jl; j <= jh; ++j) {
-            int ya, yb;
-            T cy[4];
-            coord<T>(my, j, ya, yb, cy);
-            T yv, yd;
-            wx_of<T>(sy, ya, yb, cy, yv, yd);
-            if (yv == (T)0 && yd == (T)0) continue;
-            for (int i = il; i <= ih; ++i) {
-                int xa, xb;
-                T cx[4];
-                coord<T>(mx, i, xa, xb, cx);
-                T xv, xd;
-                wx_of<T>(sx, xa, xb, cx, xv, xd);
-                const T *gp = g + ((int64_t)j * dst_w + i) * C;
-#pragma unroll
-                for (int ch = 0; ch < C; ++ch) {
-                    T gv = gp[ch];
-                    a0[ch] += gv * xv * yv;
-                    a1[ch] += gv * xd * yv;
-                    a2[ch] += gv * xv * yd;
-                    a3[ch] += gv * xd * yd;
+            } else {
+                for (int j = 0; j < nj; ++j, gp += B.g_pitch) {
+                    T uv = 0, ud = 0;
+                    for (int i = 0; i < n; ++i) {
+                        T a, b;
+                        weights(i, a, b);
+                        const T gv = gp[(int64_t)i * C];
+                        uv += gv * a;
+                        ud += gv * b;
+                    }
+                    B.row(q, s_y[j], s_cy[j], uv, ud);
                 }
             }
         }
-        int64_t o = ((int64_t)sy * src_w + sx) * C;
-#pragma unroll
-        for (int ch = 0; ch < C; ++ch) {
-            gf[o + ch] = a0[ch]; gfx[o + ch] = a1[ch]; gfy[o + ch] = a2[ch]; gfxy[o + ch] = a3[ch];
-        }
+        while (B.cur <= sy1) B.flush(q);
+    };
+    // the most output columns of a texel column in this CTA
+    using std::false_type;
+    using std::true_type;
+    if (__syncthreads_and(n <= 4)) {
+        if (__syncthreads_and(n == 4)) walk(std::integral_constant<int, 4>{}, true_type{});
+        else walk(std::integral_constant<int, 4>{}, false_type{});
+    } else if (__syncthreads_and(n <= 8)) {
+        if (__syncthreads_and(n == 8)) walk(std::integral_constant<int, 8>{}, true_type{});
+        else walk(std::integral_constant<int, 8>{}, false_type{});
+    } else {
+        walk(std::integral_constant<int, 0>{}, false_type{});
     }
 }
 
-inline bool set_smem(const void *fn, size_t bytes) {
-    if (bytes <= 48 * 1024) return true;
-    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) ==
-           cudaSuccess;
+// Output (forward) or texel (backward) rows a CTA walks: the most, up to
+// `most`, that leave at least 16 CTAs per SM.
+inline int up_rows(int64_t row_values, int n_rows, int most) {
+    const int64_t cols = (row_values + kUpThreads - 1) / kUpThreads;
+    int r = most;
+    while (r > 8 && cols * ((n_rows + r - 1) / r) < 148 * 16) r >>= 1;
+    return r;
 }
 
 template <typename T, int C>
@@ -375,11 +392,13 @@ int upscale_fwd(int mode, int src_h, int src_w, int dst_h, int dst_w, double x1,
     // the reference truncates the ROI extent to int (csrc/gradient_aware_upscaler.cu:201-202)
     UpMap mx{mode, dst_w, src_w, (int)((T)x2 - (T)x1), (double)(T)x1};
     UpMap my{mode, dst_h, src_h, (int)((T)y2 - (T)y1), (double)(T)y1};
-    size_t sm = sizeof(FwdSmem<T, C>);
-    if (!set_smem((const void *)upscale_fwd_kernel<T, C>, sm)) return LIG_ERR_LAUNCH;
-    dim3 grid((dst_w + kFwdCols - 1) / kFwdCols, (dst_h + kFwdRows - 1) / kFwdRows);
-    upscale_fwd_kernel<T, C><<<grid, kFwdThreads, sm, s>>>(mx, my, src_w, (const T *)f, (const T *)fx,
-                                                       (const T *)fy, (const T *)fxy, (T *)out);
+    const int64_t row = (int64_t)dst_w * C;
+    const int rows = up_rows(row, dst_h, kFwdMaxRows);
+    const dim3 grid((unsigned)((row + kUpThreads - 1) / kUpThreads), (dst_h + rows - 1) / rows);
+    const bool small = (int64_t)src_h * src_w * C * (int64_t)sizeof(T) <= 0xffffffffll;
+    auto k = small ? upscale_fwd_kernel<T, C, uint32_t> : upscale_fwd_kernel<T, C, uint64_t>;
+    k<<<grid, kUpThreads, 0, s>>>(mx, my, src_w, rows, (const T *)f, (const T *)fx, (const T *)fy,
+                                  (const T *)fxy, (T *)out);
     note_launches(1);
     LIG_LAUNCH_CHECK();
     return LIG_OK;
@@ -391,11 +410,12 @@ int upscale_bwd(int mode, int src_h, int src_w, int dst_h, int dst_w, double x1,
                 cudaStream_t s) {
     UpMap mx{mode, dst_w, src_w, (int)((T)x2 - (T)x1), (double)(T)x1};
     UpMap my{mode, dst_h, src_h, (int)((T)y2 - (T)y1), (double)(T)y1};
-    size_t sm = sizeof(BwdSmem<T, C>);
-    if (!set_smem((const void *)upscale_bwd_kernel<T, C>, sm)) return LIG_ERR_LAUNCH;
-    dim3 grid((src_w + kBwdTexW - 1) / kBwdTexW, (src_h + kBwdTexH - 1) / kBwdTexH);
-    upscale_bwd_kernel<T, C><<<grid, kBwdThreads, sm, s>>>(mx, my, src_w, src_h, (const T *)g,
-                                                       (T *)gf, (T *)gfx, (T *)gfy, (T *)gfxy);
+    const int64_t row = (int64_t)src_w * C;
+    const int rows = up_rows(row, src_h, kBwdMaxRows);
+    const dim3 grid((unsigned)((row + kUpThreads - 1) / kUpThreads), (src_h + rows - 1) / rows);
+    upscale_bwd_kernel<T, C><<<grid, kUpThreads, 0, s>>>(mx, my, src_w, src_h, rows,
+                                                         (const T *)g, (T *)gf, (T *)gfx,
+                                                         (T *)gfy, (T *)gfxy);
     note_launches(1);
     LIG_LAUNCH_CHECK();
     return LIG_OK;
