@@ -107,12 +107,20 @@ __device__ uint32_t g_alpha_cut;
 // forward, see sigma_half); the cull data are computed from the full conic.
 // zero (backward): also clears the Gaussian's zero_stride accumulators there
 // (zero_stride * sizeof(T) a multiple of 16 bytes, 16-byte aligned).
-// HALF (float): block 0's first warp also publishes the alpha cut.
-template <typename T, bool HALF>
+// HALF or TAME (float): block 0's first warp also publishes the alpha cut.
+// TAME (the packed gradient-aware kernels, which add a zero where a pixel
+// fails the alpha test instead of skipping it): culling data only for records
+// whose products at any pixel they are evaluated on stay finite (see
+// kTameSlope, kTameColor), so that the zero weight yields a zero; the others
+// take the kernels' skipping walk.
+constexpr float kTameSlope = 1e6f;  // largest conic entry times the reach: |sx|, |sy| < 2e6
+constexpr float kTameColor = 1e8f;
+
+template <typename T, bool HALF, bool TAME = false>
 __global__ void pack_kernel(int n, const T *__restrict__ xys, const T *__restrict__ conics,
                             const T *__restrict__ colors, const T *__restrict__ opac,
                             Rec<T> *__restrict__ recs, T *__restrict__ zero, int zero_stride) {
-    if (HALF && sizeof(T) == 4 && blockIdx.x == 0 && threadIdx.x < 32) {
+    if ((HALF || TAME) && sizeof(T) == 4 && blockIdx.x == 0 && threadIdx.x < 32) {
         const uint32_t cut = alpha_cut_search();
         if (threadIdx.x == 0) g_alpha_cut = cut;
     }
@@ -146,8 +154,10 @@ __global__ void pack_kernel(int n, const T *__restrict__ xys, const T *__restric
         double sxx = c / det, syy = a / det;
         double hx = 1.001 * sqrt(tc * sxx) + 2.0, hy = 1.001 * sqrt(tc * syy) + 2.0;
         const float reach = (float)fmax(hx, hy) + 16.f;
-        if (hx < 1e7 && hy < 1e7 &&
-            fmaxf(fmaxf((float)r.a, (float)r.c), fabsf((float)r.b)) * reach * reach < 1e36f) {
+        const float entry = fmaxf(fmaxf((float)r.a, (float)r.c), fabsf((float)r.b));
+        const bool tame = !TAME || (entry * reach < kTameSlope && (float)fabs(r.r) < kTameColor &&
+                                    (float)fabs(r.g) < kTameColor && (float)fabs(r.bl) < kTameColor);
+        if (hx < 1e7 && hy < 1e7 && entry * reach * reach < 1e36f && tame) {
             wx = (T)hx;
             wy = (T)hy;
             r.thr = (T)(0.5 * tc * 1.001 + 0.02);
@@ -824,6 +834,28 @@ __device__ __forceinline__ void fwd_tile(const TileCtx &tc, int tile, const int3
 #define LIG_RASTER_PPL4_MIN_TILES 4096  // measured: faster from 2048^2 up, not at 512^2
 #endif
 
+// Resident CTAs per SM asked of the register allocator.  Forward (128 threads),
+// 2048^2 / 1M and 512^2 / 50k: 8 CTAs (64 registers) 973 / 41 us, 9 968 / 43,
+// 7 990 / 40, 6 1110 / 47, 10 1110 / 49.  Backward (256 threads), 2047x1535 /
+// 190k and 512^2 / 50k with opacities: 3 CTAs 518 / 67 us, 2 552 / 64.
+#ifndef LIG_RASTER_GA_MINB
+#define LIG_RASTER_GA_MINB 8
+#endif
+#ifndef LIG_RASTER_GA_BWD_MINB
+#define LIG_RASTER_GA_BWD_MINB 3
+#endif
+// Lanes per Gaussian as in the lean walk; two lanes from 32 left on measured
+// 586 against 552 us, 20 / 12 / 6 left 558 (2047x1535).
+#ifndef LIG_RASTER_GA_BWD_SPLIT1
+#define LIG_RASTER_GA_BWD_SPLIT1 24
+#endif
+#ifndef LIG_RASTER_GA_BWD_SPLIT2
+#define LIG_RASTER_GA_BWD_SPLIT2 8
+#endif
+#ifndef LIG_RASTER_GA_BWD_SPLIT3
+#define LIG_RASTER_GA_BWD_SPLIT3 4
+#endif
+
 template <typename T, bool GA, int PPL, int MAXT, int MINB, bool FL = false, bool FIN = true>
 __global__ void __launch_bounds__(MAXT, MINB)
 raster_fwd_kernel(const BatchGeo geo, const int32_t *__restrict__ cum, int *work,
@@ -843,6 +875,190 @@ raster_fwd_kernel(const BatchGeo geo, const int32_t *__restrict__ cum, int *work
         const TileCtx tc = tile_ctx(geo, cum, d_total, tile);
         fwd_tile<T, GA, PPL, FL, FIN>(tc, tile, ids, tile_bins, recs, img, wsum, odx, ody, odxy,
                                       final_idx, s_rec, s_bits, l2, cut);
+    }
+}
+
+// Gradient-aware forward, float: 8x8 regions, the lane's two pixels (x, y) and
+// (x, y + 4) evaluated as a pair with f32x2 operations.  Per pixel the alphas,
+// their order and the colour sums are fwd_tile's (sigma_half's rounding, the
+// same alpha test, the cut's compare without opacities); a pixel that fails
+// the test adds zeros, so the walk has no branches.  A chunk with a record
+// that could make those zeros NaN (no culling data under TAME packing) takes a
+// scalar walk that skips failing pixels.
+// Bound by the math pipes and issue together (70% of the issue slots; a packed
+// operation takes two cycles of the FMA pipe, so packing saves issue slots
+// only).  2048^2 / 1M Gaussians: 973 us, against 1265 with one pixel a lane in
+// 8x4 regions (scalar, skipping); 8x16 regions with two pairs a lane: 1120 (fewer operations a
+// pixel, more pixels out of reach).
+struct GaAcc {
+    // colour, wsum; sums of c alpha sx, c alpha sy (negated when written) and
+    // c alpha (sx sy - b)
+    f2 c[3], w, x[3], y[3], xy[3];
+    int cur[2];
+};
+
+__device__ __forceinline__ f2 f2_add_half(f2 v, int h, float x) {
+    float lo, hi;
+    f2_unpack(v, lo, hi);
+    return h ? f2_pack(lo, hi + x) : f2_pack(lo + x, hi);
+}
+
+template <bool OP>
+__device__ __forceinline__ void ga_walk(uint32_t mask, const Rec<float> *rb, int ib, float px,
+                                        f2 py, uint32_t cut, GaAcc &A) {
+    const f2 HALF = f2_dup(0.5f);
+    while (mask) {
+        const int bit = __ffs(mask) - 1;
+        mask &= mask - 1;
+        const Rec<float> &g = rb[bit];
+        const float4 q0 = *reinterpret_cast<const float4 *>(&g.x);
+        const float4 q1 = *reinterpret_cast<const float4 *>(&g.c);
+        // sigma and the slopes' products are even in d, so d = pixel - mean
+        // gives fwd_tile's values
+        const f2 DX = f2_dup(px - q0.x), DY = f2_add(py, f2_dup(-q0.y));
+        const f2 B = f2_dup(q0.w), C = f2_dup(q1.x);
+        const f2 AX = f2_mul(f2_dup(q0.z), DX), BX = f2_mul(B, DX);
+        const f2 S = f2_fma(BX, DY, f2_fma(f2_mul(HALF, AX), DX,
+                                           f2_mul(f2_mul(f2_mul(HALF, C), DY), DY)));
+        float s0, s1;
+        f2_unpack(S, s0, s1);
+        float e0 = __expf(-s0), e1 = __expf(-s1);
+        if constexpr (OP) {
+            const float o = g.o;
+            e0 *= o;
+            e1 *= o;
+        }
+        float a0 = fminf(0.999f, e0), a1 = fminf(0.999f, e1);
+        bool no0, no1;
+        if constexpr (!OP && LIG_RASTER_ALPHA_CUT) {
+            no0 = __float_as_uint(s0) >= cut;
+            no1 = __float_as_uint(s1) >= cut;
+        } else {
+            no0 = s0 < 0.f || a0 < 1.f / 255.f;
+            no1 = s1 < 0.f || a1 < 1.f / 255.f;
+        }
+        const f2 AL = f2_pack(no0 ? 0.f : a0, no1 ? 0.f : a1);
+        A.cur[0] = no0 ? A.cur[0] : ib + bit;
+        A.cur[1] = no1 ? A.cur[1] : ib + bit;
+        const f2 SX = f2_fma(B, DY, AX), SY = f2_fma(C, DY, BX);
+        const f2 WX = f2_mul(AL, SX), WY = f2_mul(AL, SY);
+        const f2 WP = f2_mul(AL, f2_fma(SX, SY, f2_dup(-q0.w)));
+        const f2 col[3] = {f2_dup(q1.y), f2_dup(q1.z), f2_dup(q1.w)};
+        A.w = f2_add(A.w, AL);
+#pragma unroll
+        for (int ch = 0; ch < 3; ++ch) {
+            A.c[ch] = f2_fma(col[ch], AL, A.c[ch]);
+            A.x[ch] = f2_fma(col[ch], WX, A.x[ch]);
+            A.y[ch] = f2_fma(col[ch], WY, A.y[ch]);
+            A.xy[ch] = f2_fma(col[ch], WP, A.xy[ch]);
+        }
+    }
+}
+
+// The same chunk pixel by pixel, skipping what fails the alpha test.
+__device__ __noinline__ void ga_walk_skip(uint32_t mask, const Rec<float> *rb, int ib, float px,
+                                          float py0, GaAcc &A) {
+    while (mask) {
+        const int bit = __ffs(mask) - 1;
+        mask &= mask - 1;
+        const Rec<float> g = rb[bit];
+        for (int h = 0; h < 2; ++h) {
+            float dx, dy, a;
+            if (!PixelEval<float>::template alpha<true>(g, px, py0 + (float)(4 * h), dx, dy, a))
+                continue;
+            const float sx = g.a * dx + g.b * dy, sy = g.b * dx + g.c * dy;
+            const float wx = a * sx, wy = a * sy, wp = a * (sx * sy - g.b);
+            const float c[3] = {g.r, g.g, g.bl};
+#pragma unroll
+            for (int ch = 0; ch < 3; ++ch) {
+                A.c[ch] = f2_add_half(A.c[ch], h, c[ch] * a);
+                A.x[ch] = f2_add_half(A.x[ch], h, c[ch] * wx);
+                A.y[ch] = f2_add_half(A.y[ch], h, c[ch] * wy);
+                A.xy[ch] = f2_add_half(A.xy[ch], h, c[ch] * wp);
+            }
+            A.w = f2_add_half(A.w, h, a);
+            A.cur[h] = ib + bit;
+        }
+    }
+}
+
+template <bool OP, int MAXT, int MINB>
+__global__ void __launch_bounds__(MAXT, MINB)
+raster_fwd_ga_kernel(const BatchGeo geo, const int32_t *__restrict__ cum, int *work,
+                     const int32_t *__restrict__ ids, const int2 *__restrict__ tile_bins,
+                     const int32_t *__restrict__ d_total, const Rec<float> *__restrict__ recs,
+                     float *__restrict__ img, float *__restrict__ wsum, float *__restrict__ odx,
+                     float *__restrict__ ody, float *__restrict__ odxy,
+                     int32_t *__restrict__ final_idx) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ int s_slot;
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    Rec<float> *w_rec = reinterpret_cast<Rec<float> *>(smem_raw) + w * 32;
+    const int n_tiles = geo.total_tiles();
+    const uint32_t cut = OP ? 0u : g_alpha_cut;
+    for (int tile = next_tile(work, s_slot, true); tile < n_tiles;
+         tile = next_tile(work, s_slot, false)) {
+        const TileCtx tc = tile_ctx(geo, cum, d_total, tile);
+        const Regions R = Regions::make(1, tc.B);
+        int lx, ly;
+        R.pixel(w, lane, 0, lx, ly);
+        const int gx = tc.tx0 + lx, gy = tc.ty0 + ly;
+        const float px = (float)gx + 0.5f, py = (float)gy + 0.5f;
+        const f2 py2 = f2_pack(py, (float)(gy + 4) + 0.5f);
+        GaAcc A;
+        A.w = f2_zero();
+        A.cur[0] = A.cur[1] = 0;
+#pragma unroll
+        for (int ch = 0; ch < 3; ++ch) A.c[ch] = A.x[ch] = A.y[ch] = A.xy[ch] = f2_zero();
+        if (!tc.empty) {
+            const int2 range = tile_bins[tile];
+            Rec<float> pre;
+            if (range.x + lane < range.y) pre = recs[__ldg(ids + range.x + lane)];
+            for (int base = range.x; base < range.y; base += 32) {
+                const bool mine = base + lane < range.y;
+                const bool hit = mine && region_hit<float, true, false>(pre, R, w, tc.tx0, tc.ty0);
+                const bool fast = !__any_sync(FULL, mine && !(pre.wx >= 0.f));
+                __syncwarp();
+                w_rec[lane] = pre;
+                __syncwarp();
+                if (base + 32 + lane < range.y) pre = recs[__ldg(ids + base + 32 + lane)];
+                const uint32_t mask = __ballot_sync(FULL, hit);
+                if (fast) {
+                    ga_walk<OP>(mask, w_rec, base, px, py2, cut, A);
+                } else {  // through a copy, so that A itself stays in registers
+                    GaAcc t = A;
+                    ga_walk_skip(mask, w_rec, base, px, py, t);
+                    A = t;
+                }
+            }
+        } else {  // the reference's empty-list branch (rasterize.py:80-90)
+#pragma unroll
+            for (int ch = 0; ch < 3; ++ch) A.c[ch] = f2_dup(1.f);
+        }
+        float v[2][13];
+        f2_unpack(A.w, v[0][12], v[1][12]);
+#pragma unroll
+        for (int ch = 0; ch < 3; ++ch) {
+            f2_unpack(A.c[ch], v[0][ch], v[1][ch]);
+            f2_unpack(A.x[ch], v[0][3 + ch], v[1][3 + ch]);
+            f2_unpack(A.y[ch], v[0][6 + ch], v[1][6 + ch]);
+            f2_unpack(A.xy[ch], v[0][9 + ch], v[1][9 + ch]);
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            if (!(lx < tc.B && ly + 4 * h < tc.B && gx < tc.W && gy + 4 * h < tc.H)) continue;
+            const int pix = tc.poff + (gy + 4 * h) * tc.W + gx;
+            final_idx[pix] = A.cur[h];
+            wsum[pix] = v[h][12];
+#pragma unroll
+            for (int ch = 0; ch < 3; ++ch) {
+                img[3 * pix + ch] = v[h][ch];
+                odx[3 * pix + ch] = 0.f - v[h][3 + ch];
+                ody[3 * pix + ch] = 0.f - v[h][6 + ch];
+                odxy[3 * pix + ch] = v[h][9 + ch];
+            }
+        }
     }
 }
 
@@ -1655,6 +1871,330 @@ raster_bwd_kernel(const BatchGeo geo, const int32_t *__restrict__ cum, int *work
     }
 }
 
+// ------------------------------------------------ gradient-aware backward
+// Float, tiles of 16x16 (regions of 16x2 pixels) and 8x8 (8x4): the
+// reference's warps, whose |sum| makes v_xy_abs.  As in the lean walk a lane
+// takes one Gaussian (or 2 / 4 / 8 lanes share one) and loops over its
+// region's pixels; columns c and c + W/2 of a row are evaluated as a pair in
+// f32x2 arithmetic, and a pixel that fails the alpha test adds zeros.
+//
+// With d = pixel - mean, (sx, sy) = conic d, the four planes' cotangents
+// V = (v, -v_dx, -v_dy, v_dxy) and, per colour channel,
+//   E = V0 + V1 sx + V2 sy + V3 (sx sy - b),
+// a pixel's term of the loss is alpha G, G = colour . E (+ v_wsum), so
+//   v_colour = sum alpha E,
+// and with gx = dG/dsx = V1.colour + V3.colour sy, gy likewise, the
+// gradients of csrc/gradient_aware_rasterizer.cu:201-315 are linear in
+//   S_ij = sum alpha G dx^i dy^j (i + j = 1, 2),  A = sum alpha gx,
+//   B = sum alpha gy, A_x = sum alpha gx dx (A_y, B_x, B_y), D = sum alpha V3.colour:
+//   v_xy    = conic (S10 - A, S01 - B)
+//   v_conic = (A_x - S20/2, A_y + B_x - S11 - D, B_y - S02/2),
+// applied once per Gaussian and region: 44 multiply-adds a pixel instead of
+// the expanded formulas' 110.  dy is constant along a row, so the sums with dy
+// come from row sums.
+// Entries after a pixel's final index are not cut off: they fail the alpha
+// test here exactly as they did in the forward.
+// Bound by the FMA pipe (a packed operation takes two cycles of it; 70% busy at
+// 61% of the issue slots).  2047x1535 / 190k Gaussians: 518 us, against 1171
+// for the scalar walk over the expanded formulas; 512^2 / 50k with opacities:
+// 67 against 131.
+constexpr float kTameCot = 1e12f;  // larger (or non-finite) cotangents: the skipping walk
+
+struct alignas(16) GaPix {  // pixels (row, c) and (row, c + W/2)
+    float v[12][2];         // plane-major: V0.rgb, V1.rgb, V2.rgb, V3.rgb
+    float vw[2];
+    float in[2];            // 1: inside the image (read by the skipping walk only)
+};
+
+// Pairs c0, c0 + CSTEP, ... (NCP of them) in two rows of a region (pix: the
+// first row's entries, HW the entries per row), added to acc as [0, 1] v_xy, [4..6]
+// v_conic, [7..9] v_rgb, [10] v_opacity.
+template <int NCP, int CSTEP, int HW, bool OP, bool VW>
+__device__ __forceinline__ void ga_rows(const Rec<float> &g, float clamp,
+                                        const GaPix *__restrict__ pix, int c0, float px0,
+                                        float py0, float (&acc)[11]) {
+    const f2 AA = f2_dup(g.a), BB = f2_dup(g.b), CC = f2_dup(g.c), NB = f2_dup(-g.b);
+    const f2 HALF = f2_dup(0.5f);
+    const f2 CR = f2_dup(g.r), CG = f2_dup(g.g), CB = f2_dup(g.bl);
+    const float hc = 0.5f * g.c;
+    f2 wr[2], wx[2], wxx = f2_zero(), ar[2], br[2], ax = f2_zero(), bx = f2_zero();
+    f2 dd = f2_zero(), cr = f2_zero(), cg = f2_zero(), cb = f2_zero();
+    [[maybe_unused]] f2 vo = f2_zero();
+    f2 DY[2], CDD[2];
+    float dy[2];
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        wr[r] = wx[r] = ar[r] = br[r] = f2_zero();
+        dy[r] = (py0 + (float)r) - g.y;
+        DY[r] = f2_dup(dy[r]);
+        CDD[r] = f2_dup(__fmul_rn(__fmul_rn(hc, dy[r]), dy[r]));
+    }
+#pragma unroll
+    for (int k = 0; k < NCP; ++k) {
+        const int c = c0 + k * CSTEP;
+        const f2 DX = f2_pack((px0 + (float)c) - g.x, (px0 + (float)(c + HW)) - g.x);
+        const f2 AX = f2_mul(AA, DX), BX = f2_mul(BB, DX), HADX = f2_mul(HALF, AX);
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const GaPix &e = pix[r * HW + c];
+            const f2 S = f2_fma(BX, DY[r], f2_fma(HADX, DX, CDD[r]));
+            float s0, s1;
+            f2_unpack(S, s0, s1);
+            const float vis0 = __expf(-s0), vis1 = __expf(-s1);
+            const float al0 = fminf(clamp, OP ? g.o * vis0 : vis0);
+            const float al1 = fminf(clamp, OP ? g.o * vis1 : vis1);
+            const bool no0 = s0 < 0.f || al0 < 1.f / 255.f, no1 = s1 < 0.f || al1 < 1.f / 255.f;
+            const f2 AL = f2_pack(no0 ? 0.f : al0, no1 ? 0.f : al1);
+            const f2 SX = f2_fma(BB, DY[r], AX), SY = f2_fma(CC, DY[r], BX);
+            const f2 P = f2_fma(SX, SY, NB);
+            f2 V[12];
+#pragma unroll
+            for (int q = 0; q < 6; ++q) {
+                const ulonglong2 t = *reinterpret_cast<const ulonglong2 *>(e.v[2 * q]);
+                V[2 * q] = f2{t.x};
+                V[2 * q + 1] = f2{t.y};
+            }
+            const f2 ER = f2_fma(V[9], P, f2_fma(V[6], SY, f2_fma(V[3], SX, V[0])));
+            const f2 EG = f2_fma(V[10], P, f2_fma(V[7], SY, f2_fma(V[4], SX, V[1])));
+            const f2 EB = f2_fma(V[11], P, f2_fma(V[8], SY, f2_fma(V[5], SX, V[2])));
+            cr = f2_fma(AL, ER, cr);
+            cg = f2_fma(AL, EG, cg);
+            cb = f2_fma(AL, EB, cb);
+            f2 G = f2_fma(CB, EB, f2_fma(CG, EG, f2_mul(CR, ER)));
+            const f2 VX = f2_fma(CB, V[5], f2_fma(CG, V[4], f2_mul(CR, V[3])));
+            const f2 VY = f2_fma(CB, V[8], f2_fma(CG, V[7], f2_mul(CR, V[6])));
+            const f2 VP = f2_fma(CB, V[11], f2_fma(CG, V[10], f2_mul(CR, V[9])));
+            f2 W{0};
+            if constexpr (VW) {
+                W = f2{*reinterpret_cast<const unsigned long long *>(e.vw)};
+                G = f2_add(G, W);
+            }
+            if constexpr (OP) {  // vis (v . colour + v_wsum), the reference's rule
+                f2 VA = f2_fma(CB, V[2], f2_fma(CG, V[1], f2_mul(CR, V[0])));
+                if constexpr (VW) VA = f2_add(VA, W);
+                vo = f2_fma(f2_pack(no0 ? 0.f : vis0, no1 ? 0.f : vis1), VA, vo);
+            }
+            const f2 GX = f2_fma(VP, SY, VX), GY = f2_fma(VP, SX, VY);
+            const f2 ALX = f2_mul(AL, DX);
+            wr[r] = f2_fma(AL, G, wr[r]);
+            wx[r] = f2_fma(ALX, G, wx[r]);
+            wxx = f2_fma(f2_mul(ALX, DX), G, wxx);
+            ar[r] = f2_fma(AL, GX, ar[r]);
+            ax = f2_fma(ALX, GX, ax);
+            br[r] = f2_fma(AL, GY, br[r]);
+            bx = f2_fma(ALX, GY, bx);
+            dd = f2_fma(AL, VP, dd);
+        }
+    }
+    const float w0 = f2_sum(wr[0]), w1 = f2_sum(wr[1]), x0 = f2_sum(wx[0]), x1 = f2_sum(wx[1]);
+    const float a0 = f2_sum(ar[0]), a1 = f2_sum(ar[1]), b0 = f2_sum(br[0]), b1 = f2_sum(br[1]);
+    const float ux = x0 + x1 - (a0 + a1);                      // S10 - A
+    const float wy0 = w0 * dy[0], wy1 = w1 * dy[1];
+    const float uy = wy0 + wy1 - (b0 + b1);                    // S01 - B
+    acc[0] += g.a * ux + g.b * uy;
+    acc[1] += g.b * ux + g.c * uy;
+    acc[4] += f2_sum(ax) - 0.5f * f2_sum(wxx);
+    acc[5] += (a0 * dy[0] + a1 * dy[1]) + f2_sum(bx) - (x0 * dy[0] + x1 * dy[1]) - f2_sum(dd);
+    acc[6] += (b0 * dy[0] + b1 * dy[1]) - 0.5f * (wy0 * dy[0] + wy1 * dy[1]);
+    acc[7] += f2_sum(cr);
+    acc[8] += f2_sum(cg);
+    acc[9] += f2_sum(cb);
+    if constexpr (OP) acc[10] += f2_sum(vo);
+}
+
+// One Gaussian over the region's pixels part, part + step, ... one at a time
+// (rank = row W + column), skipping what fails the alpha test: records and
+// tiles whose zeros could turn into NaN.  The expanded formulas of
+// csrc/gradient_aware_rasterizer.cu:201-315.
+template <int W>
+__device__ __noinline__ void ga_pixels_skip(const Rec<float> &g, float clamp, const GaPix *pix,
+                                            int part, int step, float px0, float py0, float *acc) {
+    for (int j = part; j < 32; j += step) {
+        const int row = j / W, col = j % W, h = col / (W / 2);
+        const GaPix &e = pix[row * (W / 2) + col % (W / 2)];
+        if (e.in[h] == 0.f) continue;
+        const float dx = (px0 + (float)col) - g.x, dy = (py0 + (float)row) - g.y;
+        const float sigma = sigma_ref<float>(g.a, g.b, g.c, dx, dy);
+        const float vis = __expf(-sigma);
+        const float alpha = fminf(clamp, g.o * vis);
+        if (sigma < 0.f || alpha < 1.f / 255.f) continue;
+        const float a = g.a, b = g.b, c = g.c;
+        const float sx = a * dx + b * dy, sy = b * dx + c * dy;
+        const float ax = -alpha * sx, ay = -alpha * sy, axy = alpha * (sx * sy - b);
+        float vo[3], vx[3], vy[3], vp[3];
+        for (int ch = 0; ch < 3; ++ch) {
+            vo[ch] = e.v[ch][h];
+            vx[ch] = -e.v[3 + ch][h];
+            vy[ch] = -e.v[6 + ch][h];
+            vp[ch] = e.v[9 + ch][h];
+            acc[7 + ch] += vo[ch] * alpha + vx[ch] * ax + vy[ch] * ay + vp[ch] * axy;
+        }
+        const float va = (vo[0] * g.r + vo[1] * g.g + vo[2] * g.bl) + e.vw[h];
+        const float vax = vx[0] * g.r + vx[1] * g.g + vx[2] * g.bl;
+        const float vay = vy[0] * g.r + vy[1] * g.g + vy[2] * g.bl;
+        const float vaxy = vp[0] * g.r + vp[1] * g.g + vp[2] * g.bl;
+        const float sx2 = sx * sx, sy2 = sy * sy, sxsy = sx * sy;
+        acc[0] += alpha * (va * sx + vax * (a - sx2) + vay * (b - sxsy) +
+                           vaxy * (sx2 * sy - 2.f * b * sx - a * sy));
+        acc[1] += alpha * (va * sy + vax * (b - sxsy) + vay * (c - sy2) +
+                           vaxy * (sx * sy2 - 2.f * b * sy - c * sx));
+        const float dx2 = dx * dx, dy2 = dy * dy, dxdy = dx * dy, P = sxsy - b;
+        acc[4] += alpha * (va * (-0.5f * dx2) + vax * (0.5f * dx2 * sx - dx) +
+                           vay * (0.5f * dx2 * sy) + vaxy * (-0.5f * dx2 * P + dx * sy));
+        acc[5] += alpha * (va * (-dxdy) + vax * (dxdy * sx - dy) + vay * (dxdy * sy - dx) +
+                           vaxy * (-dxdy * P + dy * sy + dx * sx - 1.f));
+        acc[6] += alpha * (va * (-0.5f * dy2) + vax * (0.5f * dy2 * sx) +
+                           vay * (0.5f * dy2 * sy - dy) + vaxy * (-0.5f * dy2 * P + dy * sx));
+        acc[10] += vis * va;
+    }
+}
+
+template <int W, bool OP, bool VW, int MINB>
+__global__ void __launch_bounds__(W * W, MINB)
+raster_bwd_ga_kernel(const BatchGeo geo, const int32_t *__restrict__ cum, int *work,
+                     const int32_t *__restrict__ ids, const int2 *__restrict__ tile_bins,
+                     const int32_t *__restrict__ d_total, const Rec<float> *__restrict__ recs,
+                     const float *__restrict__ v_img, const float *__restrict__ v_wsum,
+                     const float *__restrict__ v_dx, const float *__restrict__ v_dy,
+                     const float *__restrict__ v_dxy, float clamp, float *__restrict__ packed) {
+    constexpr int NT = W * W, HW = W / 2, NR = 32 / W;  // threads, pairs a row, rows a region
+    constexpr int NW = NT / 32;
+    __shared__ GaPix s_pix[NW * 16];
+    __shared__ __align__(16) Rec<float> s_rec[NT];
+    __shared__ int32_t s_ids[NT];
+    __shared__ uint16_t s_list[NW][NT];
+    __shared__ int s_slot;
+    __shared__ __align__(8) unsigned long long s_mbar;
+    const unsigned FULL = 0xffffffffu;
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&s_mbar);
+    uint32_t phase = 0;
+    if (tid == 0) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(1));
+        asm volatile("fence.mbarrier_init.release.cluster;");
+    }
+    __syncthreads();
+    const int n_tiles = geo.total_tiles();
+    const GaPix *my_pix = s_pix + w * 16;
+    uint16_t *my_list = s_list[w];
+    for (int tile = next_tile(work, s_slot, true); tile < n_tiles;
+         tile = next_tile(work, s_slot, false)) {
+        const TileCtx tc = tile_ctx(geo, cum, d_total, tile);
+        if (tc.empty) continue;  // gradients stay zero (rasterize.py:156-161)
+        const int2 range = tile_bins[tile];
+        if (range.x >= range.y) continue;
+        const Regions R = Regions::make(2, W);
+        bulk_records(bar, s_rec, s_ids, ids, recs, range.x, min(NT, range.y - range.x));
+        // stage this thread's pixel: rank tid of the tile
+        const int col = tid % W, gx = tc.tx0 + col, gy = tc.ty0 + tid / W;
+        const bool inside = gx < tc.W && gy < tc.H;
+        const int p = inside ? tc.poff + gy * tc.W + gx : 0;
+        float v[13];
+#pragma unroll
+        for (int ch = 0; ch < 3; ++ch) {
+            v[ch] = inside ? v_img[3 * p + ch] : 0.f;
+            v[3 + ch] = inside ? -v_dx[3 * p + ch] : 0.f;
+            v[6 + ch] = inside ? -v_dy[3 * p + ch] : 0.f;
+            v[9 + ch] = inside ? v_dxy[3 * p + ch] : 0.f;
+        }
+        v[12] = VW && inside ? v_wsum[p] : 0.f;
+        GaPix &mine = s_pix[w * 16 + (lane / W) * HW + col % HW];
+        bool tame_cot = true;
+        mine.in[col / HW] = inside ? 1.f : 0.f;
+#pragma unroll
+        for (int q = 0; q < 13; ++q) {
+            tame_cot = tame_cot && fabsf(v[q]) < kTameCot;
+            if (q < 12) mine.v[q][col / HW] = v[q];
+            else mine.vw[col / HW] = v[q];
+        }
+        const bool wild = __syncthreads_or(!tame_cot);
+        const float px0 = (float)tc.tx0 + 0.5f, py0 = (float)(tc.ty0 + w * NR) + 0.5f;
+        for (int base = range.x; base < range.y; base += NT) {
+            const int cnt = min(NT, range.y - base);
+            if (base != range.x) {  // everyone is done with the previous batch
+                __syncthreads();
+                bulk_records(bar, s_rec, s_ids, ids, recs, base, cnt);
+            }
+            const bool ok = mbar_wait(bar, phase);
+            phase ^= 1u;
+            // as in bwd_tile: a wait that gave up abandons the tile
+            if (__syncthreads_or(!ok)) {
+                if (tid == 0) atomicAdd(&g_wait_timeouts, 1u);
+                (void)mbar_wait(bar, phase ^ 1u);
+                break;
+            }
+            // the batch's Gaussians that reach this region, in list order
+            int nmine = 0;
+            for (int m = 0; m * 32 < cnt; ++m) {
+                const int t = m * 32 + lane;
+                const bool hit =
+                    t < cnt && region_hit<float, true, false>(s_rec[t], R, w, tc.tx0, tc.ty0);
+                const uint32_t mask = __ballot_sync(FULL, hit);
+                if (hit) my_list[nmine + __popc(mask & ((1u << lane) - 1u))] = (uint16_t)t;
+                nmine += __popc(mask);
+            }
+            __syncwarp();
+            for (int g0 = 0, lsplit = 0; g0 < nmine; g0 += 32 >> lsplit) {
+                const int left = min(32, nmine - g0);
+                lsplit = left <= LIG_RASTER_GA_BWD_SPLIT3   ? 3
+                         : left <= LIG_RASTER_GA_BWD_SPLIT2 ? 2
+                         : left <= LIG_RASTER_GA_BWD_SPLIT1 ? 1 : 0;
+                const int gi = lane >> lsplit, part = lane & ((1 << lsplit) - 1);
+                const bool act = gi < left;
+                const int slot = act ? (int)my_list[g0 + gi] : 0;
+                const Rec<float> g = s_rec[slot];
+                float acc[11];
+#pragma unroll
+                for (int q = 0; q < 11; ++q) acc[q] = 0.f;
+                if (act && (wild || !(g.wx >= 0.f))) {
+                    float t[11] = {};
+                    ga_pixels_skip<W>(s_rec[slot], clamp, my_pix, part, 1 << lsplit, px0, py0, t);
+#pragma unroll
+                    for (int q = 0; q < 11; ++q) acc[q] = t[q];
+                } else if (act) {
+                    // row pairs: one for W = 16, two for W = 8 (8 lanes: one each)
+                    const int rb = W == 8 && lsplit == 3 ? part >> 2 : 0;
+                    const int re = W == 8 && lsplit == 3 ? rb + 1 : NR / 2;
+#pragma unroll 1
+                    for (int rp = rb; rp < re; ++rp) {
+                        const GaPix *rows = my_pix + 2 * rp * HW;
+                        const float py = py0 + (float)(2 * rp);
+                        switch (lsplit) {
+                        case 0:
+                            ga_rows<HW, 1, HW, OP, VW>(g, clamp, rows, 0, px0, py, acc);
+                            break;
+                        case 1:
+                            ga_rows<HW / 2, 2, HW, OP, VW>(g, clamp, rows, part, px0, py, acc);
+                            break;
+                        case 2:
+                            ga_rows<HW / 4, 4, HW, OP, VW>(g, clamp, rows, part, px0, py, acc);
+                            break;
+                        default:
+                            ga_rows<1, 8, HW, OP, VW>(g, clamp, rows, part & (HW - 1), px0, py,
+                                                      acc);
+                            break;
+                        }
+                    }
+                }
+                for (int o = 1; o < (1 << lsplit); o <<= 1) {  // combine the lane group
+#pragma unroll
+                    for (int q = 0; q < 11; ++q) {
+                        if (q == 2 || q == 3 || (!OP && q == 10)) continue;
+                        acc[q] += __shfl_xor_sync(FULL, acc[q], o);
+                    }
+                }
+                if (act && part == 0) {
+                    // v_xy_abs: |sum over the reference's warp| (= this region)
+                    float4 *d4 = reinterpret_cast<float4 *>(packed + (size_t)s_ids[slot] * 12);
+                    atomicAdd(d4, make_float4(acc[0], acc[1], fabsf(acc[0]), fabsf(acc[1])));
+                    atomicAdd(d4 + 1, make_float4(acc[4], acc[5], acc[6], acc[7]));
+                    atomicAdd(d4 + 2, make_float4(acc[8], acc[9], OP ? acc[10] : 0.f, 0.f));
+                }
+            }
+        }
+    }
+}
+
 // Packed per-Gaussian gradients [N][12] -> the five output arrays of the ABI.
 template <typename T>
 __global__ void unpack_lean_grads_kernel(int n, const T *__restrict__ packed, Grads<T> out) {
@@ -1695,11 +2235,13 @@ __global__ void unpack_grads_kernel(int n, const T *__restrict__ packed, Grads<T
 template <typename T>
 int pack(int n, const void *xys, const void *con, const void *col, const void *op, void *ws,
          size_t ws_bytes, cudaStream_t s, bool half = false, T *zero = nullptr,
-         int zero_stride = 0) {
+         int zero_stride = 0, bool tame = false) {
     if (ws_bytes < sizeof(Rec<T>) * (size_t)n) return LIG_ERR_WORKSPACE;
     if ((reinterpret_cast<uintptr_t>(ws) & 15) != 0) return LIG_ERR_INVALID;  // 16-byte records
     if (n > 0) {
-        auto k = half ? pack_kernel<T, true> : pack_kernel<T, false>;
+        auto k = half   ? pack_kernel<T, true>
+                 : tame ? pack_kernel<T, false, true>
+                        : pack_kernel<T, false>;
         k<<<(n + 255) / 256, 256, 0, s>>>(n, (const T *)xys, (const T *)con, (const T *)col,
                                           (const T *)op, (Rec<T> *)ws, zero, zero_stride);
     }
@@ -1767,6 +2309,29 @@ template <typename T> struct L2Out {
     T *loss = nullptr, *per_image = nullptr;
 };
 
+inline int raster_fwd_ga(const BatchGeo &geo, TileWalk walk, const int32_t *ids,
+                         const int32_t *bins, const int32_t *d_total, const void *ws, bool op,
+                         float *img, float *wsum, float *dx, float *dy, float *dxy, int32_t *fin,
+                         cudaStream_t s) {
+    const int nt = 32 * Regions::make(1, geo.B).count;  // at most 128; 512 for B > 16
+    const size_t sm = (size_t)nt * sizeof(Rec<float>);
+    auto fn = geo.B > 16 ? (op ? raster_fwd_ga_kernel<true, 512, 1> : raster_fwd_ga_kernel<false, 512, 1>)
+              : op       ? raster_fwd_ga_kernel<true, 128, LIG_RASTER_GA_MINB>
+                         : raster_fwd_ga_kernel<false, 128, LIG_RASTER_GA_MINB>;
+    int grid = geo.total_tiles();
+    if (walk.work) {
+        const int pg = persistent_grid((const void *)fn, nt, sm);
+        if (pg <= 0) return LIG_ERR_LAUNCH;
+        grid = grid < pg ? grid : pg;
+        cudaMemsetAsync(walk.work, 0, sizeof(int), s);
+    }
+    fn<<<grid, nt, sm, s>>>(geo, walk.cum, walk.work, ids, (const int2 *)bins, d_total,
+                            (const Rec<float> *)ws, img, wsum, dx, dy, dxy, fin);
+    note_launches(1);
+    LIG_LAUNCH_CHECK();
+    return LIG_OK;
+}
+
 template <typename T>
 int raster_fwd(const BatchGeo &geo, TileWalk walk, const int32_t *ids, const int32_t *bins,
                const int32_t *d_total, const void *xys, const void *con, const void *col,
@@ -1777,8 +2342,13 @@ int raster_fwd(const BatchGeo &geo, TileWalk walk, const int32_t *ids, const int
     const bool ga = dx != nullptr;
     // fused loss without opacities: the specialised forward (halved conic)
     const bool fl = !ga && (l2.target || l2.target_u8) && !op && LIG_RASTER_FWD_FUSED;
-    int rc = pack<T>(n, xys, con, col, op, ws, ws_bytes, s, fl);
+    int rc = pack<T>(n, xys, con, col, op, ws, ws_bytes, s, fl, nullptr, 0, ga);
     if (rc) return rc;
+    if constexpr (sizeof(T) == 4) {
+        if (ga)
+            return raster_fwd_ga(geo, walk, ids, bins, d_total, ws, op != nullptr, (float *)img,
+                                 (float *)wsum, (float *)dx, (float *)dy, (float *)dxy, fin, s);
+    }
     const bool ppl4 = !ga && geo.total_tiles() >= LIG_RASTER_PPL4_MIN_TILES;
     const bool ppl2 = !ga && !ppl4 && geo.total_tiles() >= LIG_RASTER_PPL2_MIN_TILES;
     const int nt = 32 * Regions::make(ppl4 ? 3 : (ppl2 ? 1 : 0), geo.B).count;
@@ -1834,6 +2404,34 @@ int raster_fwd(const BatchGeo &geo, TileWalk walk, const int32_t *ids, const int
     return LIG_OK;
 }
 
+inline int raster_bwd_ga(const BatchGeo &geo, TileWalk walk, const int32_t *ids,
+                         const int32_t *bins, const int32_t *d_total, const void *ws, bool op,
+                         const CotSrc<float> &cot, const float *v_dx, const float *v_dy,
+                         const float *v_dxy, float clamp, float *packed, cudaStream_t s) {
+    constexpr int M = LIG_RASTER_GA_BWD_MINB;
+    const bool vw = cot.v_wsum != nullptr;
+    auto fn = geo.B == 16 ? (op ? (vw ? raster_bwd_ga_kernel<16, true, true, M>
+                                      : raster_bwd_ga_kernel<16, true, false, M>)
+                                : (vw ? raster_bwd_ga_kernel<16, false, true, M>
+                                      : raster_bwd_ga_kernel<16, false, false, M>))
+                          : (op ? (vw ? raster_bwd_ga_kernel<8, true, true, 4 * M>
+                                      : raster_bwd_ga_kernel<8, true, false, 4 * M>)
+                                : (vw ? raster_bwd_ga_kernel<8, false, true, 4 * M>
+                                      : raster_bwd_ga_kernel<8, false, false, 4 * M>));
+    const int nt = geo.B * geo.B;
+    int grid = geo.total_tiles();
+    if (walk.work) {
+        const int pg = persistent_grid((const void *)fn, nt, 0);
+        if (pg <= 0) return LIG_ERR_LAUNCH;
+        grid = grid < pg ? grid : pg;
+        cudaMemsetAsync(walk.work, 0, sizeof(int), s);
+    }
+    fn<<<grid, nt, 0, s>>>(geo, walk.cum, walk.work, ids, (const int2 *)bins, d_total,
+                           (const Rec<float> *)ws, cot.v_img, cot.v_wsum, v_dx, v_dy, v_dxy, clamp,
+                           packed);
+    return LIG_OK;
+}
+
 // Backward workspace: packed records [N] followed by packed gradients [N][12].
 template <typename T>
 inline size_t bwd_grad_offset(int n) {
@@ -1860,10 +2458,25 @@ int raster_bwd(const BatchGeo &geo, TileWalk walk, const int32_t *ids, const int
                           sizeof(T) == 4 && LIG_RASTER_BWD_F2;
     const int stride = lean ? 8 : 12;
     T *packed = reinterpret_cast<T *>((char *)ws + goff);
+    // float gradient-aware: 16x16 and 8x8 tiles, whose reference warps are
+    // blocks of pixels
+    const bool ga_pairs = ga && sizeof(T) == 4 && cot.v_img && (geo.B == 16 || geo.B == 8);
     // records, and the packed gradients cleared in the same pass
-    int rc = pack<T>(n, xys, con, col, op, ws, goff, s, false, packed, stride);
+    int rc = pack<T>(n, xys, con, col, op, ws, goff, s, false, packed, stride, ga_pairs);
     if (rc) return rc;
     const T cl = (T)(clamp > 0 ? clamp : (ga ? 0.999 : 0.99));
+    Grads<T> g{(T *)v_xy, (T *)v_abs, (T *)v_con, (T *)v_rgb, (T *)v_op};
+    if constexpr (sizeof(T) == 4) {
+        if (ga_pairs) {
+            rc = raster_bwd_ga(geo, walk, ids, bins, d_total, ws, op || v_op, cot, (const T *)v_dx,
+                               (const T *)v_dy, (const T *)v_dxy, cl, packed, s);
+            if (rc) return rc;
+            if (n > 0) unpack_grads_kernel<T><<<(n + 255) / 256, 256, 0, s>>>(n, packed, g);
+            note_launches(n > 0 ? 2 : 1);
+            LIG_LAUNCH_CHECK();
+            return LIG_OK;
+        }
+    }
     const bool large = geo.total_tiles() >= LIG_RASTER_BWD_LARGE_MIN_TILES;
     // the float lean walks of large images: 8x8 regions (tiles up to 16x16)
     const double density = (double)n / (double)geo.total_pixels();
@@ -1919,7 +2532,6 @@ int raster_bwd(const BatchGeo &geo, TileWalk walk, const int32_t *ids, const int
                             (const Rec<T> *)ws, fin, cot, ga ? (const T *)v_dx : nullptr,
                             ga ? (const T *)v_dy : nullptr, ga ? (const T *)v_dxy : nullptr, cl,
                             packed);
-    Grads<T> g{(T *)v_xy, (T *)v_abs, (T *)v_con, (T *)v_rgb, (T *)v_op};
     if (n > 0 && lean) unpack_lean_grads_kernel<T><<<(n + 255) / 256, 256, 0, s>>>(n, packed, g);
     else if (n > 0) unpack_grads_kernel<T><<<(n + 255) / 256, 256, 0, s>>>(n, packed, g);
     note_launches(n > 0 ? 2 : 1);
