@@ -2,7 +2,9 @@
 
 Compiles every ``lig_b200/csrc/*.cu`` with nvcc for ``sm_100a`` into
 ``lig_b200/_build/*.o`` (in parallel, skipping up-to-date objects) and links
-``lig_b200/liblig_b200.so``, which ``lig_b200._lib`` loads through ctypes.
+``lig_b200/liblig_b200.so``, which ``lig_b200._lib`` loads through ctypes; then
+compiles ``lig_b200/csrc/host.cpp`` with g++ against torch's headers into
+``lig_b200/_host.so``, the native half of ``lig_b200.ops``.
 Run it as a script (``python lig_b200/build.py``): importing the package
 loads the library, which must exist first.
 
@@ -21,6 +23,8 @@ import sys
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG, "csrc")
+HOST_SRC = os.path.join(CSRC, "host.cpp")
+HOST_LIB = os.path.join(PKG, "_host.so")
 BUILD = os.path.join(PKG, "_build")
 LIB = os.path.join(PKG, "liblig_b200.so")
 INCLUDE = os.path.join(os.path.dirname(PKG), "include")
@@ -60,6 +64,29 @@ def _compile(src: str, extra) -> str:
     return obj
 
 
+def _build_host() -> None:
+    """Compile the native half of ops.py (a Python module on torch's headers,
+    linked against the CUDA library beside it)."""
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension as tx
+
+    cuda = os.path.dirname(os.path.dirname(nvcc()))
+    inc = [sysconfig.get_paths()["include"], os.path.join(cuda, "include"), *tx.include_paths()]
+    lib = os.path.join(os.path.dirname(torch.__file__), "lib")
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           "-DTORCH_EXTENSION_NAME=_host", *[f for i in inc for f in ("-isystem", i)], HOST_SRC,
+           "-o", HOST_LIB, "-L", PKG, "-l:liblig_b200.so", "-L", lib, "-lc10", "-lc10_cuda",
+           "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python",
+           "-L", os.path.join(cuda, "lib64"), "-lcudart", "-Wl,-rpath,$ORIGIN",
+           f"-Wl,-rpath,{lib}"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"g++ failed for {HOST_SRC}:\n{r.stdout}\n{r.stderr}")
+
+
 def build(verbose: bool = False, extra=()) -> str:
     """Compile (incrementally) and link liblig_b200.so; returns its path."""
     os.makedirs(BUILD, exist_ok=True)
@@ -71,8 +98,10 @@ def build(verbose: bool = False, extra=()) -> str:
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
+    if _stale(HOST_LIB, [HOST_SRC, os.path.join(INCLUDE, "lig_b200.h")]):
+        _build_host()
     if verbose:
-        print(f"built {LIB}")
+        print(f"built {LIB}, {HOST_LIB}")
     return LIB
 
 

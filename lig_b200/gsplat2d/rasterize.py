@@ -72,13 +72,9 @@ class _RasterizeGaussians(Function):
     @staticmethod
     def forward(ctx, xys, extents, conics, num_tiles_hit, colors, opacities, img_height,
                 img_width, block_width, compute_upscale_gradients, alpha_clamp=None):
-        def enqueue_raster(b):
-            return ops.raster_fwd(img_height, img_width, block_width, b.gaussian_ids_sorted,
-                                  b.tile_bins, b.total, xys, conics, colors, opacities,
-                                  compute_upscale_gradients)
-
-        binning, outs = ops.bin_gaussians(xys, extents, num_tiles_hit, img_height, img_width,
-                                          block_width, after_enqueue=enqueue_raster)
+        binning, outs = ops.bin_raster_fwd(xys, extents, num_tiles_hit, conics, colors, opacities,
+                                           img_height, img_width, block_width,
+                                           compute_upscale_gradients)
         out_img, out_wsum, out_dx, out_dy, out_dxy, final_idx = outs
         if not compute_upscale_gradients:
             out_dx = out_dy = out_dxy = None

@@ -24,6 +24,7 @@ import torch
 
 from . import _lib
 from ._lib import call as _raw_call
+from . import _host  # lig_b200/csrc/host.cpp (after _lib, which loads the CUDA library)
 
 _VP = ctypes.c_void_p
 
@@ -87,12 +88,23 @@ class KernelTimer:
         global _TIMER
         self.events = []
         _TIMER = self.events
+        _host.set_observer(self._observe)
         return self
 
     def __exit__(self, *exc):
         global _TIMER
         _TIMER = None
+        _host.set_observer(None)
         return False
+
+    def _observe(self, name, end):
+        """Calls made by the native operators: before (0) and after (1)."""
+        ev = torch.cuda.Event(enable_timing=True)
+        ev.record()
+        if end:
+            self.events.append((name, self._start, ev))
+        else:
+            self._start = ev
 
     def summary(self):
         torch.cuda.synchronize()
@@ -126,19 +138,8 @@ def probe_fp32(device=None, blocks=None, iters=4096):
 
 # ------------------------------------------------------------------ projection
 def project_fwd(in3, means2d, opacities, img_h, img_w, block, cholesky: bool):
-    _check_cuda(in3, means2d, opacities)
-    in3 = _c(in3)
-    means2d = _c(means2d, in3.dtype)
-    opacities = _c(opacities, in3.dtype)
-    n = in3.shape[0]
-    xys = torch.empty((n, 2), dtype=in3.dtype, device=in3.device)
-    ext = torch.empty((n, 2), dtype=in3.dtype, device=in3.device)
-    con = torch.empty((n, 3), dtype=in3.dtype, device=in3.device)
-    cnt = torch.empty((n,), dtype=torch.int32, device=in3.device)
-    call("lig_project_fwd", _dt(in3), n, int(cholesky), _p(in3), _p(means2d), _p(opacities),
-         int(img_h), int(img_w), int(block), _p(xys), _p(ext), _p(con), _p(cnt),
-         _stream(in3.device))
-    return xys, ext, con, cnt
+    return tuple(_host.project_fwd(in3, means2d, opacities, int(img_h), int(img_w), int(block),
+                                   bool(cholesky)))
 
 
 def project_fwd_view(in3, means2d, opacities, img_h, img_w, block, cholesky: bool,
@@ -161,27 +162,9 @@ def project_fwd_view(in3, means2d, opacities, img_h, img_w, block, cholesky: boo
     return xys, ext, con, cnt
 
 
-def _rows(t: torch.Tensor, width: int) -> torch.Tensor:
-    """Row-strided view accepted by the kernels (unit inner stride)."""
-    if t.dim() != 2 or t.shape[1] != width or t.stride(1) != 1 or t.stride(0) < width:
-        t = t.contiguous()
-    return t
-
-
 def project_bwd(in3, means2d, opacities, img_h, img_w, block, cholesky, v_xy, v_conic):
-    _check_cuda(in3, means2d, v_xy, v_conic)
-    in3 = _c(in3)
-    means2d = _c(means2d, in3.dtype)
-    opacities = _c(opacities, in3.dtype)
-    v_xy = _rows(v_xy.to(in3.dtype), 2)
-    v_conic = _rows(v_conic.to(in3.dtype), 3)
-    n = in3.shape[0]
-    v_in3 = torch.empty((n, 3), dtype=in3.dtype, device=in3.device)
-    v_mean = torch.empty((n, 2), dtype=in3.dtype, device=in3.device)
-    call("lig_project_bwd", _dt(in3), n, int(cholesky), _p(in3), _p(means2d), _p(opacities),
-         int(img_h), int(img_w), int(block), _p(v_xy), v_xy.stride(0), _p(v_conic),
-         v_conic.stride(0), _p(v_in3), _p(v_mean), _stream(in3.device))
-    return v_in3, v_mean
+    return tuple(_host.project_bwd(in3, means2d, opacities, int(img_h), int(img_w), int(block),
+                                   bool(cholesky), v_xy, v_conic))
 
 
 def project_bwd_saved(extents, in3, conics, v_xy, v_conic, cholesky: bool):
@@ -214,16 +197,7 @@ def cov2d_bounds(cov2d, opacities=None):
 def cumsum_tiles(num_tiles_hit: torch.Tensor):
     """Inclusive int32 prefix sum; returns (cum, total) with total a 1-element
     int32 device tensor (no host synchronisation)."""
-    _check_cuda(num_tiles_hit)
-    cnt = _c(num_tiles_hit.reshape(-1), torch.int32)
-    n = cnt.shape[0]
-    dev = cnt.device
-    cum = torch.empty((n,), dtype=torch.int32, device=dev)
-    total = torch.empty((1,), dtype=torch.int32, device=dev)
-    wsb = _lib.lib.lig_cumsum_workspace_bytes(n)
-    ws = torch.empty((wsb,), dtype=torch.uint8, device=dev)
-    call("lig_cumsum_tiles", n, _p(cnt), _p(cum), _p(total), _p(ws), wsb, _stream(dev))
-    return cum, total
+    return _host.cumsum_tiles(num_tiles_hit)
 
 
 @dataclass
@@ -256,26 +230,17 @@ _CAP_HINT: dict = {}
 _SLACK = 1.125
 
 
+def _guess(hint: int) -> int:
+    return int(hint * _SLACK) + 256
+
+
 def _run_bin(xys, extents, cum, total, img_h, img_w, block, capacity, want_keys):
-    dev = xys.device
-    tbx, tby = tile_bounds(img_h, img_w, block)
-    T = tbx * tby
-    n = xys.shape[0]
-    cap = max(int(capacity), 0)
-    wsb = _lib.lib.lig_bin_workspace_bytes(n, cap, T)
-    ws = torch.empty((max(wsb, 1),), dtype=torch.uint8, device=dev)
-    gid_sorted = torch.empty((max(cap, 1),), dtype=torch.int32, device=dev)
-    bins = torch.empty((T, 2), dtype=torch.int32, device=dev)
-    status = torch.empty((1,), dtype=torch.int32, device=dev)
-    isect = gids = isect_sorted = None
-    if want_keys:
-        isect = torch.empty((max(cap, 1),), dtype=torch.int64, device=dev)
-        gids = torch.empty((max(cap, 1),), dtype=torch.int32, device=dev)
-        isect_sorted = torch.empty((max(cap, 1),), dtype=torch.int64, device=dev)
-    call("lig_bin", _dt(xys), n, _p(xys), _p(extents), _p(cum), _p(total), int(img_h),
-         int(img_w), int(block), cap, _p(ws), wsb, _p(gid_sorted), _p(bins), _p(isect),
-         _p(gids), _p(isect_sorted), _p(status), _stream(dev))
-    return gid_sorted, bins, isect, gids, isect_sorted
+    return _host.run_bin(xys, extents, cum, total, int(img_h), int(img_w), int(block),
+                         int(capacity), bool(want_keys))
+
+
+def _cap_key(n, img_h, img_w, block, dev):
+    return (n, img_h, img_w, block, dev.index)
 
 
 def bin_gaussians(xys, extents, num_tiles_hit, img_h, img_w, block, want_keys=False,
@@ -294,14 +259,14 @@ def bin_gaussians(xys, extents, num_tiles_hit, img_h, img_w, block, want_keys=Fa
     host.copy_(total, non_blocking=True)
     ev = torch.cuda.Event()
     ev.record(torch.cuda.current_stream(xys.device))
-    key = (n, img_h, img_w, block, xys.device.index)
+    key = _cap_key(n, img_h, img_w, block, xys.device)
     hint = _CAP_HINT.get(key)
     if hint is None:
         ev.synchronize()
         m = int(host.item())
         cap = m
     else:
-        cap = int(hint * _SLACK) + 256
+        cap = _guess(hint)
     res = _run_bin(xys, extents, cum, total, img_h, img_w, block, cap, want_keys)
     b = Binning(-1, total, cap, cum, *res)
     extra = after_enqueue(b) if after_enqueue is not None else None
@@ -315,6 +280,19 @@ def bin_gaussians(xys, extents, num_tiles_hit, img_h, img_w, block, want_keys=Fa
     _CAP_HINT[key] = m
     b.num_intersects = m
     return (b, extra) if after_enqueue is not None else b
+
+
+def bin_raster_fwd(xys, extents, num_tiles_hit, conics, colors, opacities, img_h, img_w, block,
+                   grad_aware: bool):
+    """bin_gaussians with raster_fwd enqueued behind it, as one native call:
+    -> (Binning, (img, wsum, dx, dy, dxy, final_idx))."""
+    key = _cap_key(xys.shape[0], img_h, img_w, block, xys.device)
+    hint = _CAP_HINT.get(key)
+    m, cap, (cum, total), lists, outs = _host.bin_raster_fwd(
+        xys, extents, num_tiles_hit, conics, colors, opacities, int(img_h), int(img_w),
+        int(block), bool(grad_aware), -1 if hint is None else _guess(hint), _HostCount.slot())
+    _CAP_HINT[key] = m
+    return Binning(m, total, cap, cum, *lists), outs
 
 
 def map_intersects(xys, extents, cum, num_intersects, img_h, img_w, block):
@@ -348,52 +326,17 @@ def _raster_ws(dtype_code, n, dev):
 
 def raster_fwd(img_h, img_w, block, gaussian_ids_sorted, tile_bins, total, xys, conics,
                colors, opacities, grad_aware: bool):
-    _check_cuda(xys, conics, colors, opacities, tile_bins, total)
-    xys = _c(xys)
-    dt = xys.dtype
-    conics, colors, opacities = _c(conics, dt), _c(colors, dt), _c(opacities, dt)
-    n = xys.shape[0]
-    dev = xys.device
-    code = _dt(xys)
-    ws, wsb = _raster_ws(code, n, dev)
-    img = torch.empty((img_h, img_w, 3), dtype=dt, device=dev)
-    wsum = torch.empty((img_h, img_w), dtype=dt, device=dev)
-    fin = torch.empty((img_h, img_w), dtype=torch.int32, device=dev)
-    dx = dy = dxy = None
-    if grad_aware:
-        dx = torch.empty_like(img)
-        dy = torch.empty_like(img)
-        dxy = torch.empty_like(img)
-    call("lig_raster_fwd", code, int(img_h), int(img_w), int(block), n, _p(gaussian_ids_sorted),
-         _p(tile_bins), _p(total), _p(xys), _p(conics), _p(colors), _p(opacities), _p(ws), wsb,
-         _p(img), _p(wsum), _p(dx), _p(dy), _p(dxy), _p(fin), _stream(dev))
-    return img, wsum, dx, dy, dxy, fin
+    return tuple(_host.raster_fwd(int(img_h), int(img_w), int(block), gaussian_ids_sorted,
+                                  tile_bins, total, xys, conics, colors, opacities,
+                                  bool(grad_aware)))
 
 
 def raster_bwd(img_h, img_w, block, gaussian_ids_sorted, tile_bins, total, xys, conics, colors,
                opacities, final_idx, v_img, v_wsum, v_dx=None, v_dy=None, v_dxy=None,
                alpha_clamp: float = 0.0):
-    _check_cuda(xys, conics, colors, final_idx, v_img)
-    xys = _c(xys)
-    dt = xys.dtype
-    conics, colors, opacities = _c(conics, dt), _c(colors, dt), _c(opacities, dt)
-    v_img, v_wsum = _c(v_img, dt), _c(v_wsum, dt)
-    v_dx, v_dy, v_dxy = _c(v_dx, dt), _c(v_dy, dt), _c(v_dxy, dt)
-    n = xys.shape[0]
-    dev = xys.device
-    code = _dt(xys)
-    ws, wsb = _raster_ws(code, n, dev)
-    v_xy = torch.empty((n, 2), dtype=dt, device=dev)
-    v_abs = torch.empty((n, 2), dtype=dt, device=dev)
-    v_con = torch.empty((n, 3), dtype=dt, device=dev)
-    v_rgb = torch.empty((n, 3), dtype=dt, device=dev)
-    v_op = torch.empty((n,), dtype=dt, device=dev) if opacities is not None else None
-    call("lig_raster_bwd", code, int(img_h), int(img_w), int(block), n, _p(gaussian_ids_sorted),
-         _p(tile_bins), _p(total), _p(xys), _p(conics), _p(colors), _p(opacities),
-         _p(_c(final_idx, torch.int32)), _p(v_img), _p(v_wsum), _p(v_dx), _p(v_dy), _p(v_dxy),
-         float(alpha_clamp), _p(ws), wsb, _p(v_xy), _p(v_abs), _p(v_con), _p(v_rgb), _p(v_op),
-         _stream(dev))
-    return v_xy, v_abs, v_con, v_rgb, v_op
+    return tuple(_host.raster_bwd(int(img_h), int(img_w), int(block), gaussian_ids_sorted,
+                                  tile_bins, total, xys, conics, colors, opacities, final_idx,
+                                  v_img, v_wsum, v_dx, v_dy, v_dxy, float(alpha_clamp)))
 
 
 def raster_bwd_l2(img_h, img_w, block, gaussian_ids_sorted, tile_bins, total, xys, conics,
@@ -498,34 +441,12 @@ def l2_clamped_loss(img, target):
 def upscale_fwd(render, dx, dy, dxy, dst_h, dst_w, roi=None, mode: int = 0):
     """[H, W, C] value / dx / dy / dxy planes (C = 3, or 1 for the
     single-channel form) -> [dst_h, dst_w, C]."""
-    _check_cuda(render, dx, dy, dxy)
-    render = _c(render)
-    dt = render.dtype
-    dx, dy, dxy = _c(dx, dt), _c(dy, dt), _c(dxy, dt)
-    h, w, c = render.shape
-    if c not in (1, 3):
-        raise ValueError("gradient-aware upscale expects [H, W, 3] (or [H, W, 1]) planes")
-    if roi is None:
-        roi = (0.0, 0.0, float(w), float(h))
-    out = torch.empty((int(dst_h), int(dst_w), c), dtype=dt, device=render.device)
-    call("lig_upscale_fwd_nc", _dt(render), int(mode), c, h, w, int(dst_h), int(dst_w),
-         float(roi[0]), float(roi[1]), float(roi[2]), float(roi[3]), _p(render), _p(dx), _p(dy),
-         _p(dxy), _p(out), _stream(render.device))
-    return out
+    return _host.upscale_fwd(render, dx, dy, dxy, int(dst_h), int(dst_w), _roi(roi), int(mode))
 
 
 def upscale_bwd(grad_out, src_h, src_w, roi=None, mode: int = 0):
-    _check_cuda(grad_out)
-    grad_out = _c(grad_out)
-    dt = grad_out.dtype
-    dh, dw, c = grad_out.shape
-    if c not in (1, 3):
-        raise ValueError("gradient-aware upscale expects [H, W, 3] (or [H, W, 1]) planes")
-    if roi is None:
-        roi = (0.0, 0.0, float(src_w), float(src_h))
-    outs = [torch.empty((int(src_h), int(src_w), c), dtype=dt, device=grad_out.device)
-            for _ in range(4)]
-    call("lig_upscale_bwd_nc", _dt(grad_out), int(mode), c, int(src_h), int(src_w), dh, dw,
-         float(roi[0]), float(roi[1]), float(roi[2]), float(roi[3]), _p(grad_out),
-         *[_p(o) for o in outs], _stream(grad_out.device))
-    return tuple(outs)
+    return tuple(_host.upscale_bwd(grad_out, int(src_h), int(src_w), _roi(roi), int(mode)))
+
+
+def _roi(roi):
+    return None if roi is None else [float(roi[k]) for k in range(4)]
