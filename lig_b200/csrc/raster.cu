@@ -115,6 +115,13 @@ __device__ uint32_t g_alpha_cut;
 // take the kernels' skipping walk.
 constexpr float kTameSlope = 1e6f;  // largest conic entry times the reach: |sx|, |sy| < 2e6
 constexpr float kTameColor = 1e8f;
+constexpr float kTameCot = 1e12f;  // larger (or non-finite) cotangents: the skipping walks
+
+template <typename T>
+__device__ __forceinline__ bool tame_cotangent(T a, T b, T c, T d) {
+    return fabs(a) < (T)kTameCot && fabs(b) < (T)kTameCot && fabs(c) < (T)kTameCot &&
+           fabs(d) < (T)kTameCot;
+}
 
 template <typename T, bool HALF, bool TAME = false>
 __global__ void pack_kernel(int n, const T *__restrict__ xys, const T *__restrict__ conics,
@@ -799,6 +806,19 @@ __device__ __forceinline__ void fwd_tile(const TileCtx &tc, int tile, const int3
 #ifndef LIG_RASTER_BWD_R16_MINB
 #define LIG_RASTER_BWD_R16_MINB 14  // resident CTAs per SM of the 8x16 walk (64 threads, 72 registers)
 #endif
+// Resident CTAs per SM of the general walk (opacities, wsum cotangent), 8x4 /
+// 8x8 / 8x16 regions.  767x1023 / 150k: 4 CTAs 103 us, 3 107, 2 120 (150 for
+// the scalar walk); 2048^2 / 500k (8x8): 6 540, 7 532, 5 518 (726); 2048^2 /
+// 100k (8x16): 12 148, 14 147, 10 149 (243).
+#ifndef LIG_RASTER_GEN_MINB
+#define LIG_RASTER_GEN_MINB 4
+#endif
+#ifndef LIG_RASTER_GEN_R8_MINB
+#define LIG_RASTER_GEN_R8_MINB 5
+#endif
+#ifndef LIG_RASTER_GEN_R16_MINB
+#define LIG_RASTER_GEN_R16_MINB 12
+#endif
 #ifndef LIG_RASTER_BWD_SPLIT2
 #define LIG_RASTER_BWD_SPLIT2 8  // with up to this many Gaussians left, 4 lanes take one
 #endif
@@ -1271,7 +1291,7 @@ __device__ __forceinline__ void lean_region(const Rec<T> &g, T clamp,
 // so one 16-byte and one 8-byte load give three ready (column cp, cp + 4)
 // pairs.
 struct alignas(16) PixPair {
-    float v[8];  // v0 (cp, cp+4), v1 (cp, cp+4), v2 (cp, cp+4), unused
+    float v[8];  // v0 (cp, cp+4), v1 (cp, cp+4), v2 (cp, cp+4), v_wsum (GEN walks)
 };
 
 // lean_region in f32x2 form (float): the lane takes NCP column pairs
@@ -1287,7 +1307,9 @@ struct alignas(16) PixPair {
 // ABS: also the per-pixel absolute values of the mean gradient summed over
 // the pixels (the reference's v_xy_abs, csrc/backward.cu:146-150), in acc[2],
 // acc[3]: per pixel v_sigma (a dx + b dy) and v_sigma (b dx + c dy).
-template <int NCP, int CSTEP, int NR, bool ABS = false, int NH = 1>
+// GEN: opacities and a wsum cotangent (pair entry's fourth channel); the
+// opacity gradient's sum of exp(-sigma) v_alpha in acc[10].
+template <int NCP, int CSTEP, int NR, bool ABS = false, int NH = 1, bool GEN = false>
 __device__ __forceinline__ void lean_region_f2(const Rec<float> &g, float clamp,
                                                const PixPair *__restrict__ pp, int c0, int r0,
                                                float px0, float py0, float (&acc)[11]) {
@@ -1302,6 +1324,7 @@ __device__ __forceinline__ void lean_region_f2(const Rec<float> &g, float clamp,
     const f2 CR = f2_dup(g.r), CG = f2_dup(g.g), CB = f2_dup(g.bl);
     f2 sx = f2_zero(), sy = f2_zero(), sxx = f2_zero(), sxy = f2_zero(), syy = f2_zero();
     f2 sr = f2_zero(), sg = f2_zero(), sb = f2_zero();
+    [[maybe_unused]] f2 so = f2_zero();
     // NH blocks of NR rows, one after the other (not interleaved: the sums
     // carry over, the row and column products are rebuilt per block)
 #pragma unroll 1
@@ -1331,15 +1354,22 @@ __device__ __forceinline__ void lean_region_f2(const Rec<float> &g, float clamp,
                 const f2 S = f2_fma(BDX, DY[r], f2_fma(HADX, DX, CDD[r]));
                 float s0, s1;
                 f2_unpack(S, s0, s1);
-                const float al0 = fminf(clamp, __expf(-s0)), al1 = fminf(clamp, __expf(-s1));
-                const float a0 = (s0 < 0.f || al0 < 1.f / 255.f) ? 0.f : al0;
-                const float a1 = (s1 < 0.f || al1 < 1.f / 255.f) ? 0.f : al1;
-                const f2 A = f2_pack(a0, a1);
+                const float vis0 = __expf(-s0), vis1 = __expf(-s1);
+                const float al0 = fminf(clamp, GEN ? g.o * vis0 : vis0);
+                const float al1 = fminf(clamp, GEN ? g.o * vis1 : vis1);
+                const bool no0 = s0 < 0.f || al0 < 1.f / 255.f;
+                const bool no1 = s1 < 0.f || al1 < 1.f / 255.f;
+                const f2 A = f2_pack(no0 ? 0.f : al0, no1 ? 0.f : al1);
                 sr = f2_fma(A, V0, sr);
                 sg = f2_fma(A, V1, sg);
                 sb = f2_fma(A, V2, sb);
                 // -v_sigma per pixel
-                const f2 WV = f2_mul(A, f2_fma(CB, V2, f2_fma(CG, V1, f2_mul(CR, V0))));
+                f2 VA = f2_fma(CB, V2, f2_fma(CG, V1, f2_mul(CR, V0)));
+                if constexpr (GEN) {
+                    VA = f2_add(VA, f2{*reinterpret_cast<const unsigned long long *>(e->v + 6)});
+                    so = f2_fma(f2_pack(no0 ? 0.f : vis0, no1 ? 0.f : vis1), VA, so);
+                }
+                const f2 WV = f2_mul(A, VA);
                 wc = f2_add(wc, WV);
                 const f2 TY = f2_mul(WV, DY[r]);
                 yc = f2_add(yc, TY);
@@ -1365,6 +1395,45 @@ __device__ __forceinline__ void lean_region_f2(const Rec<float> &g, float clamp,
     if constexpr (ABS) {
         acc[2] += ax;
         acc[3] += ay;
+    }
+    if constexpr (GEN) acc[10] += f2_sum(so);
+}
+
+// GEN walks: one Gaussian over the region's pixels part, part + step, ... one
+// at a time (row-major 8-column region at pixel (rx, ry)), skipping what fails
+// the alpha test or lies outside: records and tiles whose zeros could turn
+// into NaN.  csrc/backward.cu:102-150; leaves the gradients themselves (no
+// moments) in acc.
+__device__ __noinline__ void sum_pixels_skip(const Rec<float> &g, float clamp,
+                                             const PixPair *pp, int npix, int part, int step,
+                                             int rx, int ry, int x_end, int y_end, float *acc) {
+    for (int j = part; j < npix; j += step) {
+        const int row = j >> 3, col = j & 7, h = col >> 2;
+        if (rx + col >= x_end || ry + row >= y_end) continue;
+        const float *v = pp[row * 4 + (col & 3)].v;
+        const float dx = g.x - ((float)(rx + col) + 0.5f), dy = g.y - ((float)(ry + row) + 0.5f);
+        const float sigma = sigma_ref<float>(g.a, g.b, g.c, dx, dy);
+        const float vis = __expf(-sigma);
+        const float alpha = fminf(clamp, g.o * vis);
+        if (sigma < 0.f || alpha < 1.f / 255.f) continue;
+        acc[7] += alpha * v[h];
+        acc[8] += alpha * v[2 + h];
+        acc[9] += alpha * v[4 + h];
+        float v_alpha = 0.f;
+        v_alpha += g.r * v[h];
+        v_alpha += g.g * v[2 + h];
+        v_alpha += g.bl * v[4 + h];
+        v_alpha += v[6 + h];
+        acc[10] += vis * v_alpha;
+        const float v_sigma = -alpha * v_alpha;
+        acc[4] += 0.5f * v_sigma * dx * dx;
+        acc[5] += v_sigma * dx * dy;
+        acc[6] += 0.5f * v_sigma * dy * dy;
+        const float gx = v_sigma * (g.a * dx + g.b * dy), gy = v_sigma * (g.b * dx + g.c * dy);
+        acc[0] += gx;
+        acc[1] += gy;
+        acc[2] += fabsf(gx);
+        acc[3] += fabsf(gy);
     }
 }
 
@@ -1432,7 +1501,12 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t phase) {
 // Against 8x4 regions a Gaussian meets fewer regions, so the per-pair costs —
 // the warps' region tests, the per-round set-up, the lane-group reduction and
 // the atomics — are paid fewer times, for more pixel evaluations per pair.
-template <typename T, bool GA, bool LEAN, bool ABS = false, int RR = 4>
+// GEN (with ABS): opacities and a wsum cotangent in the pair walk, where an
+// opacity costs a product and a multiply-add a pixel; bound by the FMA pipe and
+// issue as the lean walk.  Records
+// without culling data (under TAME packing) and tiles with a cotangent above
+// kTameCot or non-finite take sum_pixels_skip.
+template <typename T, bool GA, bool LEAN, bool ABS = false, int RR = 4, bool GEN = false>
 __device__ __forceinline__ void bwd_tile(const TileCtx &tc, int tile,
                                          const int32_t *__restrict__ ids,
                                          const int2 *__restrict__ tile_bins,
@@ -1446,6 +1520,8 @@ __device__ __forceinline__ void bwd_tile(const TileCtx &tc, int tile,
     // float lean backward: pixel pairs in f32x2 arithmetic (lean_region_f2)
     constexpr bool kPairs = LEAN && !GA && LIG_RASTER_BWD_F2 && sizeof(T) == 4;
     static_assert(!ABS || kPairs, "the |v_xy| sums of the lean walk need its pair form");
+    static_assert(!GEN || ABS, "the general pair walk keeps the |v_xy| sums");
+    [[maybe_unused]] bool tame_cot = true;
     // records staged by bulk async copies (no register prefetch, no region
     // masks: the warps test the box and ellipse themselves)
     constexpr bool kBulk = kPairs && LIG_RASTER_BWD_BULK;
@@ -1502,7 +1578,7 @@ __device__ __forceinline__ void bwd_tile(const TileCtx &tc, int tile,
             R.pixel(w, lane, p2, lx, ly);
             const int gx = tx0 + lx, gy = ty0 + ly;
             const bool inside = lx < B && ly < B && gx < W && gy < H;
-            T v0 = (T)0, v1 = (T)0, v2 = (T)0, vw;
+            T v0 = (T)0, v1 = (T)0, v2 = (T)0, vw = (T)0;
             if (inside) cot.get(tc.poff + gy * W + gx, v0, v1, v2, vw);
             PixPair *e = reinterpret_cast<PixPair *>(smem_raw) + w * RR * 4 +
                          ((lane >> 3) + 4 * p2) * 4 + (lane & 3);
@@ -1510,6 +1586,10 @@ __device__ __forceinline__ void bwd_tile(const TileCtx &tc, int tile,
             e->v[h] = v0;
             e->v[2 + h] = v1;
             e->v[4 + h] = v2;
+            if constexpr (GEN) {
+                e->v[6 + h] = vw;
+                tame_cot = tame_cot && tame_cotangent(v0, v1, v2, vw);
+            }
         }
     } else {
         int lx, ly;
@@ -1540,6 +1620,10 @@ __device__ __forceinline__ void bwd_tile(const TileCtx &tc, int tile,
             e->v[h] = c.vo0;
             e->v[2 + h] = c.vo1;
             e->v[4 + h] = c.vo2;
+            if constexpr (GEN) {
+                e->v[6 + h] = c.vw;
+                tame_cot = tame_cotangent(c.vo0, c.vo1, c.vo2, c.vw);
+            }
         } else {
             s_pix[tid] = c;
         }
@@ -1560,6 +1644,8 @@ __device__ __forceinline__ void bwd_tile(const TileCtx &tc, int tile,
             pre = recs[pre_id];
         }
     }
+    [[maybe_unused]] bool wild = false;
+    if constexpr (GEN) wild = __syncthreads_or(!tame_cot);
     for (int base = range.x; base < end; base += nt) {
         const int cnt = min(nt, end - base);
         if constexpr (kBulk) {
@@ -1638,6 +1724,7 @@ __device__ __forceinline__ void bwd_tile(const TileCtx &tc, int tile,
 #pragma unroll
             for (int q = 0; q < 11; ++q) acc[q] = 0;
             bool touched = false;
+            [[maybe_unused]] bool direct = false;  // acc holds gradients, not moments
             if constexpr (kPairs) {
                 // as below, two pixels per packed operation: lanes of a group
                 // take column pairs (1 / 2 / 4 lanes) or column pairs and row
@@ -1646,21 +1733,30 @@ __device__ __forceinline__ void bwd_tile(const TileCtx &tc, int tile,
                 const float px0 = (float)(tx0 + (w % R.nbx) * 8) + 0.5f;
                 const float py0 = (float)(ty0 + (w / R.nbx) * kRows) + 0.5f;
                 const PixPair *pp = reinterpret_cast<const PixPair *>(smem_raw) + w * kRows * 4;
-                if (act && RR > 4) {
+                if constexpr (GEN) direct = act && (wild || !(g.wx >= (T)0));
+                if (GEN && direct) {
+                    float t[11] = {};
+                    const int rx = tx0 + (w % R.nbx) * 8, ry = ty0 + (w / R.nbx) * kRows;
+                    sum_pixels_skip(reinterpret_cast<const Rec<float> &>(s_rec[slot]), clamp, pp,
+                                    kRows * 8, part, jstep, rx, ry, min(W, tx0 + B),
+                                    min(H, ty0 + B), t);
+#pragma unroll
+                    for (int q = 0; q < 11; ++q) acc[q] = t[q];
+                } else if (act && RR > 4) {
                     // the region in blocks of four rows (8 lanes: one half each)
                     constexpr int NB = RR / 4;
                     switch (lsplit) {
                     case 0:
-                        lean_region_f2<4, 1, 4, ABS, NB>(g, clamp, pp, 0, 0, px0, py0, acc);
+                        lean_region_f2<4, 1, 4, ABS, NB, GEN>(g, clamp, pp, 0, 0, px0, py0, acc);
                         break;
                     case 1:
-                        lean_region_f2<2, 2, 4, ABS, NB>(g, clamp, pp, part, 0, px0, py0, acc);
+                        lean_region_f2<2, 2, 4, ABS, NB, GEN>(g, clamp, pp, part, 0, px0, py0, acc);
                         break;
                     case 2:
-                        lean_region_f2<1, 1, 4, ABS, NB>(g, clamp, pp, part, 0, px0, py0, acc);
+                        lean_region_f2<1, 1, 4, ABS, NB, GEN>(g, clamp, pp, part, 0, px0, py0, acc);
                         break;
                     default:
-                        lean_region_f2<1, 1, 4, ABS, NB / 2>(g, clamp, pp, part & 3,
+                        lean_region_f2<1, 1, 4, ABS, NB / 2, GEN>(g, clamp, pp, part & 3,
                                                              (RR / 2) * (part >> 2), px0, py0,
                                                              acc);
                         break;
@@ -1668,16 +1764,16 @@ __device__ __forceinline__ void bwd_tile(const TileCtx &tc, int tile,
                 } else if (act) {
                     switch (lsplit) {
                     case 0:
-                        lean_region_f2<4, 1, 4, ABS>(g, clamp, pp, 0, 0, px0, py0, acc);
+                        lean_region_f2<4, 1, 4, ABS, 1, GEN>(g, clamp, pp, 0, 0, px0, py0, acc);
                         break;
                     case 1:
-                        lean_region_f2<2, 2, 4, ABS>(g, clamp, pp, part, 0, px0, py0, acc);
+                        lean_region_f2<2, 2, 4, ABS, 1, GEN>(g, clamp, pp, part, 0, px0, py0, acc);
                         break;
                     case 2:
-                        lean_region_f2<1, 1, 4, ABS>(g, clamp, pp, part, 0, px0, py0, acc);
+                        lean_region_f2<1, 1, 4, ABS, 1, GEN>(g, clamp, pp, part, 0, px0, py0, acc);
                         break;
                     default:
-                        lean_region_f2<1, 1, 2, ABS>(g, clamp, pp, part & 3, 2 * (part >> 2),
+                        lean_region_f2<1, 1, 2, ABS, 1, GEN>(g, clamp, pp, part & 3, 2 * (part >> 2),
                                                      px0, py0, acc);
                         break;
                     }
@@ -1789,13 +1885,13 @@ __device__ __forceinline__ void bwd_tile(const TileCtx &tc, int tile,
             for (int o = 1; o < (1 << lsplit); o <<= 1) {  // combine the lane group
 #pragma unroll
                 for (int q = 0; q < 11; ++q) {
-                    if (LEAN && (q == 10 || (!ABS && (q == 2 || q == 3)))) continue;
+                    if (LEAN && ((q == 10 && !GEN) || (!ABS && (q == 2 || q == 3)))) continue;
                     acc[q] += __shfl_xor_sync(FULL, acc[q], o);
                 }
                 touched = __shfl_xor_sync(FULL, (int)touched, o) || touched;
             }
             if (touched && part == 0) {
-                if constexpr (LEAN && !GA) {
+                if (LEAN && !GA && !direct) {
                     // v_xy = (a Sx + b Sy, b Sx + c Sy); v_conic = (Sxx/2, Sxy, Syy/2)
                     const T sx = acc[0], sy = acc[1];
                     acc[0] = g.a * sx + g.b * sy;
@@ -1808,11 +1904,11 @@ __device__ __forceinline__ void bwd_tile(const TileCtx &tc, int tile,
                     acc[3] = M::abs_(acc[1]);
                 }
                 if constexpr (LEAN && ABS) {
-                    // the general [N][12] layout, no opacity gradient
+                    // the general [N][12] layout
                     float4 *d4 = reinterpret_cast<float4 *>(packed + (size_t)s_ids[slot] * 12);
                     atomicAdd(d4, make_float4(acc[0], acc[1], acc[2], acc[3]));
                     atomicAdd(d4 + 1, make_float4(acc[4], acc[5], acc[6], acc[7]));
-                    atomicAdd(d4 + 2, make_float4(acc[8], acc[9], 0.f, 0.f));
+                    atomicAdd(d4 + 2, make_float4(acc[8], acc[9], GEN ? acc[10] : 0.f, 0.f));
                 } else if constexpr (LEAN) {
                     // [xy, conic, rgb]
                     T *dst = packed + (size_t)s_ids[slot] * 8;
@@ -1843,7 +1939,8 @@ __device__ __forceinline__ void bwd_tile(const TileCtx &tc, int tile,
     }
 }
 
-template <typename T, bool GA, bool LEAN, int MAXT, int MINB, bool ABS = false, int RR = 4>
+template <typename T, bool GA, bool LEAN, int MAXT, int MINB, bool ABS = false, int RR = 4,
+          bool GEN = false>
 __global__ void __launch_bounds__(MAXT, MINB)
 raster_bwd_kernel(const BatchGeo geo, const int32_t *__restrict__ cum, int *work,
                   const int32_t *__restrict__ ids, const int2 *__restrict__ tile_bins,
@@ -1866,8 +1963,8 @@ raster_bwd_kernel(const BatchGeo geo, const int32_t *__restrict__ cum, int *work
     for (int tile = next_tile(work, s_slot, true); tile < n_tiles;
          tile = next_tile(work, s_slot, false)) {
         const TileCtx tc = tile_ctx(geo, cum, d_total, tile);
-        bwd_tile<T, GA, LEAN, ABS, RR>(tc, tile, ids, tile_bins, recs, final_idx, cot, v_dx, v_dy,
-                                   v_dxy, clamp, packed, s_end, bar, phase);
+        bwd_tile<T, GA, LEAN, ABS, RR, GEN>(tc, tile, ids, tile_bins, recs, final_idx, cot, v_dx,
+                                            v_dy, v_dxy, clamp, packed, s_end, bar, phase);
     }
 }
 
@@ -1898,8 +1995,6 @@ raster_bwd_kernel(const BatchGeo geo, const int32_t *__restrict__ cum, int *work
 // 61% of the issue slots).  2047x1535 / 190k Gaussians: 518 us, against 1171
 // for the scalar walk over the expanded formulas; 512^2 / 50k with opacities:
 // 67 against 131.
-constexpr float kTameCot = 1e12f;  // larger (or non-finite) cotangents: the skipping walk
-
 struct alignas(16) GaPix {  // pixels (row, c) and (row, c + W/2)
     float v[12][2];         // plane-major: V0.rgb, V1.rgb, V2.rgb, V3.rgb
     float vw[2];
@@ -2461,8 +2556,10 @@ int raster_bwd(const BatchGeo &geo, TileWalk walk, const int32_t *ids, const int
     // float gradient-aware: 16x16 and 8x8 tiles, whose reference warps are
     // blocks of pixels
     const bool ga_pairs = ga && sizeof(T) == 4 && cot.v_img && (geo.B == 16 || geo.B == 8);
+    // float sum backward with opacities or a wsum cotangent: the pair walk too
+    const bool gen = !ga && !lean && !lean_abs && sizeof(T) == 4;
     // records, and the packed gradients cleared in the same pass
-    int rc = pack<T>(n, xys, con, col, op, ws, goff, s, false, packed, stride, ga_pairs);
+    int rc = pack<T>(n, xys, con, col, op, ws, goff, s, false, packed, stride, ga_pairs || gen);
     if (rc) return rc;
     const T cl = (T)(clamp > 0 ? clamp : (ga ? 0.999 : 0.99));
     Grads<T> g{(T *)v_xy, (T *)v_abs, (T *)v_con, (T *)v_rgb, (T *)v_op};
@@ -2482,7 +2579,7 @@ int raster_bwd(const BatchGeo &geo, TileWalk walk, const int32_t *ids, const int
     const double density = (double)n / (double)geo.total_pixels();
     const int rr_auto = density <= LIG_RASTER_BWD_R16_MAX_DENSITY ? 16 : 8;
     const int rr = (LIG_RASTER_BWD_RROWS != 4 && sizeof(T) == 4 && LIG_RASTER_BWD_F2 &&
-                    (lean || lean_abs) && large && geo.B <= 16)
+                    !ga && large && geo.B <= 16)
                        ? (LIG_RASTER_BWD_RROWS ? LIG_RASTER_BWD_RROWS : rr_auto)
                        : 4;
     const int nt = 32 * Regions::make(ga ? 2 : (rr == 8 ? 1 : rr == 16 ? 3 : 0), geo.B).count;
@@ -2495,30 +2592,37 @@ int raster_bwd(const BatchGeo &geo, TileWalk walk, const int32_t *ids, const int
                        const T *, const T *, T, T *);
     const bool small = nt <= 256;
     constexpr bool kAbs = sizeof(T) == 4 && LIG_RASTER_BWD_F2;
-    K fn = ga ? (small ? raster_bwd_kernel<T, true, false, 256, LIG_RASTER_BWD_MINB>
-                       : raster_bwd_kernel<T, true, false, 1024, 1>)
-         : lean_abs ? (small ? (large ? raster_bwd_kernel<T, false, true, 256,
-                                                          LIG_RASTER_BWD_LEAN_MINB_LARGE, kAbs>
-                                      : raster_bwd_kernel<T, false, true, 256,
-                                                          LIG_RASTER_BWD_LEAN_MINB, kAbs>)
-                             : raster_bwd_kernel<T, false, true, 1024, 1, kAbs>)
-              : lean ? (small ? (geo.total_tiles() >= LIG_RASTER_BWD_LARGE_MIN_TILES
-                                     ? raster_bwd_kernel<T, false, true, 256,
-                                                         LIG_RASTER_BWD_LEAN_MINB_LARGE>
-                                     : raster_bwd_kernel<T, false, true, 256,
-                                                         LIG_RASTER_BWD_LEAN_MINB>)
-                              : raster_bwd_kernel<T, false, true, 1024, 1>)
-                     : (small ? raster_bwd_kernel<T, false, false, 256, LIG_RASTER_BWD_MINB>
-                              : raster_bwd_kernel<T, false, false, 1024, 1>);
+    constexpr int kMin = LIG_RASTER_BWD_LEAN_MINB, kMinL = LIG_RASTER_BWD_LEAN_MINB_LARGE;
+    K fn;
+    if (ga) {
+        fn = small ? raster_bwd_kernel<T, true, false, 256, LIG_RASTER_BWD_MINB>
+                   : raster_bwd_kernel<T, true, false, 1024, 1>;
+    } else if (lean) {
+        fn = !small  ? raster_bwd_kernel<T, false, true, 1024, 1>
+             : large ? raster_bwd_kernel<T, false, true, 256, kMinL>
+                     : raster_bwd_kernel<T, false, true, 256, kMin>;
+    } else if constexpr (kAbs) {
+        if (lean_abs)
+            fn = !small  ? raster_bwd_kernel<T, false, true, 1024, 1, true>
+                 : large ? raster_bwd_kernel<T, false, true, 256, kMinL, true>
+                         : raster_bwd_kernel<T, false, true, 256, kMin, true>;
+        else
+            fn = !small  ? raster_bwd_kernel<T, false, true, 1024, 1, true, 4, true>
+                         : raster_bwd_kernel<T, false, true, 256, LIG_RASTER_GEN_MINB, true, 4, true>;
+    } else {
+        fn = small ? raster_bwd_kernel<T, false, false, 256, LIG_RASTER_BWD_MINB>
+                   : raster_bwd_kernel<T, false, false, 1024, 1>;
+    }
     if constexpr (kAbs) {
+        constexpr int M8 = LIG_RASTER_BWD_RROWS_MINB, M16 = LIG_RASTER_BWD_R16_MINB;
         if (rr == 8)
-            fn = lean_abs ? raster_bwd_kernel<T, false, true, 128, LIG_RASTER_BWD_RROWS_MINB, true, 8>
-                          : raster_bwd_kernel<T, false, true, 128, LIG_RASTER_BWD_RROWS_MINB, false,
-                                              8>;
+            fn = gen        ? raster_bwd_kernel<T, false, true, 128, LIG_RASTER_GEN_R8_MINB, true, 8, true>
+                 : lean_abs ? raster_bwd_kernel<T, false, true, 128, M8, true, 8>
+                            : raster_bwd_kernel<T, false, true, 128, M8, false, 8>;
         else if (rr == 16)
-            fn = lean_abs ? raster_bwd_kernel<T, false, true, 64, LIG_RASTER_BWD_R16_MINB, true, 16>
-                          : raster_bwd_kernel<T, false, true, 64, LIG_RASTER_BWD_R16_MINB, false,
-                                              16>;
+            fn = gen        ? raster_bwd_kernel<T, false, true, 64, LIG_RASTER_GEN_R16_MINB, true, 16, true>
+                 : lean_abs ? raster_bwd_kernel<T, false, true, 64, M16, true, 16>
+                            : raster_bwd_kernel<T, false, true, 64, M16, false, 16>;
     }
     if (!set_dyn_smem((const void *)fn, sm)) return LIG_ERR_LAUNCH;
     int grid = geo.total_tiles();
