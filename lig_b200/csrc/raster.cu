@@ -2444,7 +2444,9 @@ int raster_fwd(const BatchGeo &geo, TileWalk walk, const int32_t *ids, const int
             return raster_fwd_ga(geo, walk, ids, bins, d_total, ws, op != nullptr, (float *)img,
                                  (float *)wsum, (float *)dx, (float *)dy, (float *)dxy, fin, s);
     }
-    const bool ppl4 = !ga && geo.total_tiles() >= LIG_RASTER_PPL4_MIN_TILES;
+    // (tiles of up to 8 rows would leave half of an 8x16 region outside: 8x8
+    // tiles at 2048^2 / 150k take 126 us with two pixels a lane, 190 with four)
+    const bool ppl4 = !ga && geo.B > 8 && geo.total_tiles() >= LIG_RASTER_PPL4_MIN_TILES;
     const bool ppl2 = !ga && !ppl4 && geo.total_tiles() >= LIG_RASTER_PPL2_MIN_TILES;
     const int nt = 32 * Regions::make(ppl4 ? 3 : (ppl2 ? 1 : 0), geo.B).count;
     const size_t sm = (size_t)nt * (sizeof(Rec<T>) + sizeof(uint32_t));
@@ -2575,9 +2577,11 @@ int raster_bwd(const BatchGeo &geo, TileWalk walk, const int32_t *ids, const int
         }
     }
     const bool large = geo.total_tiles() >= LIG_RASTER_BWD_LARGE_MIN_TILES;
-    // the float lean walks of large images: 8x8 regions (tiles up to 16x16)
+    // the float pair walks of large images: taller regions (tiles up to 16x16)
     const double density = (double)n / (double)geo.total_pixels();
-    const int rr_auto = density <= LIG_RASTER_BWD_R16_MAX_DENSITY ? 16 : 8;
+    // (8x8 tiles fill half of an 8x16 region: 2048^2 / 150k 185 us with 8x8
+    // regions, 275 with 8x16)
+    const int rr_auto = density <= LIG_RASTER_BWD_R16_MAX_DENSITY && geo.B > 8 ? 16 : 8;
     const int rr = (LIG_RASTER_BWD_RROWS != 4 && sizeof(T) == 4 && LIG_RASTER_BWD_F2 &&
                     !ga && large && geo.B <= 16)
                        ? (LIG_RASTER_BWD_RROWS ? LIG_RASTER_BWD_RROWS : rr_auto)
