@@ -7,10 +7,12 @@
 // runs without a host round trip (the reference reads it back with .item(),
 // gsplat2d/gsplat2d/utils.py:66).
 //
-// Ordering (default, LIG_BIN_SCATTER): per-tile counters, their exclusive
-// scan, an atomic scatter of every slot into its tile's range and a per-tile
-// sort by Gaussian index (see "scatter binning" below); workspace: two
-// counters per tile, the scan state and the long-tile list.  Alternative kept for comparison: keys are 32-bit tile
+// Ordering (default, LIG_BIN_SCATTER): per-tile counters, their scan, a scatter
+// of every slot into its tile's range and a per-tile sort by Gaussian index —
+// in one CTA for small problems, on shared-memory counters while the tiles fit
+// them, on global atomics beyond (see "scatter binning" and the two sections
+// after it); workspace: two counters per tile, the scan state, the long-tile
+// list and, for the shared counters, their histogram.  Alternative kept for comparison: keys are 32-bit tile
 // ids (the reference's int64 (tile << 32) | depth keys carry depth 0, so only
 // ceil(log2 T) bits hold information) sorted by a stable LSD radix sort over
 // exactly those bits with <= 10-bit digits, then tile ranges from the
@@ -119,7 +121,8 @@ scan_kernel(const uint32_t *__restrict__ in, int n, uint32_t *__restrict__ out, 
     __shared__ uint32_t s_warp[32];
     __shared__ uint32_t s_tile, s_prefix;
     __shared__ int s_ok;
-    if (threadIdx.x == 0) s_tile = atomicAdd(ticket, 1u);
+    const bool alone = gridDim.x == 1;  // one CTA: no look-back, no state
+    if (threadIdx.x == 0) s_tile = alone ? 0u : atomicAdd(ticket, 1u);
     __syncthreads();
     const int tile = (int)s_tile;
     const int64_t base = (int64_t)tile * kScanTile + (int64_t)threadIdx.x * kScanItems;
@@ -148,7 +151,7 @@ scan_kernel(const uint32_t *__restrict__ in, int n, uint32_t *__restrict__ out, 
         uint32_t excl = 0;
         bool ok = true;
         if (tile == 0) {
-            if (threadIdx.x == 0) st_relaxed_u64(&state[0], kScanFlagPre | total);
+            if (threadIdx.x == 0 && !alone) st_relaxed_u64(&state[0], kScanFlagPre | total);
         } else {
             if (threadIdx.x == 0) st_relaxed_u64(&state[tile], kScanFlagAgg | total);
             ok = scan_look_back(state, tile, excl);
@@ -211,7 +214,8 @@ inline int device_scan(const uint32_t *in, uint32_t *out, int n, bool inclusive,
         return LIG_OK;
     }
     const int nb = scan_blocks(n);
-    if (!zeroed) cudaMemsetAsync(state, 0, sizeof(uint64_t) * scan_state_words(n), s);
+    if (!zeroed && nb > 1)
+        cudaMemsetAsync(state, 0, sizeof(uint64_t) * scan_state_words(n), s);
     scan_kernel<<<nb, kScanThreads, 0, s>>>(in, n, out, inclusive, total_out, state,
                                             reinterpret_cast<uint32_t *>(state + nb));
     note_launches(1);
@@ -254,42 +258,50 @@ struct SlotWarp {
     uint32_t base, magic;
 };
 
+// g0: the warp's first Gaussian; n: end of its range.  False when the warp has
+// no slots (a view's Gaussians are mostly outside it: those cost one load).
 template <typename T>
-__device__ __forceinline__ bool slot_warp(int n, const T *__restrict__ xys,
+__device__ __forceinline__ bool slot_warp(int64_t g0, int n, const T *__restrict__ xys,
                                           const T *__restrict__ extents,
                                           const int32_t *__restrict__ cum, const BatchGeo &geo,
                                           int32_t *__restrict__ status, SlotWarp &sw) {
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
-    sw.g0 = (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32;
-    if (sw.g0 >= n) return false;
-    const int g = (int)(sw.g0 + lane);
-    int cnt = 0, start = 0;
+    sw.g0 = g0;
+    if (g0 >= n) return false;
+    const int g = (int)(g0 + lane);
+    const int last = g < n ? cum[g] : 0;
+    int start = __shfl_up_sync(FULL, last, 1);
+    if (lane == 0) start = g0 > 0 ? cum[g0 - 1] : 0;
+    const int cnt = g < n ? last - start : 0;
+    if (!__any_sync(FULL, cnt != 0)) return false;
     sw.bw = 1;
     sw.stride = -1;
     sw.base = 0;
     sw.magic = 0;
     if (g < n) {
-        const int im = geo.image_of_gauss(g);
+        // the image of the warp's first Gaussian, then this lane's
+        int im = geo.image_of_gauss((int)g0);
+        while (im + 1 < geo.n_img && g >= geo.g_off[im + 1]) ++im;
         const int tbx = geo.tbx[im];
         sw.base = (uint32_t)geo.tile_off[im];
-        const int prev = g > 0 ? cum[g - 1] : 0;
-        start = prev;
-        cnt = cum[g] - prev;
-        const T ex = extents[2 * g], ey = extents[2 * g + 1];
-        if (!(ex <= (T)0 || ey <= (T)0) && cnt > 0) {
-            int x0, y0, x1, y1;
-            tile_bbox(xys[2 * g], xys[2 * g + 1], ex, ey, tbx, geo.tby(im), geo.B, x0, y0, x1, y1);
-            const int w = x1 - x0, h = y1 - y0;
-            if (w <= 0 || w * h != cnt) {
-                // inconsistent inputs: emit phantoms (in range) and flag it
-                if (status) atomicOr(status, LIG_STATUS_BADBOX);
-            } else {
-                sw.bw = w;
-                sw.stride = tbx - w;
-                sw.base += (uint32_t)y0 * (uint32_t)tbx + (uint32_t)x0;
-                if (w > 1 && (uint64_t)cnt * (uint64_t)w <= 0xffffffffull)
-                    sw.magic = 0xffffffffu / (uint32_t)w + 1u;
+        if (cnt > 0) {
+            const T ex = extents[2 * g], ey = extents[2 * g + 1];
+            if (!(ex <= (T)0 || ey <= (T)0)) {
+                int x0, y0, x1, y1;
+                tile_bbox(xys[2 * g], xys[2 * g + 1], ex, ey, tbx, geo.tby(im), geo.B, x0, y0, x1,
+                          y1);
+                const int w = x1 - x0, h = y1 - y0;
+                if (w <= 0 || w * h != cnt) {
+                    // inconsistent inputs: emit phantoms (in range) and flag it
+                    if (status) atomicOr(status, LIG_STATUS_BADBOX);
+                } else {
+                    sw.bw = w;
+                    sw.stride = tbx - w;
+                    sw.base += (uint32_t)y0 * (uint32_t)tbx + (uint32_t)x0;
+                    if (w > 1 && (uint64_t)cnt * (uint64_t)w <= 0xffffffffull)
+                        sw.magic = 0xffffffffu / (uint32_t)w + 1u;
+                }
             }
         }
     }
@@ -304,6 +316,10 @@ __device__ __forceinline__ bool slot_warp(int n, const T *__restrict__ xys,
     sw.excl = incl - cnt;
     sw.slot_base = start - sw.excl;
     return true;
+}
+
+__device__ __forceinline__ int64_t warp_first_gauss() {  // one warp per 32 Gaussians
+    return (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32;
 }
 
 // Flattened slot sl of the warp (all lanes call it together): false when sl
@@ -345,7 +361,7 @@ __device__ __forceinline__ void for_each_slot(int n, const T *__restrict__ xys,
                                               const BatchGeo &geo, int capacity,
                                               int32_t *__restrict__ status, F f) {
     SlotWarp sw;
-    if (!slot_warp<T>(n, xys, extents, cum, geo, status, sw)) return;
+    if (!slot_warp<T>(warp_first_gauss(), n, xys, extents, cum, geo, status, sw)) return;
     const int lane = threadIdx.x & 31;
     bool overflow = false;
     for (int s0 = 0; s0 < sw.total; s0 += 32) {
@@ -591,6 +607,12 @@ __global__ void flag_overflow_kernel(const int32_t *d_total, int capacity, int32
 #ifndef LIG_SORT_LONG_CTAS_PER_SM
 #define LIG_SORT_LONG_CTAS_PER_SM 8  // CTAs per SM of the long-tile sort (one tile per CTA at a time)
 #endif
+#ifndef LIG_BIN_HIST_RUN
+// Gaussians per CTA of the shared-counter binning (at least).  512^2 / 50k:
+// count and scatter 4.5 + 4.7 us with 512, 4.7 + 5.0 with 256, 6.4 + 7.6 with
+// 1024, 9.3 + 11.6 with 2048 (global atomics: 10.7 + 12.5).
+#define LIG_BIN_HIST_RUN 512
+#endif
 #ifndef LIG_SORT_REG512
 #define LIG_SORT_REG512 1  // tiles of 257..512 entries sorted by a warp in registers
 #endif
@@ -629,7 +651,7 @@ __global__ void tile_scatter_kernel(int n, const T *__restrict__ xys, const T *_
                                     int64_t *__restrict__ keys64, int32_t *__restrict__ gids) {
     constexpr int K = LIG_BIN_SCATTER_ILP;
     SlotWarp sw;
-    if (!slot_warp<T>(n, xys, ext, cum, geo, nullptr, sw)) return;
+    if (!slot_warp<T>(warp_first_gauss(), n, xys, ext, cum, geo, nullptr, sw)) return;
     const int lane = threadIdx.x & 31;
     for (int s0 = 0; s0 < sw.total; s0 += 32 * K) {
         int sl[K];
@@ -711,6 +733,20 @@ __device__ __forceinline__ void sort_segment_regs(uint32_t *seg, int L, int32_t 
     }
 }
 
+// One tile by a warp in registers; false when it is too long.
+__device__ __forceinline__ bool sort_tile_warp(uint32_t *seg, int L, int32_t *dst,
+                                               const BatchGeo &geo) {
+    if (L <= 32) sort_segment_regs<1>(seg, L, dst, geo);
+    else if (L <= 64) sort_segment_regs<2>(seg, L, dst, geo);
+    else if (L <= 128) sort_segment_regs<4>(seg, L, dst, geo);
+    else if (L <= 256) sort_segment_regs<8>(seg, L, dst, geo);
+#if LIG_SORT_REG512
+    else if (L <= 512) sort_segment_regs<16>(seg, L, dst, geo);
+#endif
+    else return false;
+    return true;
+}
+
 // 4. one warp per tile: sort its entries (from `vals`, written to `ids` as
 // Gaussian ids), write tile_bins ((0, 0) for an empty tile, as the
 // reference's zero-initialised edges) and, when asked, the sorted 64-bit
@@ -740,14 +776,8 @@ tile_sort_kernel(BatchGeo geo, const uint32_t *__restrict__ tcount,
             for (int i = lane; i < L; i += 32) isect_sorted[a + i] = (int64_t)t << 32;
         uint32_t *seg = vals + a;
         int32_t *dst = ids + a;
-        if (L <= 32) sort_segment_regs<1>(seg, L, dst, geo);
-        else if (L <= 64) sort_segment_regs<2>(seg, L, dst, geo);
-        else if (L <= 128) sort_segment_regs<4>(seg, L, dst, geo);
-        else if (L <= 256) sort_segment_regs<8>(seg, L, dst, geo);
-#if LIG_SORT_REG512
-        else if (L <= 512) sort_segment_regs<16>(seg, L, dst, geo);
-#endif
-        else if (lane == 0) long_list[1 + atomicAdd(long_list, 1)] = t;
+        if (!sort_tile_warp(seg, L, dst, geo) && lane == 0)
+            long_list[1 + atomicAdd(long_list, 1)] = t;
     }
 }
 
@@ -761,6 +791,44 @@ tile_sort_kernel(BatchGeo geo, const uint32_t *__restrict__ tcount,
 // padding up to a power of two (conceptually the largest key, always at the
 // higher index of a comparator) never moves and is not stored: every
 // comparator that reaches past the segment is skipped.
+__device__ __forceinline__ void sort_tile_cta(int a, int L, uint32_t *__restrict__ vals,
+                                              int32_t *__restrict__ ids, const BatchGeo &geo,
+                                              uint32_t *s_buf) {
+    int P = 1;
+    while (P < L) P <<= 1;
+    const bool smem = P <= kSegSmem;
+    uint32_t *seg = smem ? s_buf : vals + a;
+    if (smem)
+        for (int i = threadIdx.x; i < P; i += blockDim.x)
+            s_buf[i] = i < L ? vals[a + i] : 0xffffffffu;
+    __syncthreads();
+    const int n = smem ? P : L;  // elements that exist
+    for (int size = 2; size <= P; size <<= 1) {
+        for (int j = size >> 1; j > 0; j >>= 1) {
+            for (int p = threadIdx.x; p < P / 2; p += blockDim.x) {
+                int i, k;
+                if (j == size >> 1) {  // mirrored pair of the block
+                    const int blk = p / j, o = p - blk * j;
+                    i = blk * size + o;
+                    k = blk * size + size - 1 - o;
+                } else {  // half-cleaner at distance j
+                    i = 2 * p - (p & (j - 1));
+                    k = i + j;
+                }
+                if (k >= n) continue;
+                const uint32_t x = seg[i], y = seg[k];
+                if (x > y) {
+                    seg[i] = y;
+                    seg[k] = x;
+                }
+            }
+            __syncthreads();
+        }
+    }
+    for (int i = threadIdx.x; i < L; i += blockDim.x) ids[a + i] = slot_id(seg[i], geo);
+    __syncthreads();
+}
+
 constexpr int kLongThreads = 256;
 __global__ void __launch_bounds__(kLongThreads)
 tile_sort_long_kernel(BatchGeo geo, const uint32_t *__restrict__ tcount,
@@ -773,40 +841,200 @@ tile_sort_long_kernel(BatchGeo geo, const uint32_t *__restrict__ tcount,
         const int t = long_list[1 + q];
         const int a = (int)min((uint32_t)capacity, tend[t] - tcount[t]);
         const int b = (int)min((uint32_t)capacity, tend[t]);
-        const int L = b - a;
-        int P = 1;
-        while (P < L) P <<= 1;
-        const bool smem = P <= kSegSmem;
-        uint32_t *seg = smem ? s_buf : vals + a;
-        if (smem)
-            for (int i = threadIdx.x; i < P; i += blockDim.x)
-                s_buf[i] = i < L ? vals[a + i] : 0xffffffffu;
-        __syncthreads();
-        const int n = smem ? P : L;  // elements that exist
-        for (int size = 2; size <= P; size <<= 1) {
-            for (int j = size >> 1; j > 0; j >>= 1) {
-                for (int p = threadIdx.x; p < P / 2; p += blockDim.x) {
-                    int i, k;
-                    if (j == size >> 1) {  // mirrored pair of the block
-                        const int blk = p / j, o = p - blk * j;
-                        i = blk * size + o;
-                        k = blk * size + size - 1 - o;
-                    } else {  // half-cleaner at distance j
-                        i = 2 * p - (p & (j - 1));
-                        k = i + j;
-                    }
-                    if (k >= n) continue;
-                    const uint32_t x = seg[i], y = seg[k];
-                    if (x > y) {
-                        seg[i] = y;
-                        seg[k] = x;
-                    }
-                }
-                __syncthreads();
-            }
+        sort_tile_cta(a, b - a, vals, ids, geo, s_buf);
+    }
+}
+
+// ---------------------------------------------- binning on shared counters
+// While the tile counters fit an SM's shared memory (up to kHistMaxTiles), the
+// global atomics of count and scatter — what those kernels wait for: 6M slots
+// at 2048^2 / 1M Gaussians took 37 and 63 us, at any enumeration cost — become
+// shared-memory atomics.  CTA c of `parts` takes the c-th run of Gaussians:
+//   1. tile_hist_kernel: its slots' tile counts in shared memory, written as
+//      row c of hist [parts][tiles];
+//   2. hist_prefix_kernel: per tile the exclusive prefix over the rows (in
+//      place) and the tile's total;
+//   3. the inclusive scan of the totals gives every tile's end;
+//   4. hist_scatter_kernel: cursors (tile start + row prefix) in shared memory,
+//      one shared atomic per slot;
+// then the per-tile sort as above.  Count, prefix and scatter against global
+// atomics: 512^2 / 50k 11.5 us against 23, 16 images of 1.1M Gaussians 56
+// against 99, 2048^2 / 1M 88 against 100, eight views of 500k 139 against 236;
+// what is left is the enumeration and the scattered 4-byte stores.  Slots past the capacity are dropped by
+// position (outputs are incomplete then, and flagged).
+constexpr int kHistThreads = 1024;
+constexpr int kHistMaxTiles = 48 * 1024;  // 192 KB of counters
+constexpr int kHistTwoTiles = 24 * 1024;  // two CTAs' counters fit an SM up to here
+constexpr int kHistMaxParts = 2 * 148;
+
+// Rows of the histogram (CTAs): LIG_BIN_HIST_RUN Gaussians each, up to one per
+// SM; two per SM from kHistTwoMinPoints Gaussians on, where the second CTA's
+// warps hide more of the enumeration than the longer prefix costs (eight
+// views, 4M Gaussians / 17k tiles: 174 -> 139 us; 2048^2 / 1M: 87 -> 88).
+constexpr int kHistTwoMinPoints = 2000000;
+inline int hist_parts(int n, size_t tiles) {
+    const bool two = tiles <= kHistTwoTiles && n >= kHistTwoMinPoints;
+    return std::min(std::max(n / LIG_BIN_HIST_RUN, 1), two ? kHistMaxParts : kHistMaxParts / 2);
+}
+
+// f(slot, tile key, sort value) for every slot of Gaussians [g0, g1), by the
+// CTA's warps.
+template <typename T, typename F>
+__device__ __forceinline__ void for_each_slot_of_run(int g0, int g1, const T *__restrict__ xys,
+                                                     const T *__restrict__ ext,
+                                                     const int32_t *__restrict__ cum,
+                                                     const BatchGeo &geo,
+                                                     int32_t *__restrict__ status, F f) {
+    const int lane = threadIdx.x & 31;
+    for (int64_t g = g0 + (int)(threadIdx.x >> 5) * 32; g < g1; g += blockDim.x) {
+        SlotWarp sw;
+        if (!slot_warp<T>(g, g1, xys, ext, cum, geo, status, sw)) continue;
+        for (int s0 = 0; s0 < sw.total; s0 += 32) {
+            int slot;
+            uint32_t key, val;
+            if (slot_at(sw, s0 + lane, slot, key, val)) f(slot, key, val);
         }
-        for (int i = threadIdx.x; i < L; i += blockDim.x) ids[a + i] = slot_id(seg[i], geo);
-        __syncthreads();
+    }
+}
+
+__device__ __forceinline__ void run_of_part(int n, int &g0, int &g1) {
+    g0 = (int)((int64_t)n * blockIdx.x / gridDim.x);
+    g1 = (int)((int64_t)n * (blockIdx.x + 1) / gridDim.x);
+}
+
+// clear: words cleared for the later kernels (the scan's state, the long-tile
+// list's length)
+template <typename T>
+__global__ void __launch_bounds__(kHistThreads, 2)
+tile_hist_kernel(int n, int tiles, const T *__restrict__ xys, const T *__restrict__ ext,
+                 const int32_t *__restrict__ cum, const int32_t *d_total, BatchGeo geo,
+                 int capacity, uint32_t *__restrict__ hist, int32_t *__restrict__ status,
+                 uint32_t *__restrict__ clear, int n_clear) {
+    extern __shared__ uint32_t s_tile[];
+    if (blockIdx.x == 0) {
+        for (int i = threadIdx.x; i < n_clear; i += blockDim.x) clear[i] = 0;
+        if (threadIdx.x == 0 && *d_total > capacity) atomicOr(status, LIG_STATUS_OVERFLOW);
+    }
+    for (int t = threadIdx.x; t < tiles; t += blockDim.x) s_tile[t] = 0;
+    __syncthreads();
+    int g0, g1;
+    run_of_part(n, g0, g1);
+    for_each_slot_of_run<T>(g0, g1, xys, ext, cum, geo, status,
+                            [&](int, uint32_t key, uint32_t) { atomicAdd(&s_tile[key], 1u); });
+    __syncthreads();
+    uint32_t *row = hist + (size_t)blockIdx.x * tiles;
+    for (int t = threadIdx.x; t < tiles; t += blockDim.x) row[t] = s_tile[t];
+}
+
+// 32 tiles per CTA; warp y takes rows y K .. y K + K - 1 (32 K >= parts).
+template <int K>
+__global__ void __launch_bounds__(1024)
+hist_prefix_kernel(int tiles, int parts, uint32_t *__restrict__ hist,
+                   uint32_t *__restrict__ tcount) {
+    __shared__ uint32_t s[32][33];
+    const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+    const int t = blockIdx.x * 32 + x;
+    uint32_t v[K], sum = 0;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        const int c = y * K + k;
+        v[k] = c < parts && t < tiles ? hist[(size_t)c * tiles + t] : 0u;
+        sum += v[k];
+    }
+    s[y][x] = sum;
+    __syncthreads();
+    uint32_t incl = s[x][y];  // warp y: tile y of the CTA, lane = row group
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t u = __shfl_up_sync(0xffffffffu, incl, o);
+        if (x >= o) incl += u;
+    }
+    __syncthreads();
+    s[x][y] = incl;
+    __syncthreads();
+    uint32_t run = s[y][x] - sum;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        const int c = y * K + k;
+        if (c < parts && t < tiles) hist[(size_t)c * tiles + t] = run;
+        run += v[k];
+    }
+    if (y == 31 && t < tiles) tcount[t] = run;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kHistThreads, 2)
+hist_scatter_kernel(int n, int tiles, const T *__restrict__ xys, const T *__restrict__ ext,
+                    const int32_t *__restrict__ cum, BatchGeo geo, int capacity,
+                    const uint32_t *__restrict__ hist, const uint32_t *__restrict__ tcount,
+                    const uint32_t *__restrict__ tend, uint32_t *__restrict__ out) {
+    extern __shared__ uint32_t s_tile[];
+    const uint32_t *row = hist + (size_t)blockIdx.x * tiles;
+    for (int t = threadIdx.x; t < tiles; t += blockDim.x)
+        s_tile[t] = tend[t] - tcount[t] + row[t];
+    __syncthreads();
+    int g0, g1;
+    run_of_part(n, g0, g1);
+    for_each_slot_of_run<T>(g0, g1, xys, ext, cum, geo, nullptr,
+                            [&](int, uint32_t key, uint32_t val) {
+                                const uint32_t pos = atomicAdd(&s_tile[key], 1u);
+                                if (pos < (uint32_t)capacity) out[pos] = val;
+                            });
+}
+
+// ------------------------------------------------------- small binnings
+// Up to kSmallPoints Gaussians on kSmallTiles tiles with kSmallSlots slots: one
+// CTA does all of it — count, scan, scatter and the tiles' sorts — in one
+// launch.  A thumbnail's binning is eight dependent launches otherwise, whose
+// cost is their latency (64x80 / 400 Gaussians: 7.5 us against 17 and the
+// host's launches: the whole render 81 -> 64).  Beyond these sizes the one SM's throughput would count.
+constexpr int kSmallPoints = 2048, kSmallTiles = 1024, kSmallSlots = 8192;
+
+template <typename T>
+__global__ void __launch_bounds__(1024)
+bin_small_kernel(int n, int tiles, const T *__restrict__ xys, const T *__restrict__ ext,
+                 const int32_t *__restrict__ cum, const int32_t *d_total, BatchGeo geo,
+                 int capacity, uint32_t *__restrict__ vals, int32_t *__restrict__ ids,
+                 int2 *__restrict__ tile_bins, int32_t *__restrict__ status) {
+    __shared__ uint32_t s_cnt[kSmallTiles], s_cur[kSmallTiles], s_buf[kSegSmem], s_warp[32];
+    __shared__ int s_long[kSmallTiles], s_nlong;
+    const int tid = threadIdx.x, lane = tid & 31;
+    if (tid == 0) {
+        s_nlong = 0;
+        *status = *d_total > capacity ? LIG_STATUS_OVERFLOW : 0;
+    }
+    s_cnt[tid] = 0;
+    __syncthreads();
+    for_each_slot_of_run<T>(0, n, xys, ext, cum, geo, status,
+                            [&](int, uint32_t key, uint32_t) { atomicAdd(&s_cnt[key], 1u); });
+    __syncthreads();
+    const uint32_t c = s_cnt[tid];
+    uint32_t total;
+    const uint32_t first = block_incl_scan(c, total, s_warp) - c;
+    s_cur[tid] = first;
+    if (tid < tiles) {
+        const int a = (int)min((uint32_t)capacity, first), b = (int)min((uint32_t)capacity, first + c);
+        tile_bins[tid] = c ? make_int2(a, b) : make_int2(0, 0);
+    }
+    __syncthreads();
+    for_each_slot_of_run<T>(0, n, xys, ext, cum, geo, nullptr,
+                            [&](int, uint32_t key, uint32_t val) {
+                                const uint32_t pos = atomicAdd(&s_cur[key], 1u);
+                                if (pos < (uint32_t)capacity) vals[pos] = val;
+                            });
+    __syncthreads();  // the scattered values are read by other threads of this CTA
+    for (int t = tid >> 5; t < tiles; t += 32) {
+        const uint32_t e = s_cur[t];
+        const int a = (int)min((uint32_t)capacity, e - s_cnt[t]);
+        const int L = (int)min((uint32_t)capacity, e) - a;
+        if (L > 0 && !sort_tile_warp(vals + a, L, ids + a, geo) && lane == 0)
+            s_long[atomicAdd(&s_nlong, 1)] = t;
+    }
+    __syncthreads();
+    for (int q = 0; q < s_nlong; ++q) {
+        const int t = s_long[q];
+        const int a = (int)min((uint32_t)capacity, s_cur[t] - s_cnt[t]);
+        sort_tile_cta(a, (int)min((uint32_t)capacity, s_cur[t]) - a, vals, ids, geo, s_buf);
     }
 }
 
@@ -846,11 +1074,12 @@ inline BinPlan make_plan(int capacity, int num_tiles) {
 // (they start as the scan of the counts).  The first three are adjacent so
 // that one memset clears the counts, the scan state and the list length.
 // The sort keys are scattered into gid_sorted itself and sorted in place.
+// With shared counters: the same, and the histogram behind it.
 struct ScatterPlan {
-    size_t off_count, off_part, off_long, off_cursor, total;
+    size_t off_count, off_part, off_long, off_cursor, off_hist, total, total_hist;
 };
 
-inline ScatterPlan make_scatter_plan(int num_tiles) {
+inline ScatterPlan make_scatter_plan(int n, int num_tiles) {
     ScatterPlan p{};
     size_t t = (size_t)(num_tiles > 0 ? num_tiles : 1);
     size_t off = 0;
@@ -859,7 +1088,29 @@ inline ScatterPlan make_scatter_plan(int num_tiles) {
     p.off_long = off; off = align_up(off + 4 * (t + 1));
     p.off_cursor = off; off = align_up(off + 4 * t);
     p.total = off;
+    p.off_hist = off;
+    p.total_hist = t <= kHistMaxTiles ? align_up(off + 4 * t * hist_parts(n, t)) : off;
     return p;
+}
+
+// Opt a kernel into the shared memory of kHistMaxTiles counters, once per
+// device.
+template <typename T> bool hist_smem_opt_in() {
+    static std::mutex mu;
+    static bool done[128] = {};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 128) return false;
+    std::lock_guard<std::mutex> lock(mu);
+    if (!done[dev]) {
+        const int bytes = kHistMaxTiles * (int)sizeof(uint32_t);
+        if (cudaFuncSetAttribute(tile_hist_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 bytes) != cudaSuccess ||
+            cudaFuncSetAttribute(hist_scatter_kernel<T>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess)
+            return false;
+        done[dev] = true;
+    }
+    return true;
 }
 
 template <typename T>
@@ -869,13 +1120,23 @@ int run_bin_scatter(const BatchGeo &geo, const void *xys, const void *ext, const
                     int64_t *isect_sorted, int32_t *status, cudaStream_t s) {
     const int n = geo.total_points();
     const int T_ = geo.total_tiles();
-    ScatterPlan p = make_scatter_plan(T_);
+    ScatterPlan p = make_scatter_plan(n, T_);
     if (ws_bytes < p.total) return LIG_ERR_WORKSPACE;
     char *base = (char *)ws;
     uint32_t *tcount = (uint32_t *)(base + p.off_count);
     uint32_t *cursor = (uint32_t *)(base + p.off_cursor);
     uint64_t *part = (uint64_t *)(base + p.off_part);
     int32_t *long_list = (int32_t *)(base + p.off_long);
+    uint32_t *vals = (uint32_t *)gid_sorted;
+    if (n > 0 && n <= kSmallPoints && T_ <= kSmallTiles && capacity > 0 &&
+        capacity <= kSmallSlots && !isect && !isect_sorted) {
+        bin_small_kernel<T><<<1, 1024, 0, s>>>(n, T_, (const T *)xys, (const T *)ext, cum, d_total,
+                                               geo, capacity, vals, gid_sorted, (int2 *)tile_bins,
+                                               status);
+        note_launches(1);
+        LIG_LAUNCH_CHECK();
+        return LIG_OK;
+    }
     cudaMemsetAsync(status, 0, sizeof(int32_t), s);
     if (n == 0 || capacity == 0) {
         cudaMemsetAsync(tile_bins, 0, sizeof(int32_t) * 2 * (size_t)T_, s);
@@ -884,19 +1145,42 @@ int run_bin_scatter(const BatchGeo &geo, const void *xys, const void *ext, const
         LIG_LAUNCH_CHECK();
         return LIG_OK;
     }
-    // counts, scan state and the long-list length in one memset
-    cudaMemsetAsync(tcount, 0, p.off_long + sizeof(int32_t) - p.off_count, s);
-    const int warps = (n + 31) / 32;
-    const int eblocks = (warps * 32 + 255) / 256;
-    tile_count_kernel<T><<<eblocks, 256, 0, s>>>(n, (const T *)xys, (const T *)ext, cum, d_total,
-                                                 geo, capacity, tcount, status);
-    note_launches(1);
-    LIG_LAUNCH_CHECK();
-    int rc = device_scan(tcount, cursor, T_, false, part, nullptr, s, /*zeroed=*/true);
-    if (rc) return rc;
-    uint32_t *vals = (uint32_t *)gid_sorted;
-    tile_scatter_kernel<T><<<eblocks, 256, 0, s>>>(n, (const T *)xys, (const T *)ext, cum, geo,
-                                                   capacity, cursor, vals, isect, gids);
+    // shared counters while they fit (the emission-order outputs keep the
+    // slot-order kernels)
+    const bool hist_path = T_ <= kHistMaxTiles && !isect && ws_bytes >= p.total_hist;
+    if (hist_path) {
+        if (!hist_smem_opt_in<T>()) return LIG_ERR_LAUNCH;
+        uint32_t *hist = (uint32_t *)(base + p.off_hist);
+        const int parts = hist_parts(n, (size_t)T_);
+        const size_t sm = sizeof(uint32_t) * (size_t)T_;
+        const int n_clear = (int)((p.off_long + sizeof(int32_t) - p.off_part) / sizeof(uint32_t));
+        tile_hist_kernel<T><<<parts, kHistThreads, sm, s>>>(n, T_, (const T *)xys, (const T *)ext,
+                                                            cum, d_total, geo, capacity, hist,
+                                                            status, (uint32_t *)part, n_clear);
+        static_assert(kHistMaxParts <= 320, "rows of the histogram");
+        auto prefix = parts <= 160 ? hist_prefix_kernel<5> : hist_prefix_kernel<10>;
+        prefix<<<(T_ + 31) / 32, 1024, 0, s>>>(T_, parts, hist, tcount);
+        note_launches(2);
+        LIG_LAUNCH_CHECK();
+        int rc = device_scan(tcount, cursor, T_, true, part, nullptr, s, /*zeroed=*/true);
+        if (rc) return rc;
+        hist_scatter_kernel<T><<<parts, kHistThreads, sm, s>>>(n, T_, (const T *)xys,
+                                                               (const T *)ext, cum, geo, capacity,
+                                                               hist, tcount, cursor, vals);
+    } else {
+        // counts, scan state and the long-list length in one memset
+        cudaMemsetAsync(tcount, 0, p.off_long + sizeof(int32_t) - p.off_count, s);
+        const int warps = (n + 31) / 32;
+        const int eblocks = (warps * 32 + 255) / 256;
+        tile_count_kernel<T><<<eblocks, 256, 0, s>>>(n, (const T *)xys, (const T *)ext, cum,
+                                                     d_total, geo, capacity, tcount, status);
+        note_launches(1);
+        LIG_LAUNCH_CHECK();
+        int rc = device_scan(tcount, cursor, T_, false, part, nullptr, s, /*zeroed=*/true);
+        if (rc) return rc;
+        tile_scatter_kernel<T><<<eblocks, 256, 0, s>>>(n, (const T *)xys, (const T *)ext, cum, geo,
+                                                       capacity, cursor, vals, isect, gids);
+    }
     const int sort_blocks = (int)std::min<int64_t>(((int64_t)T_ + kSegWarps - 1) / kSegWarps,
                                                    148 * 32);
     tile_sort_kernel<<<sort_blocks, 32 * kSegWarps, 0, s>>>(geo, tcount, cursor, capacity, vals,
@@ -1024,8 +1308,7 @@ extern "C" int lig_cumsum_tiles(int n, const int32_t *counts, int32_t *cum, int3
 }
 
 extern "C" size_t lig_bin_workspace_bytes(int n, int capacity, int num_tiles) {
-    (void)n;
-    if (LIG_BIN_SCATTER) return make_scatter_plan(num_tiles).total;
+    if (LIG_BIN_SCATTER) return make_scatter_plan(n, num_tiles).total_hist;
     return make_plan(capacity, num_tiles).total;
 }
 
