@@ -4,7 +4,8 @@
 // Residual (train.py:113-126): resid = gt - up + 0.5, min-max normalised to
 // [0, 1]; the level's store_min / store_max are the min and max.  Two passes
 // over gt and up (the min/max reduction, then the normalised write) instead
-// of six elementwise / reduction launches; every value is computed with the
+// of six elementwise / reduction launches, vectorised (402 MB read at 4095x4093:
+// 75 us; 603 MB read and written, some of it from L2: 84, 129 before); every value is computed with the
 // same IEEE operations in the same order as the torch expression
 // ((gt - up) + 0.5, then (r - lo) / (hi - lo) with a correctly rounded
 // division), so the result is bit-identical.
@@ -16,12 +17,16 @@
 // clamp(render, 0, 1) * (hi - lo) - 0.5 + lo is added; the last level is
 // clamped to [0, 1].  One pass per level, no intermediate resized image.
 #include <cfloat>
+#include <type_traits>
 
 #include "common.cuh"
 
 namespace lig {
 
 constexpr int kLevelThreads = 256;
+// Elementwise passes: 6 CTAs per SM, 4 vectors in flight per thread (4095x4093:
+// minmax / normalise 75 / 84 us; 8 CTAs 75 / 87, 4 79 / 95, 2 in flight 74 / 99).
+constexpr int kLevelCtas = 6, kLevelUnroll = 4;
 
 __device__ __forceinline__ float atomic_min_f(float *a, float v) {
     // order-preserving int mapping of finite floats
@@ -51,17 +56,33 @@ __global__ void minmax_init_kernel(float *mm) {
     mm[1] = -FLT_MAX;
 }
 
+// Elements are taken four at a time where the arrays are 16-byte aligned (VEC;
+// the remainder, or everything otherwise, one at a time).
 // pass 1: min / max of gt - up + 0.5 (NaNs are ignored by the comparisons)
+template <bool VEC>
 __global__ void __launch_bounds__(kLevelThreads)
 resid_minmax_kernel(int64_t n, const float *__restrict__ gt, const float *__restrict__ up,
                     float *__restrict__ mm) {
     float lo = FLT_MAX, hi = -FLT_MAX;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const float r = __fadd_rn(__fsub_rn(gt[i], up[i]), 0.5f);
+    const int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t step = (int64_t)gridDim.x * blockDim.x;
+    auto take = [&](float a, float b) {
+        const float r = __fadd_rn(__fsub_rn(a, b), 0.5f);
         lo = fminf(lo, r);
         hi = fmaxf(hi, r);
+    };
+    const int64_t nv = VEC ? n / 4 : 0;
+    const float4 *g4 = reinterpret_cast<const float4 *>(gt);
+    const float4 *u4 = reinterpret_cast<const float4 *>(up);
+#pragma unroll kLevelUnroll
+    for (int64_t i = i0; i < nv; i += step) {
+        const float4 a = g4[i], b = u4[i];
+        take(a.x, b.x);
+        take(a.y, b.y);
+        take(a.z, b.z);
+        take(a.w, b.w);
     }
+    for (int64_t i = 4 * nv + i0; i < n; i += step) take(gt[i], up[i]);
 #pragma unroll
     for (int o = 16; o >= 1; o >>= 1) {
         lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
@@ -80,72 +101,144 @@ resid_minmax_kernel(int64_t n, const float *__restrict__ gt, const float *__rest
     }
 }
 
-// pass 2: (r - lo) / (hi - lo), correctly rounded
+// pass 2: (r - lo) / (hi - lo), correctly rounded.  Walks from the end, where
+// pass 1 stopped: up to the L2's size of the inputs is still there, and the
+// streaming stores leave it there.
+template <bool VEC>
 __global__ void __launch_bounds__(kLevelThreads)
 resid_normalise_kernel(int64_t n, const float *__restrict__ gt, const float *__restrict__ up,
                        const float *__restrict__ mm, float *__restrict__ out) {
     const float lo = mm[0], hi = mm[1];
     const float den = __fsub_rn(hi, lo);
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const float r = __fadd_rn(__fsub_rn(gt[i], up[i]), 0.5f);
-        out[i] = __fdiv_rn(__fsub_rn(r, lo), den);
+    const int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t step = (int64_t)gridDim.x * blockDim.x;
+    auto norm = [&](float a, float b) {
+        const float r = __fadd_rn(__fsub_rn(a, b), 0.5f);
+        return __fdiv_rn(__fsub_rn(r, lo), den);
+    };
+    const int64_t nv = VEC ? n / 4 : 0;
+    const float4 *g4 = reinterpret_cast<const float4 *>(gt);
+    const float4 *u4 = reinterpret_cast<const float4 *>(up);
+    float4 *o4 = reinterpret_cast<float4 *>(out);
+    for (int64_t i = 4 * nv + i0; i < n; i += step) out[i] = norm(gt[i], up[i]);
+#pragma unroll kLevelUnroll
+    for (int64_t i = nv - 1 - i0; i >= 0; i -= step) {
+        const float4 a = g4[i], b = u4[i];
+        __stcs(o4 + i, make_float4(norm(a.x, b.x), norm(a.y, b.y), norm(a.z, b.z),
+                                   norm(a.w, b.w)));
     }
 }
 
 // Compose one level: out = base + (clamp(render) * (hi - lo) - 0.5 + lo),
-// base = bilinear resize of prev [ph, pw, 3] to [H, W] (or prev itself when
-// the sizes agree), clamp_out: final clamp to [0, 1].
+// base = bilinear resize of prev [ph, pw, 3] to [H, W] (RESIZE), prev itself
+// when the sizes agree, or 0; clamp_out: final clamp to [0, 1].
+// A thread owns one value (column, channel) of a row — coalesced loads and
+// stores — and walks kComposeRows rows, kComposeBatch of them with all their
+// loads (the render's value and four taps of prev, which hit L1) on their way
+// together.  The rows' taps and weights come from a table the CTA fills once:
+// the float / integer conversions run at a quarter of the other operations'
+// rate and cost more than the memory traffic when every value makes its own.
+// Off: unsigned type of a byte offset into prev.
+// 4095x4093 from 2047x2046 (69 us of traffic): 92 us, against 115 with one
+// pixel a thread and a 64-bit division each, 131 with the conversions per value
+// and 146 with four flat values a thread.  Issue-bound (75% of the slots).
+constexpr int kComposeRows = 16, kComposeBatch = 4;  // 32 rows 95 us, batches of 2 / 8 98 / 104
+
+template <typename Off> struct RowTap {
+    Off a, b;        // byte offsets of the upper and lower row of prev
+    float ly0, ly1;  // their weights
+};
+
+template <bool RESIZE, typename Off>
 __global__ void __launch_bounds__(kLevelThreads)
 compose_kernel(int ph, int pw, const float *__restrict__ prev, int H, int W,
                const float *__restrict__ render, const float *__restrict__ mm, float lo_h,
                float hi_h, int clamp_render, int clamp_out, float *__restrict__ out) {
-    const int64_t np = (int64_t)H * W;
+    __shared__ RowTap<Off> s_row[kComposeRows];
+    const int64_t pitch = 3 * (int64_t)W;
+    const uint32_t q = blockIdx.x * kLevelThreads + threadIdx.x;
+    const int r0 = blockIdx.y * kComposeRows, nr = min(kComposeRows, H - r0);
+    // the half-pixel source index and weights written as the bilinear
+    // definition states them (src = s (d + 0.5) - 0.5, negative -> 0;
+    // lambda1 = src - floor, lambda0 = 1 - lambda1), so that the
+    // compiler contracts them as it does torch's upsample kernel
+    if (RESIZE && threadIdx.x < nr) {
+        const float sh = __fdiv_rn((float)ph, (float)H);
+        float ry = sh * ((float)(r0 + threadIdx.x) + 0.5f) - 0.5f;
+        ry = ry < 0.f ? 0.f : ry;
+        const int y0 = (int)ry, y1 = y0 + (y0 < ph - 1 ? 1 : 0);
+        const float ly1 = ry - (float)y0;
+        const Off p = (Off)pw * 12u;
+        s_row[threadIdx.x] = RowTap<Off>{(Off)y0 * p, (Off)y1 * p, 1.f - ly1, ly1};
+    }
     const float lo = mm ? mm[0] : lo_h, hi = mm ? mm[1] : hi_h;
     const float rng = __fsub_rn(hi, lo);
-    const bool same = ph == H && pw == W;
-    const float sh = __fdiv_rn((float)ph, (float)H), sw = __fdiv_rn((float)pw, (float)W);
-    for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < np;
-         p += (int64_t)gridDim.x * blockDim.x) {
-        const int y = (int)(p / W), x = (int)(p - (int64_t)y * W);
-        float base[3];
-        if (same || !prev) {
+    const uint32_t x = q / 3u, c = q - 3u * x;
+    float lx0 = 0.f, lx1 = 0.f;
+    Off oa = 0, ob = 0;
+    if constexpr (RESIZE) {
+        const float sw = __fdiv_rn((float)pw, (float)W);
+        float rx = sw * ((float)x + 0.5f) - 0.5f;
+        rx = rx < 0.f ? 0.f : rx;
+        const int x0 = (int)rx;
+        lx1 = rx - (float)x0;
+        lx0 = 1.f - lx1;
+        oa = ((Off)3 * (Off)x0 + c) * 4u;
+        ob = oa + (x0 < pw - 1 ? 12u : 0u);
+        __syncthreads();
+    }
+    if (q >= pitch) return;
+    auto at = [](const float *p, Off o) {
+        return *reinterpret_cast<const float *>(reinterpret_cast<const char *>(p) + o);
+    };
+    // this CTA's rows: one base per array, offsets in bytes
+    const float *rend = render + r0 * pitch, *prv = prev;
+    if (!RESIZE && prev) prv = prev + r0 * pitch;
+    float *dst = out + r0 * pitch;
+    const Off row = (Off)(pitch * 4);
+    auto rows = [&](int k0, auto full_tag) {  // FULL: the whole batch lies inside
+        constexpr bool FULL = decltype(full_tag)::value;
+        float v[kComposeBatch], t[kComposeBatch][4];
 #pragma unroll
-            for (int c = 0; c < 3; ++c) base[c] = prev ? prev[3 * p + c] : 0.f;
-        } else {
-            // the half-pixel source index and weights written as the bilinear
-            // definition states them (src = s (d + 0.5) - 0.5, negative -> 0;
-            // lambda1 = src - floor, lambda0 = 1 - lambda1), so that the
-            // compiler contracts them as it does torch's upsample kernel
-            float ry = sh * ((float)y + 0.5f) - 0.5f;
-            float rx = sw * ((float)x + 0.5f) - 0.5f;
-            ry = ry < 0.f ? 0.f : ry;
-            rx = rx < 0.f ? 0.f : rx;
-            const int y0 = (int)ry, x0 = (int)rx;
-            const int y1 = y0 + (y0 < ph - 1 ? 1 : 0), x1 = x0 + (x0 < pw - 1 ? 1 : 0);
-            const float ly1 = ry - (float)y0, lx1 = rx - (float)x0;
-            const float ly0 = 1.f - ly1, lx0 = 1.f - lx1;
-            const float *r0 = prev + 3 * ((int64_t)y0 * pw), *r1 = prev + 3 * ((int64_t)y1 * pw);
-#pragma unroll
-            for (int c = 0; c < 3; ++c)
-                base[c] = ly0 * (lx0 * r0[3 * x0 + c] + lx1 * r0[3 * x1 + c]) +
-                          ly1 * (lx0 * r1[3 * x0 + c] + lx1 * r1[3 * x1 + c]);
+        for (int k = 0; k < kComposeBatch; ++k) {
+            if (!FULL && k0 + k >= nr) break;
+            const Off o = (Off)(k0 + k) * row + (Off)q * 4u;
+            v[k] = at(rend, o);
+            if constexpr (RESIZE) {
+                const RowTap<Off> r = s_row[k0 + k];
+                t[k][0] = at(prv, r.a + oa);
+                t[k][1] = at(prv, r.a + ob);
+                t[k][2] = at(prv, r.b + oa);
+                t[k][3] = at(prv, r.b + ob);
+            } else {
+                t[k][0] = prev ? at(prv, o) : 0.f;
+            }
         }
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            float r = render[3 * p + c];
+        for (int k = 0; k < kComposeBatch; ++k) {
+            if (!FULL && k0 + k >= nr) break;
+            float base = t[k][0];
+            if constexpr (RESIZE) {
+                const float ly0 = s_row[k0 + k].ly0, ly1 = s_row[k0 + k].ly1;
+                base = ly0 * (lx0 * t[k][0] + lx1 * t[k][1]) + ly1 * (lx0 * t[k][2] + lx1 * t[k][3]);
+            }
+            float r = v[k];
             if (clamp_render) r = fminf(fmaxf(r, 0.f), 1.f);
             const float est = __fadd_rn(__fsub_rn(__fmul_rn(r, rng), 0.5f), lo);
-            float v = __fadd_rn(base[c], est);
-            if (clamp_out) v = fminf(fmaxf(v, 0.f), 1.f);
-            out[3 * p + c] = v;
+            float o = __fadd_rn(base, est);
+            if (clamp_out) o = fminf(fmaxf(o, 0.f), 1.f);
+            *reinterpret_cast<float *>(reinterpret_cast<char *>(dst) + (Off)(k0 + k) * row +
+                                       (Off)q * 4u) = o;
         }
-    }
+    };
+    int k0 = 0;
+    for (; k0 + kComposeBatch <= nr; k0 += kComposeBatch) rows(k0, std::true_type{});
+    if (k0 < nr) rows(k0, std::false_type{});
 }
 
 inline int level_blocks(int64_t n) {
     int64_t b = (n + kLevelThreads - 1) / kLevelThreads;
-    const int64_t cap = 148 * 16;
+    const int64_t cap = 148 * kLevelCtas;
     return (int)(b < 1 ? 1 : (b > cap ? cap : b));
 }
 
@@ -158,8 +251,13 @@ extern "C" int lig_level_residual(int64_t n, const float *gt, const float *up, f
     if (n <= 0 || !gt || !up || !out || !minmax) return LIG_ERR_INVALID;
     cudaStream_t s = (cudaStream_t)stream;
     minmax_init_kernel<<<1, 1, 0, s>>>(minmax);
-    resid_minmax_kernel<<<level_blocks(n), kLevelThreads, 0, s>>>(n, gt, up, minmax);
-    resid_normalise_kernel<<<level_blocks(n), kLevelThreads, 0, s>>>(n, gt, up, minmax, out);
+    const bool vec = ((reinterpret_cast<uintptr_t>(gt) | reinterpret_cast<uintptr_t>(up) |
+                       reinterpret_cast<uintptr_t>(out)) & 15) == 0;
+    const int blocks = level_blocks(vec ? (n + 3) / 4 : n);
+    auto minmax_k = vec ? resid_minmax_kernel<true> : resid_minmax_kernel<false>;
+    auto norm_k = vec ? resid_normalise_kernel<true> : resid_normalise_kernel<false>;
+    minmax_k<<<blocks, kLevelThreads, 0, s>>>(n, gt, up, minmax);
+    norm_k<<<blocks, kLevelThreads, 0, s>>>(n, gt, up, minmax, out);
     note_launches(3);
     LIG_LAUNCH_CHECK();
     return LIG_OK;
@@ -172,10 +270,16 @@ extern "C" int lig_level_compose(int prev_h, int prev_w, const float *prev, int 
     if (H <= 0 || W <= 0 || !render || !out || (prev && (prev_h <= 0 || prev_w <= 0)))
         return LIG_ERR_INVALID;
     cudaStream_t s = (cudaStream_t)stream;
-    const int64_t np = (int64_t)H * W;
-    compose_kernel<<<level_blocks(np), kLevelThreads, 0, s>>>(
-        prev_h, prev_w, prev, H, W, render, minmax, (float)store_min, (float)store_max,
-        clamp_render, clamp_out, out);
+    const bool resize = prev && !(prev_h == H && prev_w == W);
+    const dim3 grid((unsigned)((3 * (int64_t)W + kLevelThreads - 1) / kLevelThreads),
+                    (H + kComposeRows - 1) / kComposeRows);
+    const bool small = 12 * (int64_t)prev_h * prev_w <= 0xffffffffll &&
+                       12 * (int64_t)W * kComposeRows <= 0xffffffffll;
+    auto k = !resize ? compose_kernel<false, uint32_t>
+             : small ? compose_kernel<true, uint32_t>
+                     : compose_kernel<true, uint64_t>;
+    k<<<grid, kLevelThreads, 0, s>>>(prev_h, prev_w, prev, H, W, render, minmax, (float)store_min,
+                                     (float)store_max, clamp_render, clamp_out, out);
     note_launches(1);
     LIG_LAUNCH_CHECK();
     return LIG_OK;
