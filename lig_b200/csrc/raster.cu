@@ -81,9 +81,8 @@ __device__ __forceinline__ uint32_t alpha_cut_search() {
     return hi;
 }
 
-// The cut on this device, written by every pack launch for the fused forward
-// (always the same value) and read by that forward, launched after it on the
-// same stream.
+// The cut on this device, written by every float pack launch (always the same
+// value) and read by the rasterizer launched after it on the same stream.
 __device__ uint32_t g_alpha_cut;
 
 // ------------------------------------------------------------------ pack
@@ -107,7 +106,7 @@ __device__ uint32_t g_alpha_cut;
 // forward, see sigma_half); the cull data are computed from the full conic.
 // zero (backward): also clears the Gaussian's zero_stride accumulators there
 // (zero_stride * sizeof(T) a multiple of 16 bytes, 16-byte aligned).
-// HALF or TAME (float): block 0's first warp also publishes the alpha cut.
+// Float: block 0's first warp also publishes the alpha cut.
 // TAME (the packed gradient-aware kernels, which add a zero where a pixel
 // fails the alpha test instead of skipping it): culling data only for records
 // whose products at any pixel they are evaluated on stay finite (see
@@ -127,7 +126,7 @@ template <typename T, bool HALF, bool TAME = false>
 __global__ void pack_kernel(int n, const T *__restrict__ xys, const T *__restrict__ conics,
                             const T *__restrict__ colors, const T *__restrict__ opac,
                             Rec<T> *__restrict__ recs, T *__restrict__ zero, int zero_stride) {
-    if ((HALF || TAME) && sizeof(T) == 4 && blockIdx.x == 0 && threadIdx.x < 32) {
+    if (sizeof(T) == 4 && blockIdx.x == 0 && threadIdx.x < 32) {
         const uint32_t cut = alpha_cut_search();
         if (threadIdx.x == 0) g_alpha_cut = cut;
     }
@@ -801,7 +800,9 @@ __device__ __forceinline__ void fwd_tile(const TileCtx &tc, int tile, const int3
 #define LIG_RASTER_BWD_R16_MAX_DENSITY 0.04
 #endif
 #ifndef LIG_RASTER_BWD_RROWS_MINB
-#define LIG_RASTER_BWD_RROWS_MINB 8  // resident CTAs per SM of the 8x8 walk (128 threads)
+// resident CTAs per SM of the 8x8 walk (128 threads): 2048^2 / 1M 681 us with 7
+// (72 registers), 696 with 6, 705 with 8 (64, spilling)
+#define LIG_RASTER_BWD_RROWS_MINB 7
 #endif
 #ifndef LIG_RASTER_BWD_R16_MINB
 #define LIG_RASTER_BWD_R16_MINB 14  // resident CTAs per SM of the 8x16 walk (64 threads, 72 registers)
@@ -1309,10 +1310,12 @@ struct alignas(16) PixPair {
 // acc[3]: per pixel v_sigma (a dx + b dy) and v_sigma (b dx + c dy).
 // GEN: opacities and a wsum cotangent (pair entry's fourth channel); the
 // opacity gradient's sum of exp(-sigma) v_alpha in acc[10].
-template <int NCP, int CSTEP, int NR, bool ABS = false, int NH = 1, bool GEN = false>
+template <int NCP, int CSTEP, int NR, bool ABS = false, int NH = 1, bool GEN = false,
+          bool CUT = false>
 __device__ __forceinline__ void lean_region_f2(const Rec<float> &g, float clamp,
                                                const PixPair *__restrict__ pp, int c0, int r0,
-                                               float px0, float py0, float (&acc)[11]) {
+                                               float px0, float py0, uint32_t cut,
+                                               float (&acc)[11]) {
     const float ha = 0.5f * g.a, hc = 0.5f * g.c;
     const f2 HA = f2_dup(ha), BB = f2_dup(g.b);
     f2 AA, CC;
@@ -1357,8 +1360,8 @@ __device__ __forceinline__ void lean_region_f2(const Rec<float> &g, float clamp,
                 const float vis0 = __expf(-s0), vis1 = __expf(-s1);
                 const float al0 = fminf(clamp, GEN ? g.o * vis0 : vis0);
                 const float al1 = fminf(clamp, GEN ? g.o * vis1 : vis1);
-                const bool no0 = s0 < 0.f || al0 < 1.f / 255.f;
-                const bool no1 = s1 < 0.f || al1 < 1.f / 255.f;
+                const bool no0 = CUT ? __float_as_uint(s0) >= cut : s0 < 0.f || al0 < 1.f / 255.f;
+                const bool no1 = CUT ? __float_as_uint(s1) >= cut : s1 < 0.f || al1 < 1.f / 255.f;
                 const f2 A = f2_pack(no0 ? 0.f : al0, no1 ? 0.f : al1);
                 sr = f2_fma(A, V0, sr);
                 sg = f2_fma(A, V1, sg);
@@ -1437,9 +1440,46 @@ __device__ __noinline__ void sum_pixels_skip(const Rec<float> &g, float clamp,
     }
 }
 
+// Lean walks: the alpha cut's compare (one operation of the half-rate ALU pipe
+// instead of two per pixel) where every Gaussian of a warp's round has culling
+// data.  8192^2 1992 -> 1891 us, 2048^2 / 1M 747 -> 705 (681 at 7 CTAs
+// per SM), 16 images 402 -> 371.
+#ifndef LIG_RASTER_BWD_CUT
+#define LIG_RASTER_BWD_CUT 1
+#endif
 #ifndef LIG_RASTER_BWD_BULK
 #define LIG_RASTER_BWD_BULK 1  // lean backward (float): records staged by bulk async copies
 #endif
+// One lane's share of a Gaussian over its region, in blocks of four rows: 1 / 2 /
+// 4 / 8 lanes (lsplit) share the Gaussian, taking column pairs (1 / 2 / 4 lanes)
+// or column pairs and row halves (8 lanes).
+template <int RR, bool ABS, bool GEN, bool CUT>
+__device__ __forceinline__ void lean_round(const Rec<float> &g, float clamp,
+                                           const PixPair *__restrict__ pp, int lsplit, int part,
+                                           float px0, float py0, uint32_t cut, float (&acc)[11]) {
+    constexpr int NB = RR / 4;
+    switch (lsplit) {
+    case 0:
+        lean_region_f2<4, 1, 4, ABS, NB, GEN, CUT>(g, clamp, pp, 0, 0, px0, py0, cut, acc);
+        break;
+    case 1:
+        lean_region_f2<2, 2, 4, ABS, NB, GEN, CUT>(g, clamp, pp, part, 0, px0, py0, cut, acc);
+        break;
+    case 2:
+        lean_region_f2<1, 1, 4, ABS, NB, GEN, CUT>(g, clamp, pp, part, 0, px0, py0, cut, acc);
+        break;
+    default:
+        if constexpr (RR == 4)
+            lean_region_f2<1, 1, 2, ABS, 1, GEN, CUT>(g, clamp, pp, part & 3, 2 * (part >> 2), px0,
+                                                      py0, cut, acc);
+        else
+            lean_region_f2<1, 1, 4, ABS, NB / 2, GEN, CUT>(g, clamp, pp, part & 3,
+                                                           (RR / 2) * (part >> 2), px0, py0, cut,
+                                                           acc);
+        break;
+    }
+}
+
 // Bounded device waits that gave up (a malfunction; read by lig_wait_timeouts).
 __device__ unsigned int g_wait_timeouts;
 // SM clock cycles (about 1 ms) before an mbarrier wait is abandoned: a
@@ -1525,6 +1565,8 @@ __device__ __forceinline__ void bwd_tile(const TileCtx &tc, int tile,
     // records staged by bulk async copies (no register prefetch, no region
     // masks: the warps test the box and ellipse themselves)
     constexpr bool kBulk = kPairs && LIG_RASTER_BWD_BULK;
+    constexpr bool kCut = kPairs && !GEN && LIG_RASTER_BWD_CUT;
+    [[maybe_unused]] const uint32_t cut = kCut ? g_alpha_cut : 0u;
     static_assert(RR == 4 || kPairs, "taller regions are walked by the pair form only");
     static_assert(RR == 4 || RR == 8 || RR == 16, "region rows");
     constexpr int kRows = RR;  // pair entries per region: kRows * 4
@@ -1742,40 +1784,17 @@ __device__ __forceinline__ void bwd_tile(const TileCtx &tc, int tile,
                                     min(H, ty0 + B), t);
 #pragma unroll
                     for (int q = 0; q < 11; ++q) acc[q] = t[q];
-                } else if (act && RR > 4) {
-                    // the region in blocks of four rows (8 lanes: one half each)
-                    constexpr int NB = RR / 4;
-                    switch (lsplit) {
-                    case 0:
-                        lean_region_f2<4, 1, 4, ABS, NB, GEN>(g, clamp, pp, 0, 0, px0, py0, acc);
-                        break;
-                    case 1:
-                        lean_region_f2<2, 2, 4, ABS, NB, GEN>(g, clamp, pp, part, 0, px0, py0, acc);
-                        break;
-                    case 2:
-                        lean_region_f2<1, 1, 4, ABS, NB, GEN>(g, clamp, pp, part, 0, px0, py0, acc);
-                        break;
-                    default:
-                        lean_region_f2<1, 1, 4, ABS, NB / 2, GEN>(g, clamp, pp, part & 3,
-                                                             (RR / 2) * (part >> 2), px0, py0,
-                                                             acc);
-                        break;
-                    }
-                } else if (act) {
-                    switch (lsplit) {
-                    case 0:
-                        lean_region_f2<4, 1, 4, ABS, 1, GEN>(g, clamp, pp, 0, 0, px0, py0, acc);
-                        break;
-                    case 1:
-                        lean_region_f2<2, 2, 4, ABS, 1, GEN>(g, clamp, pp, part, 0, px0, py0, acc);
-                        break;
-                    case 2:
-                        lean_region_f2<1, 1, 4, ABS, 1, GEN>(g, clamp, pp, part, 0, px0, py0, acc);
-                        break;
-                    default:
-                        lean_region_f2<1, 1, 2, ABS, 1, GEN>(g, clamp, pp, part & 3, 2 * (part >> 2),
-                                                     px0, py0, acc);
-                        break;
+                } else {
+                    // the cut's compare where every Gaussian of the round has
+                    // culling data (no opacities)
+                    bool fast = false;
+                    if constexpr (kCut)
+                        fast = __all_sync(FULL, !act || reinterpret_cast<const Rec<float> &>(g).wx >= 0.f);
+                    if (act) {
+                        if (kCut && fast)
+                            lean_round<RR, ABS, GEN, kCut>(g, clamp, pp, lsplit, part, px0, py0, cut, acc);
+                        else
+                            lean_round<RR, ABS, GEN, false>(g, clamp, pp, lsplit, part, px0, py0, cut, acc);
                     }
                 }
             } else if constexpr (LEAN && !GA && LIG_RASTER_BWD_COLS) {
@@ -2007,7 +2026,7 @@ struct alignas(16) GaPix {  // pixels (row, c) and (row, c + W/2)
 template <int NCP, int CSTEP, int HW, bool OP, bool VW>
 __device__ __forceinline__ void ga_rows(const Rec<float> &g, float clamp,
                                         const GaPix *__restrict__ pix, int c0, float px0,
-                                        float py0, float (&acc)[11]) {
+                                        float py0, uint32_t cut, float (&acc)[11]) {
     const f2 AA = f2_dup(g.a), BB = f2_dup(g.b), CC = f2_dup(g.c), NB = f2_dup(-g.b);
     const f2 HALF = f2_dup(0.5f);
     const f2 CR = f2_dup(g.r), CG = f2_dup(g.g), CB = f2_dup(g.bl);
@@ -2038,7 +2057,14 @@ __device__ __forceinline__ void ga_rows(const Rec<float> &g, float clamp,
             const float vis0 = __expf(-s0), vis1 = __expf(-s1);
             const float al0 = fminf(clamp, OP ? g.o * vis0 : vis0);
             const float al1 = fminf(clamp, OP ? g.o * vis1 : vis1);
-            const bool no0 = s0 < 0.f || al0 < 1.f / 255.f, no1 = s1 < 0.f || al1 < 1.f / 255.f;
+            bool no0, no1;
+            if constexpr (!OP && LIG_RASTER_ALPHA_CUT) {
+                no0 = __float_as_uint(s0) >= cut;
+                no1 = __float_as_uint(s1) >= cut;
+            } else {
+                no0 = s0 < 0.f || al0 < 1.f / 255.f;
+                no1 = s1 < 0.f || al1 < 1.f / 255.f;
+            }
             const f2 AL = f2_pack(no0 ? 0.f : al0, no1 ? 0.f : al1);
             const f2 SX = f2_fma(BB, DY[r], AX), SY = f2_fma(CC, DY[r], BX);
             const f2 P = f2_fma(SX, SY, NB);
@@ -2170,6 +2196,7 @@ raster_bwd_ga_kernel(const BatchGeo geo, const int32_t *__restrict__ cum, int *w
     }
     __syncthreads();
     const int n_tiles = geo.total_tiles();
+    const uint32_t cut = OP ? 0u : g_alpha_cut;
     const GaPix *my_pix = s_pix + w * 16;
     uint16_t *my_list = s_list[w];
     for (int tile = next_tile(work, s_slot, true); tile < n_tiles;
@@ -2256,16 +2283,16 @@ raster_bwd_ga_kernel(const BatchGeo geo, const int32_t *__restrict__ cum, int *w
                         const float py = py0 + (float)(2 * rp);
                         switch (lsplit) {
                         case 0:
-                            ga_rows<HW, 1, HW, OP, VW>(g, clamp, rows, 0, px0, py, acc);
+                            ga_rows<HW, 1, HW, OP, VW>(g, clamp, rows, 0, px0, py, cut, acc);
                             break;
                         case 1:
-                            ga_rows<HW / 2, 2, HW, OP, VW>(g, clamp, rows, part, px0, py, acc);
+                            ga_rows<HW / 2, 2, HW, OP, VW>(g, clamp, rows, part, px0, py, cut, acc);
                             break;
                         case 2:
-                            ga_rows<HW / 4, 4, HW, OP, VW>(g, clamp, rows, part, px0, py, acc);
+                            ga_rows<HW / 4, 4, HW, OP, VW>(g, clamp, rows, part, px0, py, cut, acc);
                             break;
                         default:
-                            ga_rows<1, 8, HW, OP, VW>(g, clamp, rows, part & (HW - 1), px0, py,
+                            ga_rows<1, 8, HW, OP, VW>(g, clamp, rows, part & (HW - 1), px0, py, cut,
                                                       acc);
                             break;
                         }

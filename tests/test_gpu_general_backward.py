@@ -97,3 +97,26 @@ def test_non_finite_values_stay_where_the_alpha_test_lets_them(H, W, B, n):
     for a, b in zip(*res):
         assert torch.equal(torch.isnan(a), torch.isnan(b))
         assert (torch.isfinite(a) & torch.isfinite(b)).any()
+
+
+@pytest.mark.parametrize("H,W,B,n", [(61, 77, 16, 300), (1030, 1041, 16, 20000),
+                                     (1030, 1041, 16, 90000), (517, 515, 8, 9000)])
+def test_lean_walk_with_records_without_culling_data(H, W, B, n):
+    """Without opacities a warp's round takes the alpha cut's compare or, with an
+    indefinite or nearly degenerate conic among its Gaussians, the float test."""
+    def spoil(con, col):
+        con[5::41, 1] = 1.2 * con[5::41, 0]                       # indefinite
+        con[7::53, 1] = (0.9996 * con[7::53, 0] * con[7::53, 2]).sqrt()
+
+    args = _setup(H, W, B, n, None, spoil)
+    cot = torch.randn(H, W, 3, generator=torch.Generator().manual_seed(7)).cuda()
+    res = []
+    for dt in (torch.float32, torch.float64):
+        a = args(dt)
+        fin = ops.raster_fwd(*a, False)[5]
+        res.append(ops.raster_bwd(*a, fin, cot.to(dt), None))
+    # the degenerate records' own sums reach far and cancel: held apart
+    ok = torch.ones(n, dtype=torch.bool, device="cuda")
+    ok[5::41] = ok[7::53] = False
+    _check([t[ok] for t in res[0] if t is not None], [t[ok] for t in res[1] if t is not None])
+    assert all(torch.isfinite(t).all() for t in res[0] if t is not None)
