@@ -381,20 +381,14 @@ __device__ __forceinline__ int next_tile(int *work, int &s_slot, bool first) {
 }
 
 // --------------------------------------------------------------- forward
-#ifndef LIG_RASTER_FWD_WARPS
-#define LIG_RASTER_FWD_WARPS 1  // sum forward: warps stream the tile list independently
-#endif
 #ifndef LIG_RASTER_FWD_ELLIPSE
 #define LIG_RASTER_FWD_ELLIPSE 1  // sum forward: exact ellipse test per region
 #endif
 #ifndef LIG_RASTER_FWD_ELLIPSE_GA
 #define LIG_RASTER_FWD_ELLIPSE_GA 1  // the same in the gradient-aware forward
 #endif
-#ifndef LIG_RASTER_FWD_FUSED
-#define LIG_RASTER_FWD_FUSED 1  // specialised fused-loss forward (no opacities)
-#endif
 #ifndef LIG_RASTER_ALPHA_CUT
-#define LIG_RASTER_ALPHA_CUT 1  // fused forward: alpha test by the cut's compare
+#define LIG_RASTER_ALPHA_CUT 1  // forwards without opacities: alpha test by the cut's compare
 #endif
 // One CTA per tile, warp w = region w (8x4 pixels), one pixel per lane.
 // Batches of blockDim Gaussians (list order) are staged in shared memory, one
@@ -447,24 +441,15 @@ __device__ __forceinline__ T sigma_half(T ha, T b, T hc, T dx, T dy) {
 
 template <typename T>
 struct PixelEval {
-    // csrc/forward.cu:250-259 (sum) / csrc/gradient_aware_rasterizer.cu:436-445
-    // (gradient-aware: d = p - mu); returns false when the term is skipped.
-    template <bool GA>
+    // gradient-aware, csrc/gradient_aware_rasterizer.cu:436-445 (d = p - mu);
+    // returns false when the term is skipped.
     static __device__ __forceinline__ bool alpha(const Rec<T> &g, T px, T py, T &dx, T &dy,
                                                  T &a) {
         using M = Math<T>;
-        if (!GA) { dx = g.x - px; dy = g.y - py; }
-        else { dx = px - g.x; dy = py - g.y; }
+        dx = px - g.x;
+        dy = py - g.y;
         const T sigma = sigma_ref<T>(g.a, g.b, g.c, dx, dy);
         a = M::min_((T)0.999, g.o * M::exp_(-sigma));
-        return !(sigma < (T)0 || a < (T)1 / (T)255);
-    }
-    // the fused-loss forward: halved conic in the record, no opacities (o = 1,
-    // so o * exp(-sigma) is exp(-sigma) exactly)
-    static __device__ __forceinline__ bool alpha_fused(const Rec<T> &g, T px, T py, T &a) {
-        using M = Math<T>;
-        const T sigma = sigma_half<T>(g.a, g.b, g.c, g.x - px, g.y - py);
-        a = M::min_((T)0.999, M::exp_(-sigma));
         return !(sigma < (T)0 || a < (T)1 / (T)255);
     }
 };
@@ -474,16 +459,18 @@ struct FwdAcc {
     T r = 0, g = 0, b = 0, w = 0;
     T dx[GA ? 3 : 1] = {}, dy[GA ? 3 : 1] = {}, dxy[GA ? 3 : 1] = {};
     int cur = 0;
-    // fused-loss forward: colour and, with FIN, the final index (no wsum, not GA)
-    template <bool FIN = true>
-    __device__ __forceinline__ void add_fused(const Rec<T> &q, T a, int idx) {
+    // sum: colour, with FIN the final index and with WS the weight sum
+    template <bool FIN, bool WS>
+    __device__ __forceinline__ void add_sum(const Rec<T> &q, T a, int idx) {
+        // csrc/forward.cu:264-269
         r += q.r * a;
         g += q.g * a;
         b += q.bl * a;
+        if constexpr (WS) w += a;
         if constexpr (FIN) cur = idx;
     }
     __device__ __forceinline__ void add(const Rec<T> &q, T dxp, T dyp, T a, int idx) {
-        // csrc/forward.cu:264-269, csrc/gradient_aware_rasterizer.cu:451-482
+        // csrc/gradient_aware_rasterizer.cu:451-482
         r += q.r * a;
         g += q.g * a;
         b += q.bl * a;
@@ -586,27 +573,31 @@ __device__ __forceinline__ double fwd_write(const FwdAcc<T, GA> &acc, bool insid
     return 0.0;
 }
 
-// PPL pixels per lane: 1 (8x4 regions, two Gaussians per iteration), 2 (8x8
-// regions, lane owns (x, y) and (x, y + 4)) or 4 (8x16, (x, y + 4p)); each
-// Gaussian's record and loop overhead are shared by the lane's evaluations,
-// whose independent sigma / exp chains overlap.  Per pixel the terms are
-// added in list order either way.
-// FL: the fused-loss forward without opacities (records carry the halved
-// conic; no wsum): per pixel the same alphas and colour sums, fewer operations.
-template <typename T, bool GA, int PPL, bool FL, bool FIN = true>
+// PPL pixels per lane: 1 (8x4 regions, two Gaussians per iteration; gradient-
+// aware), 2 (8x8 regions, lane owns (x, y) and (x, y + 4)) or 4 (8x16, (x, y +
+// 4p)); each Gaussian's record and loop overhead are shared by the lane's
+// evaluations, whose independent sigma / exp chains overlap.  Per pixel the
+// terms are added in list order either way.
+// The sum forward's records carry the halved conic (see sigma_half); a lane's
+// pixels share their column, so dx, (a/2) dx and b dx are formed once per
+// Gaussian.  OP: opacities.  FIN, WS: final indices and weight sums are wanted
+// (the fused loss needs neither).  Without opacities, chunks whose records all
+// carry culling data test alpha by the cut's compare: bound by instruction
+// issue; eight views of 500k Gaussians with weight sums and indices 401 us, against
+// 498 with the full conic, an opacity product and the float test.
+template <typename T, bool GA, int PPL, bool OP, bool FIN, bool WS>
 __device__ __forceinline__ void fwd_tile(const TileCtx &tc, int tile, const int32_t *__restrict__ ids,
                                          const int2 *__restrict__ tile_bins,
                                          const Rec<T> *__restrict__ recs, T *__restrict__ img,
                                          T *__restrict__ wsum, T *__restrict__ odx,
                                          T *__restrict__ ody, T *__restrict__ odxy,
                                          int32_t *__restrict__ final_idx, Rec<T> *s_rec,
-                                         uint32_t *s_bits, const L2Fwd<T> &l2, uint32_t cut) {
-    // the alpha cut's compare: the fused forward's pixel pairs (float)
-    constexpr bool kCut = FL && PPL > 1 && sizeof(T) == 4 && LIG_RASTER_ALPHA_CUT;
+                                         const L2Fwd<T> &l2, uint32_t cut) {
+    constexpr bool kCut = !GA && !OP && sizeof(T) == 4 && LIG_RASTER_ALPHA_CUT;
     const unsigned FULL = 0xffffffffu;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const int B = tc.B, tx0 = tc.tx0, ty0 = tc.ty0;
-    static_assert(PPL == 1 || PPL == 2 || PPL == 4, "one, two or four pixels per lane");
+    static_assert(GA ? PPL == 1 : PPL == 2 || PPL == 4, "pixels per lane");
     const Regions R = Regions::make(PPL == 1 ? 0 : (PPL == 2 ? 1 : 3), B);
     // a warp lists only the Gaussians whose alpha >= 1/255 ellipse meets
     // its region (one test per Gaussian and region)
@@ -628,31 +619,10 @@ __device__ __forceinline__ void fwd_tile(const TileCtx &tc, int tile, const int3
     FwdAcc<T, GA> acc[PPL];
     // walk the Gaussians of `mask` (bits of the 32 records at rb, list
     // indices ib + bit) in list order; fast_tag true: every record has
-    // culling data, so the fused forward tests alpha by the cut's compare
+    // culling data, so alpha is tested by the cut's compare
     auto walk = [&](uint32_t mask, const Rec<T> *rb, int ib, auto fast_tag) {
         [[maybe_unused]] constexpr bool FAST = decltype(fast_tag)::value;
-        if constexpr (FL && PPL == 1) {
-            while (mask) {
-                const int b1 = __ffs(mask) - 1;
-                mask &= mask - 1;
-                const Rec<T> g1 = rb[b1];
-                T a1;
-                const bool ok1 = PixelEval<T>::alpha_fused(g1, px[0], py[0], a1);
-                if (mask) {
-                    const int b2 = __ffs(mask) - 1;
-                    mask &= mask - 1;
-                    const Rec<T> g2 = rb[b2];
-                    T a2;
-                    const bool ok2 = PixelEval<T>::alpha_fused(g2, px[0], py[0], a2);
-                    if (ok1) acc[0].template add_fused<FIN>(g1, a1, ib + b1);
-                    if (ok2) acc[0].template add_fused<FIN>(g2, a2, ib + b2);
-                } else if (ok1) {
-                    acc[0].template add_fused<FIN>(g1, a1, ib + b1);
-                }
-            }
-        } else if constexpr (FL) {
-            // a lane's pixels share their column: dx, (a/2) dx and
-            // b dx once per Gaussian (sigma_half's products)
+        if constexpr (!GA) {
             using M = Math<T>;
             while (mask) {
                 const int b1 = __ffs(mask) - 1;
@@ -666,95 +636,58 @@ __device__ __forceinline__ void fwd_tile(const TileCtx &tc, int tile, const int3
                 for (int p = 0; p < PPL; ++p) {
                     const T dy = g1.y - py[p];
                     const T sg = fma_rn(bdx, dy, fma_rn(hadx, dx, mul_rn(mul_rn(g1.c, dy), dy)));
-                    ap[p] = M::min_((T)0.999, M::exp_(-sg));
+                    const T e = M::exp_(-sg);
+                    ap[p] = M::min_((T)0.999, OP ? g1.o * e : e);
                     if constexpr (FAST) okp[p] = __float_as_uint((float)sg) < cut;
                     else okp[p] = !(sg < (T)0 || ap[p] < (T)1 / (T)255);
                 }
 #pragma unroll
                 for (int p = 0; p < PPL; ++p)
-                    if (okp[p]) acc[p].template add_fused<FIN>(g1, ap[p], ib + b1);
+                    if (okp[p]) acc[p].template add_sum<FIN, WS>(g1, ap[p], ib + b1);
             }
-        } else if constexpr (PPL == 1) {
+        } else {
             while (mask) {
                 const int b1 = __ffs(mask) - 1;
                 mask &= mask - 1;
                 const Rec<T> g1 = rb[b1];
                 T dx1, dy1, a1;
-                const bool ok1 =
-                    PixelEval<T>::template alpha<GA>(g1, px[0], py[0], dx1, dy1, a1);
+                const bool ok1 = PixelEval<T>::alpha(g1, px[0], py[0], dx1, dy1, a1);
                 if (mask) {
                     const int b2 = __ffs(mask) - 1;
                     mask &= mask - 1;
                     const Rec<T> g2 = rb[b2];
                     T dx2, dy2, a2;
-                    const bool ok2 =
-                        PixelEval<T>::template alpha<GA>(g2, px[0], py[0], dx2, dy2, a2);
+                    const bool ok2 = PixelEval<T>::alpha(g2, px[0], py[0], dx2, dy2, a2);
                     if (ok1) acc[0].add(g1, dx1, dy1, a1, ib + b1);
                     if (ok2) acc[0].add(g2, dx2, dy2, a2, ib + b2);
                 } else if (ok1) {
                     acc[0].add(g1, dx1, dy1, a1, ib + b1);
                 }
             }
-        } else {
-            while (mask) {
-                const int b1 = __ffs(mask) - 1;
-                mask &= mask - 1;
-                const Rec<T> g1 = rb[b1];
-                T dxp[PPL], dyp[PPL], ap[PPL];
-                bool okp[PPL];
-#pragma unroll
-                for (int p = 0; p < PPL; ++p)
-                    okp[p] = PixelEval<T>::template alpha<GA>(g1, px[p], py[p], dxp[p],
-                                                              dyp[p], ap[p]);
-#pragma unroll
-                for (int p = 0; p < PPL; ++p)
-                    if (okp[p]) acc[p].add(g1, dxp[p], dyp[p], ap[p], ib + b1);
-            }
         }
     };
     if (!tc.empty) {
         const int2 range = tile_bins[tile];
-        if constexpr (LIG_RASTER_FWD_WARPS) {
-            // each warp streams the tile's list in chunks of 32 on its own
-            // (its region's test only, no block barriers: warps whose
-            // regions have short lists do not wait for the others)
-            Rec<T> *w_rec = s_rec + w * 32;
-            Rec<T> pre;
-            if (range.x + lane < range.y) pre = recs[__ldg(ids + range.x + lane)];
-            for (int base = range.x; base < range.y; base += 32) {
-                const bool hit =
-                    base + lane < range.y && region_hit<T, ELL, FL>(pre, R, w, tx0, ty0);
-                // a chunk whose records all carry culling data takes the cut
-                bool fast = false;
-                if constexpr (kCut)
-                    fast = !__any_sync(FULL, base + lane < range.y && !(pre.wx >= (T)0));
-                __syncwarp();
-                w_rec[lane] = pre;
-                __syncwarp();
-                if (base + 32 + lane < range.y) pre = recs[__ldg(ids + base + 32 + lane)];
-                const uint32_t mask = __ballot_sync(FULL, hit);
-                if (fast) walk(mask, w_rec, base, std::true_type{});
-                else walk(mask, w_rec, base, std::false_type{});
-            }
-        } else {
-            const int nt = blockDim.x;
-            Rec<T> pre;
-            if (range.x + tid < range.y) pre = recs[__ldg(ids + range.x + tid)];
-            for (int base = range.x; base < range.y; base += nt) {
-                const int cnt = min(nt, range.y - base);
-                __syncthreads();
-                if (tid < cnt) {
-                    s_rec[tid] = pre;
-                    s_bits[tid] = region_bits<T, ELL, FL>(pre, R, tx0, ty0);
-                }
-                __syncthreads();
-                if (base + nt + tid < range.y) pre = recs[__ldg(ids + base + nt + tid)];
-                for (int m = 0; m * 32 < cnt; ++m) {
-                    const int t = m * 32 + lane;
-                    walk(__ballot_sync(FULL, t < cnt && ((s_bits[t] >> w) & 1u)), s_rec + m * 32,
-                         base + m * 32, std::false_type{});
-                }
-            }
+        // each warp streams the tile's list in chunks of 32 on its own
+        // (its region's test only, no block barriers: warps whose
+        // regions have short lists do not wait for the others)
+        Rec<T> *w_rec = s_rec + w * 32;
+        Rec<T> pre;
+        if (range.x + lane < range.y) pre = recs[__ldg(ids + range.x + lane)];
+        for (int base = range.x; base < range.y; base += 32) {
+            const bool hit =
+                base + lane < range.y && region_hit<T, ELL, !GA>(pre, R, w, tx0, ty0);
+            // a chunk whose records all carry culling data takes the cut
+            bool fast = false;
+            if constexpr (kCut)
+                fast = !__any_sync(FULL, base + lane < range.y && !(pre.wx >= (T)0));
+            __syncwarp();
+            w_rec[lane] = pre;
+            __syncwarp();
+            if (base + 32 + lane < range.y) pre = recs[__ldg(ids + base + 32 + lane)];
+            const uint32_t mask = __ballot_sync(FULL, hit);
+            if (kCut && fast) walk(mask, w_rec, base, std::bool_constant<kCut>{});
+            else walk(mask, w_rec, base, std::false_type{});
         }
     } else {  // the reference's empty-list branch (rasterize.py:80-90)
 #pragma unroll
@@ -768,9 +701,8 @@ __device__ __forceinline__ void fwd_tile(const TileCtx &tc, int tile, const int3
 }
 
 // Launch bounds: tiles of B <= 16 launch <= 256 threads, and their
-// instantiation asks for LIG_RASTER_FWD_MINB / LIG_RASTER_BWD_MINB resident
-// CTAs per SM (the register budget follows); larger tiles use the 1024-thread
-// instantiation.
+// instantiations ask for a number of resident CTAs per SM (the register budget
+// follows); larger tiles use instantiations for more threads.
 #ifndef LIG_RASTER_FWD_MINB
 #define LIG_RASTER_FWD_MINB 4
 #endif
@@ -845,12 +777,9 @@ __device__ __forceinline__ void fwd_tile(const TileCtx &tc, int tile, const int3
 #define LIG_RASTER_BWD_MINB 5
 #endif
 
-// Sum forward: two pixels per lane from LIG_RASTER_PPL2_MIN_TILES tiles on,
-// four from LIG_RASTER_PPL4_MIN_TILES on (fewer warps per tile, so small
-// images keep more pixels in flight with fewer pixels per lane).
-#ifndef LIG_RASTER_PPL2_MIN_TILES
-#define LIG_RASTER_PPL2_MIN_TILES 0
-#endif
+// Sum forward: two pixels per lane, four from LIG_RASTER_PPL4_MIN_TILES tiles on
+// (fewer warps per tile, so small images keep more pixels in flight with fewer
+// pixels per lane).
 #ifndef LIG_RASTER_PPL4_MIN_TILES
 #define LIG_RASTER_PPL4_MIN_TILES 4096  // measured: faster from 2048^2 up, not at 512^2
 #endif
@@ -877,7 +806,8 @@ __device__ __forceinline__ void fwd_tile(const TileCtx &tc, int tile, const int3
 #define LIG_RASTER_GA_BWD_SPLIT3 4
 #endif
 
-template <typename T, bool GA, int PPL, int MAXT, int MINB, bool FL = false, bool FIN = true>
+template <typename T, bool GA, int PPL, int MAXT, int MINB, bool OP = true, bool FIN = true,
+          bool WS = true>
 __global__ void __launch_bounds__(MAXT, MINB)
 raster_fwd_kernel(const BatchGeo geo, const int32_t *__restrict__ cum, int *work,
                   const int32_t *__restrict__ ids, const int2 *__restrict__ tile_bins,
@@ -888,14 +818,13 @@ raster_fwd_kernel(const BatchGeo geo, const int32_t *__restrict__ cum, int *work
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int s_slot;
     Rec<T> *s_rec = reinterpret_cast<Rec<T> *>(smem_raw);
-    uint32_t *s_bits = reinterpret_cast<uint32_t *>(s_rec + blockDim.x);
     const int n_tiles = geo.total_tiles();
-    const uint32_t cut = FL && sizeof(T) == 4 ? g_alpha_cut : 0u;
+    const uint32_t cut = !GA && !OP && sizeof(T) == 4 ? g_alpha_cut : 0u;
     for (int tile = next_tile(work, s_slot, true); tile < n_tiles;
          tile = next_tile(work, s_slot, false)) {
         const TileCtx tc = tile_ctx(geo, cum, d_total, tile);
-        fwd_tile<T, GA, PPL, FL, FIN>(tc, tile, ids, tile_bins, recs, img, wsum, odx, ody, odxy,
-                                      final_idx, s_rec, s_bits, l2, cut);
+        fwd_tile<T, GA, PPL, OP, FIN, WS>(tc, tile, ids, tile_bins, recs, img, wsum, odx, ody,
+                                          odxy, final_idx, s_rec, l2, cut);
     }
 }
 
@@ -985,7 +914,7 @@ __device__ __noinline__ void ga_walk_skip(uint32_t mask, const Rec<float> *rb, i
         const Rec<float> g = rb[bit];
         for (int h = 0; h < 2; ++h) {
             float dx, dy, a;
-            if (!PixelEval<float>::template alpha<true>(g, px, py0 + (float)(4 * h), dx, dy, a))
+            if (!PixelEval<float>::alpha(g, px, py0 + (float)(4 * h), dx, dy, a))
                 continue;
             const float sx = g.a * dx + g.b * dy, sy = g.b * dx + g.c * dy;
             const float wx = a * sx, wy = a * sy, wp = a * (sx * sy - g.b);
@@ -2462,9 +2391,9 @@ int raster_fwd(const BatchGeo &geo, TileWalk walk, const int32_t *ids, const int
                L2Fwd<T> l2 = L2Fwd<T>{nullptr, nullptr}, L2Out<T> l2o = L2Out<T>{}) {
     const int n = geo.total_points();
     const bool ga = dx != nullptr;
-    // fused loss without opacities: the specialised forward (halved conic)
-    const bool fl = !ga && (l2.target || l2.target_u8) && !op && LIG_RASTER_FWD_FUSED;
-    int rc = pack<T>(n, xys, con, col, op, ws, ws_bytes, s, fl, nullptr, 0, ga);
+    const bool fused = l2.target || l2.target_u8;
+    // the sum forward reads the halved conic (see sigma_half)
+    int rc = pack<T>(n, xys, con, col, op, ws, ws_bytes, s, !ga, nullptr, 0, ga);
     if (rc) return rc;
     if constexpr (sizeof(T) == 4) {
         if (ga)
@@ -2474,34 +2403,46 @@ int raster_fwd(const BatchGeo &geo, TileWalk walk, const int32_t *ids, const int
     // (tiles of up to 8 rows would leave half of an 8x16 region outside: 8x8
     // tiles at 2048^2 / 150k take 126 us with two pixels a lane, 190 with four)
     const bool ppl4 = !ga && geo.B > 8 && geo.total_tiles() >= LIG_RASTER_PPL4_MIN_TILES;
-    const bool ppl2 = !ga && !ppl4 && geo.total_tiles() >= LIG_RASTER_PPL2_MIN_TILES;
-    const int nt = 32 * Regions::make(ppl4 ? 3 : (ppl2 ? 1 : 0), geo.B).count;
-    const size_t sm = (size_t)nt * (sizeof(Rec<T>) + sizeof(uint32_t));
+    const int nt = 32 * Regions::make(ga ? 0 : (ppl4 ? 3 : 1), geo.B).count;
+    const size_t sm = (size_t)nt * sizeof(Rec<T>);
     using K = void (*)(const BatchGeo, const int32_t *, int *, const int32_t *, const int2 *,
                        const int32_t *, const Rec<T> *, T *, T *, T *, T *, T *, int32_t *,
                        L2Fwd<T>);
     const bool small = nt <= 256;
     constexpr int FM = LIG_RASTER_FWD_MINB;
-    K fn = ga ? (small ? raster_fwd_kernel<T, true, 1, 256, FM>
-                       : raster_fwd_kernel<T, true, 1, 1024, 1>)
-         : fl && fin ? (ppl4 ? (small ? raster_fwd_kernel<T, false, 4, 256, FM, true>
-                                      : raster_fwd_kernel<T, false, 4, 1024, 1, true>)
-                        : ppl2 ? (small ? raster_fwd_kernel<T, false, 2, 256, FM, true>
-                                        : raster_fwd_kernel<T, false, 2, 1024, 1, true>)
-                               : (small ? raster_fwd_kernel<T, false, 1, 256, FM, true>
-                                        : raster_fwd_kernel<T, false, 1, 1024, 1, true>))
-         : fl ? (ppl4 ? (small ? raster_fwd_kernel<T, false, 4, 256, FM, true, false>
-                               : raster_fwd_kernel<T, false, 4, 1024, 1, true, false>)
-                 : ppl2 ? (small ? raster_fwd_kernel<T, false, 2, 256, FM, true, false>
-                                 : raster_fwd_kernel<T, false, 2, 1024, 1, true, false>)
-                        : (small ? raster_fwd_kernel<T, false, 1, 256, FM, true, false>
-                                 : raster_fwd_kernel<T, false, 1, 1024, 1, true, false>))
-              : ppl4 ? (small ? raster_fwd_kernel<T, false, 4, 256, LIG_RASTER_FWD_MINB>
-                              : raster_fwd_kernel<T, false, 4, 1024, 1>)
-              : ppl2 ? (small ? raster_fwd_kernel<T, false, 2, 256, LIG_RASTER_FWD_MINB>
-                              : raster_fwd_kernel<T, false, 2, 1024, 1>)
-                     : (small ? raster_fwd_kernel<T, false, 1, 256, LIG_RASTER_FWD_MINB>
-                              : raster_fwd_kernel<T, false, 1, 1024, 1>);
+    auto sum = [&](auto ppl, auto op_t, auto fin_t, auto ws_t) -> K {
+        constexpr int P = decltype(ppl)::value;
+        constexpr bool O = decltype(op_t)::value, F = decltype(fin_t)::value,
+                       S = decltype(ws_t)::value;
+        // tiles of up to 16x16: at most 64 threads with four pixels a lane, 128 with two
+        constexpr int kMaxT = P == 4 ? 64 : 128;
+        // resident CTAs per SM: the fused loss's 8192^2 / 2M 1378 us with 16 (64
+        // registers), 1436 with 14; with weight sums and indices eight views
+        // 401 with 14, 412 with 16 (spilling); 8x8 regions, 512^2 / 50k 26.8
+        // with 9, 27.8 with 8, 27.4 with 10 (767x1023 with opacities 63 / 65 / 69)
+        constexpr int kMinB = P == 4 ? (S ? 14 : 16) : 9;
+        return nt <= kMaxT ? raster_fwd_kernel<T, false, P, kMaxT, kMinB, O, F, S>
+                           : raster_fwd_kernel<T, false, P, 512, 2, O, F, S>;
+    };
+    auto pick = [&](auto ppl) -> K {
+        using std::false_type;
+        using std::true_type;
+        if (!fused)
+            return op ? sum(ppl, true_type{}, true_type{}, true_type{})
+                      : sum(ppl, false_type{}, true_type{}, true_type{});
+        return op    ? sum(ppl, true_type{}, true_type{}, false_type{})
+               : fin ? sum(ppl, false_type{}, true_type{}, false_type{})
+                     : sum(ppl, false_type{}, false_type{}, false_type{});
+    };
+    K fn;
+    if (ga) {  // (double: float has its own kernel above)
+        if constexpr (sizeof(T) == 4) return LIG_ERR_INVALID;
+        else
+            fn = small ? raster_fwd_kernel<T, true, 1, 256, FM>
+                       : raster_fwd_kernel<T, true, 1, 1024, 1>;
+    } else {
+        fn = ppl4 ? pick(std::integral_constant<int, 4>{}) : pick(std::integral_constant<int, 2>{});
+    }
     if (!set_dyn_smem((const void *)fn, sm)) return LIG_ERR_LAUNCH;
     int grid = geo.total_tiles();
     if (walk.work) {
@@ -2514,7 +2455,7 @@ int raster_fwd(const BatchGeo &geo, TileWalk walk, const int32_t *ids, const int
                             (const Rec<T> *)ws, (T *)img, (T *)wsum, ga ? (T *)dx : nullptr,
                             ga ? (T *)dy : nullptr, ga ? (T *)dxy : nullptr, fin, l2);
     int launches = 1;
-    if (l2.target || l2.target_u8) {
+    if (fused) {
         const TileChunks ch = tile_chunks(geo);
         double *chunk_sum = l2.tile_partial + geo.total_tiles();
         if (ch.chunk_off[geo.n_img] > 0)
