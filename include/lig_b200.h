@@ -493,6 +493,40 @@ int lig_adam_step_batch(int n_img, const int32_t *counts, float *params, const f
  * denominator on the device.  No reference counterpart (measurement aid). */
 int lig_probe_fp32(int blocks, int iters, float *out, void *stream);
 
+/* The fit engine's iteration behind the binning of a batch (fp32, Cholesky
+ * parameters, no opacities), in two calls on one workspace:
+ *
+ * lig_fit_forward_batch: lig_raster_fwd_l2_batch (target fp32, or bytes with
+ * target_u8) without final indices; leaves its records and cleared gradient
+ * sums in `workspace` (lig_raster_workspace_bytes) for the second call, and
+ * forms this step's Adam scalars in `scratch` (lig_adam_batch_scratch_bytes)
+ * as lig_adam_step_batch does: steps[i] counts an applied step; with
+ * LIG_STATUS_OVERFLOW in *status the step is skipped and *skipped counted.
+ * *skipped_host (pinned, device-accessible host memory) receives *skipped.
+ *
+ * lig_fit_backward_batch: lig_raster_bwd_diff_batch on the same lists, workspace
+ * and diff, lig_project_bwd_batch and the Adam update of the flat buffer
+ * params [means 2N | cholesky 3N | rgb 3N] (grads laid out likewise, written
+ * even when the update is skipped). */
+int lig_fit_forward_batch(int n_img, const int32_t *heights, const int32_t *widths,
+                          const int32_t *counts, int block_width, const int32_t *gaussian_ids_sorted,
+                          const int32_t *tile_bins, const int32_t *num_intersects,
+                          const int32_t *cum_tiles_hit, const float *xys, const float *conics,
+                          const float *colors, const void *target, int target_u8, int persistent,
+                          int32_t *work, void *workspace, size_t workspace_bytes,
+                          double *tile_partials, float *diff, float *loss, float *per_image,
+                          const int32_t *status, int32_t *steps, int32_t *skipped,
+                          int32_t *skipped_host, double lr, double beta1, double beta2,
+                          void *scratch, size_t scratch_bytes, void *stream);
+int lig_fit_backward_batch(int n_img, const int32_t *heights, const int32_t *widths,
+                           const int32_t *counts, int block_width,
+                           const int32_t *gaussian_ids_sorted, const int32_t *tile_bins,
+                           const int32_t *num_intersects, const int32_t *cum_tiles_hit,
+                           const float *diff, const float *grad_loss, int persistent,
+                           int32_t *work, void *workspace, size_t workspace_bytes, float *params,
+                           float *grads, float *exp_avg, float *exp_avg_sq, double beta1,
+                           double beta2, double eps, const void *scratch, void *stream);
+
 #ifdef __cplusplus
 }
 #endif

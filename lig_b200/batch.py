@@ -304,26 +304,19 @@ class BatchedFit:
         st = self._stream()
         tgt = self.target if target is None else target
         self._bin(st)
-        fwd = "lig_raster_fwd_l2_u8_batch" if tgt.dtype == torch.uint8 else "lig_raster_fwd_l2_batch"
-        call(fwd, _lib.LIG_F32, *L.args(), L.block, _p(self.gids),
-             _p(self.bins), _p(self.total), _p(self.cum), _p(self.xys), _p(self.con),
-             _p(self.rgbs), None, _p(tgt), int(self.persistent), _p(self.work),
-             _p(self.r_ws), self.r_ws.numel(), _p(self.partials), _p(self.img), None,
-             _p(self.loss), _p(self.per_image), st)
         # no opacities: the backward reads no final indices, so the forward
-        # neither tracks nor writes them
-        call("lig_raster_bwd_diff_batch", _lib.LIG_F32, *L.args(), L.block, _p(self.gids),
-             _p(self.bins), _p(self.total), _p(self.cum), _p(self.xys), _p(self.con),
-             _p(self.rgbs), None, None, _p(self.img), _p(self.one), 0.0,
-             int(self.persistent), _p(self.work), _p(self.r_ws), self.r_ws.numel(),
-             _p(self.v_xy), _p(self.v_abs), _p(self.v_con), _p(self.g_rgbs), None, st)
-        call("lig_project_bwd_batch", _lib.LIG_F32, *L.args(), 1, _p(self.chol), _p(self.means),
-             None, L.block, _p(self.v_xy), 2, _p(self.v_con), 3, _p(self.g_chol),
-             _p(self.g_means), st)
-        call("lig_adam_step_batch", L.n, L.args()[3], _p(self.flat), _p(self.grad), _p(self.m),
-             _p(self.v), self.lr, self.b1, self.b2, self.eps, _p(self.status), _p(self.steps),
-             _p(self.skipped), _p(self.adam_scratch), self.adam_scratch.numel(), st)
-        self.host_skipped.copy_(self.skipped, non_blocking=True)
+        # neither tracks nor writes them; its records serve the backward
+        call("lig_fit_forward_batch", *L.args(), L.block, _p(self.gids), _p(self.bins),
+             _p(self.total), _p(self.cum), _p(self.xys), _p(self.con), _p(self.rgbs), _p(tgt),
+             int(tgt.dtype == torch.uint8), int(self.persistent), _p(self.work), _p(self.r_ws),
+             self.r_ws.numel(), _p(self.partials), _p(self.img), _p(self.loss),
+             _p(self.per_image), _p(self.status), _p(self.steps), _p(self.skipped),
+             _p(self.host_skipped), self.lr, self.b1, self.b2, _p(self.adam_scratch),
+             self.adam_scratch.numel(), st)
+        call("lig_fit_backward_batch", *L.args(), L.block, _p(self.gids), _p(self.bins),
+             _p(self.total), _p(self.cum), _p(self.img), _p(self.one), int(self.persistent),
+             _p(self.work), _p(self.r_ws), self.r_ws.numel(), _p(self.flat), _p(self.grad),
+             _p(self.m), _p(self.v), self.b1, self.b2, self.eps, _p(self.adam_scratch), st)
 
     def _capture(self, target: Optional[torch.Tensor] = None):
         """Capture one iteration on a side stream.  capture_begin/end rather
