@@ -527,6 +527,28 @@ int lig_fit_backward_batch(int n_img, const int32_t *heights, const int32_t *wid
                            float *grads, float *exp_avg, float *exp_avg_sq, double beta1,
                            double beta2, double eps, const void *scratch, void *stream);
 
+/* A batch of decodes (fp32), projection to images: view i shows the set
+ * (in3[i], means[i], opac[i] or NULL, rgb[i]; chol[i]: Cholesky rows) of
+ * counts[i] Gaussians under origins[2i..], scales[2i..], as
+ * lig_project_fwd_view, on a heights[i] x widths[i] output.
+ * lig_views_project writes num_tiles_hit for every Gaussian (concatenated in
+ * view order), and xys, extents and, to ws (lig_raster_workspace_bytes), the
+ * raster records for those with tiles and each view's first: all that
+ * lig_bin_batch and lig_views_raster read.  lig_views_raster renders the lists
+ * from those records into imgs[i], each [heights[i]][widths[i]][3];
+ * with_opacities: some opac[i] was given.  The arrays of pointers, flags and
+ * numbers are host memory. */
+int lig_views_project(int n_img, const int32_t *heights, const int32_t *widths,
+                      const int32_t *counts, int block_width, const float *const *in3,
+                      const float *const *means, const float *const *opac,
+                      const float *const *rgb, const int32_t *chol, const double *origins,
+                      const double *scales, void *ws, size_t ws_bytes, float *xys,
+                      float *extents, int32_t *num_tiles_hit, void *stream);
+int lig_views_raster(int n_img, const int32_t *heights, const int32_t *widths,
+                     const int32_t *counts, int block_width, const int32_t *gaussian_ids,
+                     const int32_t *tile_bins, const int32_t *cum, int with_opacities,
+                     const void *ws, size_t ws_bytes, float *const *imgs, void *stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -139,34 +139,10 @@ __device__ __forceinline__ bool tame_cotangent(T a, T b, T c, T d) {
     return fabs(a) < (T)kTameCot && fabs(b) < (T)kTameCot && fabs(c) < (T)kTameCot &&
            fabs(d) < (T)kTameCot;
 }
-
-template <typename T, bool HALF, bool TAME = false>
-__global__ void pack_kernel(int n, const T *__restrict__ xys, const T *__restrict__ conics,
-                            const T *__restrict__ colors, const T *__restrict__ opac,
-                            Rec<T> *__restrict__ recs, T *__restrict__ zero, int zero_stride,
-                            uint32_t *__restrict__ ticket) {
-    if (ticket && blockIdx.x == 0 && threadIdx.x == 32) *ticket = 0;
-    if (sizeof(T) == 4 && blockIdx.x == 0 && threadIdx.x < 32) {
-        const uint32_t cut = alpha_cut_search();
-        if (threadIdx.x == 0) g_alpha_cut = cut;
-    }
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    if (zero) {
-        float4 *z = reinterpret_cast<float4 *>(zero + (size_t)i * zero_stride);
-        const int nv = zero_stride * (int)sizeof(T) / 16;
-        for (int k = 0; k < nv; ++k) z[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-    Rec<T> r;
-    r.x = xys[2 * i];
-    r.y = xys[2 * i + 1];
-    r.a = conics[3 * i];
-    r.b = conics[3 * i + 1];
-    r.c = conics[3 * i + 2];
-    r.o = opac ? opac[i] : (T)1;
-    r.r = colors[3 * i];
-    r.g = colors[3 * i + 1];
-    r.bl = colors[3 * i + 2];
+// Completes a record whose inputs are set: the culling data, and with HALF the
+// halved conic.
+template <typename T, bool HALF, bool TAME>
+__device__ __forceinline__ void finish_rec(Rec<T> &r) {
     r.thr = 0;
     double a = r.a, b = r.b, c = r.c, o = r.o;
     double det = a * c - b * b;
@@ -195,6 +171,104 @@ __global__ void pack_kernel(int n, const T *__restrict__ xys, const T *__restric
         r.a *= (T)0.5;
         r.c *= (T)0.5;
     }
+}
+
+
+template <typename T, bool HALF, bool TAME = false>
+__global__ void pack_kernel(int n, const T *__restrict__ xys, const T *__restrict__ conics,
+                            const T *__restrict__ colors, const T *__restrict__ opac,
+                            Rec<T> *__restrict__ recs, T *__restrict__ zero, int zero_stride,
+                            uint32_t *__restrict__ ticket) {
+    if (ticket && blockIdx.x == 0 && threadIdx.x == 32) *ticket = 0;
+    if (sizeof(T) == 4 && blockIdx.x == 0 && threadIdx.x < 32) {
+        const uint32_t cut = alpha_cut_search();
+        if (threadIdx.x == 0) g_alpha_cut = cut;
+    }
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    if (zero) {
+        float4 *z = reinterpret_cast<float4 *>(zero + (size_t)i * zero_stride);
+        const int nv = zero_stride * (int)sizeof(T) / 16;
+        for (int k = 0; k < nv; ++k) z[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    Rec<T> r;
+    r.x = xys[2 * i];
+    r.y = xys[2 * i + 1];
+    r.a = conics[3 * i];
+    r.b = conics[3 * i + 1];
+    r.c = conics[3 * i + 2];
+    r.o = opac ? opac[i] : (T)1;
+    r.r = colors[3 * i];
+    r.g = colors[3 * i + 1];
+    r.bl = colors[3 * i + 2];
+    finish_rec<T, HALF, TAME>(r);
+    recs[i] = r;
+}
+
+// The views of a batch of decodes, each with its own set and transform:
+// projection (as project_kernel's) and the forward's records in one launch, one
+// CTA per 256 Gaussians of one view.  A Gaussian outside its view costs its
+// input and a zero count: nothing reads its other outputs, except those of each
+// view's first, which phantom slots name (slot_id in binning.cu).
+// Bound by the records' fp64 and the reads of every Gaussian.  Eight views of
+// 500k Gaussians: 71 us, against 44 for eight projections, 51 for the colours'
+// copies and 54 for packing every record.
+struct ViewSet {
+    const float *in3, *means, *opac, *rgb;
+    float ox, oy, sx, sy;
+    int chol;
+};
+struct ViewSets {
+    int block_off[kMaxBatch + 1];
+    ViewSet v[kMaxBatch];
+};
+
+__global__ void __launch_bounds__(256)
+project_views_kernel(const BatchGeo geo, const ViewSets sets, float *__restrict__ xys,
+                     float *__restrict__ extents, int32_t *__restrict__ counts,
+                     Rec<float> *__restrict__ recs) {
+    if (blockIdx.x == 0 && threadIdx.x < 32) {
+        const uint32_t cut = alpha_cut_search();
+        if (threadIdx.x == 0) g_alpha_cut = cut;
+    }
+    const int im = BatchGeo::find(sets.block_off, geo.n_img, blockIdx.x);
+    const int k = (blockIdx.x - sets.block_off[im]) * blockDim.x + threadIdx.x;
+    const int i = geo.g_off[im] + k;
+    if (i >= geo.g_off[im + 1]) return;
+    const ViewSet &s = sets.v[im];
+    const View<float> view{s.ox, s.oy, s.sx, s.sy, true};
+    float cx, cy, cz;
+    input_cov<float, true>(s.chol != 0, s.in3, k, cx, cy, cz, view);
+    const float o = s.opac ? s.opac[k] : 1.f;
+    const float mx = (s.means[2 * k] - view.ox) * view.sx;
+    const float my = (s.means[2 * k + 1] - view.oy) * view.sy;
+    Rec<float> r;
+    float ex = 0, ey = 0;
+    r.a = r.b = r.c = 0;
+    const bool ok = cov2d_bounds(cx, cy, cz, o, r.a, r.b, r.c, ex, ey);
+    int32_t area = 0;
+    if (ok) {
+        int x0, y0, x1, y1;
+        tile_bbox(mx, my, ex, ey, (unsigned)geo.tbx[im], (unsigned)geo.tby(im), (unsigned)geo.B, x0,
+                  y0, x1, y1);
+        area = (int32_t)((unsigned)(x1 - x0) * (unsigned)(y1 - y0));
+    } else {
+        r.a = r.b = r.c = 0;
+    }
+    const bool hit = area > 0;
+    counts[i] = hit ? area : 0;
+    if (!hit && k != 0) return;
+    r.x = hit ? mx : 0.f;
+    r.y = hit ? my : 0.f;
+    xys[2 * i] = r.x;
+    xys[2 * i + 1] = r.y;
+    extents[2 * i] = hit ? ex : 0.f;
+    extents[2 * i + 1] = hit ? ey : 0.f;
+    r.o = o;
+    r.r = s.rgb[3 * k];
+    r.g = s.rgb[3 * k + 1];
+    r.bl = s.rgb[3 * k + 2];
+    finish_rec<float, true, false>(r);
     recs[i] = r;
 }
 
@@ -522,6 +596,11 @@ struct FwdAcc {
 // residual-correction step (Markstein): e = fma(-q, 255, b), t = fma(e, r, q)
 // — equal to the correctly rounded b / 255 for every byte b (checked against
 // the host's division for all 256 values), with no division.
+// A batch of decodes: each view's image is its own allocation.
+struct ViewImages {
+    float *img[kMaxBatch];
+};
+
 template <typename T> struct L2Fwd {
     const T *target;
     double *tile_partial;  // [total tiles]
@@ -581,7 +660,7 @@ __device__ __forceinline__ double fwd_write(const FwdAcc<T, GA> &acc, bool insid
     img[3 * pix] = acc.r;
     img[3 * pix + 1] = acc.g;
     img[3 * pix + 2] = acc.b;
-    wsum[pix] = acc.w;
+    if (wsum) wsum[pix] = acc.w;
     if (GA) {
 #pragma unroll
         for (int ch = 0; ch < 3; ++ch) {
@@ -846,6 +925,23 @@ raster_fwd_kernel(const BatchGeo geo, const int32_t *__restrict__ cum, int *work
         fwd_tile<T, GA, PPL, OP, FIN, WS>(tc, tile, ids, tile_bins, recs, img, wsum, odx, ody,
                                           odxy, final_idx, s_rec, l2, cut);
     }
+}
+
+// The sum forward of a batch of decodes, images only (no weight sums, no final
+// indices), each into its own allocation: eight views of 500k Gaussians 355 us,
+// against 401 with both, and no copies out of a shared buffer (55 us).
+template <int PPL, int MAXT, int MINB, bool OP>
+__global__ void __launch_bounds__(MAXT, MINB)
+raster_views_kernel(const BatchGeo geo, const int32_t *__restrict__ cum,
+                    const int32_t *__restrict__ ids, const int2 *__restrict__ tile_bins,
+                    const Rec<float> *__restrict__ recs, const ViewImages out) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    TileCtx tc = tile_ctx(geo, cum, nullptr, blockIdx.x);
+    tc.poff = 0;
+    fwd_tile<float, false, PPL, OP, false, false>(
+        tc, blockIdx.x, ids, tile_bins, recs, out.img[tc.im], nullptr, nullptr, nullptr, nullptr,
+        nullptr, reinterpret_cast<Rec<float> *>(smem_raw), L2Fwd<float>{nullptr, nullptr},
+        OP ? 0u : g_alpha_cut);
 }
 
 // Gradient-aware forward, float: 8x8 regions, the lane's two pixels (x, y) and
@@ -2929,6 +3025,78 @@ extern "C" int lig_raster_fwd_batch(int dtype, int n_img, const int32_t *heights
         return raster_fwd<double>(geo, walk, ids, bins, d_total, xys, con, col, op, ws, ws_bytes,
                                   img, wsum, dx, dy, dxy, fin, s);
     return LIG_ERR_INVALID;
+}
+
+extern "C" int lig_views_project(int n_img, const int32_t *heights, const int32_t *widths,
+                                 const int32_t *counts, int B, const float *const *in3,
+                                 const float *const *means, const float *const *opac,
+                                 const float *const *rgb, const int32_t *chol,
+                                 const double *origins, const double *scales, void *ws,
+                                 size_t ws_bytes, float *xys, float *extents,
+                                 int32_t *num_tiles_hit, void *stream) {
+    BatchGeo geo;
+    if (!in3 || !means || !opac || !rgb || !chol || !origins || !scales ||
+        !batch_geo(n_img, heights, widths, counts, B, geo))
+        return LIG_ERR_INVALID;
+    const int n = geo.total_points();
+    if (n > 0 && (!ws || !xys || !extents || !num_tiles_hit)) return LIG_ERR_INVALID;
+    if (ws_bytes < sizeof(Rec<float>) * (size_t)n) return LIG_ERR_WORKSPACE;
+    if ((reinterpret_cast<uintptr_t>(ws) & 15) != 0) return LIG_ERR_INVALID;  // 16-byte records
+    ViewSets sets;
+    sets.block_off[0] = 0;
+    for (int i = 0; i < n_img; ++i) {
+        const double ox = origins[2 * i], oy = origins[2 * i + 1];
+        const double sx = scales[2 * i], sy = scales[2 * i + 1];
+        if (!(sx > 0.0) || !(sy > 0.0) || !std::isfinite(sx) || !std::isfinite(sy) ||
+            !std::isfinite(ox) || !std::isfinite(oy) ||
+            (counts[i] > 0 && (!in3[i] || !means[i] || !rgb[i])))
+            return LIG_ERR_INVALID;
+        sets.block_off[i + 1] = sets.block_off[i] + (counts[i] + 255) / 256;
+        sets.v[i] = ViewSet{in3[i],    means[i],  opac[i],   rgb[i], (float)ox,
+                            (float)oy, (float)sx, (float)sy, chol[i]};
+    }
+    if (n == 0) return LIG_OK;
+    project_views_kernel<<<sets.block_off[n_img], 256, 0, (cudaStream_t)stream>>>(
+        geo, sets, xys, extents, num_tiles_hit, (Rec<float> *)ws);
+    note_launches(1);
+    LIG_LAUNCH_CHECK();
+    return LIG_OK;
+}
+
+extern "C" int lig_views_raster(int n_img, const int32_t *heights, const int32_t *widths,
+                                const int32_t *counts, int B, const int32_t *ids,
+                                const int32_t *bins, const int32_t *cum, int with_opacities,
+                                const void *ws, size_t ws_bytes, float *const *imgs,
+                                void *stream) {
+    BatchGeo geo;
+    if (!bins || !cum || !imgs || !batch_geo(n_img, heights, widths, counts, B, geo))
+        return LIG_ERR_INVALID;
+    const int n = geo.total_points();
+    if (n > 0 && (!ids || !ws)) return LIG_ERR_INVALID;
+    if (ws_bytes < sizeof(Rec<float>) * (size_t)n) return LIG_ERR_WORKSPACE;
+    if ((reinterpret_cast<uintptr_t>(ws) & 15) != 0) return LIG_ERR_INVALID;
+    ViewImages out;
+    for (int i = 0; i < n_img; ++i) {
+        if (!imgs[i]) return LIG_ERR_INVALID;
+        out.img[i] = imgs[i];
+    }
+    // pixels a lane and CTAs per SM as in raster_fwd
+    const bool ppl4 = B > 8 && geo.total_tiles() >= LIG_RASTER_PPL4_MIN_TILES;
+    const int nt = 32 * Regions::make(ppl4 ? 3 : 1, B).count;
+    const size_t sm = (size_t)nt * sizeof(Rec<float>);
+    auto pick = [&](auto op_t) {
+        constexpr bool O = decltype(op_t)::value;
+        return ppl4 ? (nt <= 64 ? raster_views_kernel<4, 64, 16, O> : raster_views_kernel<4, 512, 2, O>)
+                    : (nt <= 128 ? raster_views_kernel<2, 128, 9, O>
+                                 : raster_views_kernel<2, 512, 2, O>);
+    };
+    auto fn = with_opacities ? pick(std::true_type{}) : pick(std::false_type{});
+    if (!set_dyn_smem((const void *)fn, sm)) return LIG_ERR_LAUNCH;
+    fn<<<geo.total_tiles(), nt, sm, (cudaStream_t)stream>>>(
+        geo, cum, ids, (const int2 *)bins, (const Rec<float> *)ws, out);
+    note_launches(1);
+    LIG_LAUNCH_CHECK();
+    return LIG_OK;
 }
 
 extern "C" int lig_raster_bwd_l2_batch(int dtype, int n_img, const int32_t *heights,

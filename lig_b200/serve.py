@@ -29,6 +29,7 @@ request's device work (a CUDA event on its stream).
 from __future__ import annotations
 
 import collections
+import ctypes
 import math
 import sys
 import threading
@@ -87,10 +88,10 @@ def render_views(views, block: int = 16) -> List[torch.Tensor]:
     """Decode several views in one launch chain per stage.
 
     views: [(GaussianSet, out_h, out_w, origin, scale), ...] (at most
-    LIG_MAX_BATCH).  Each view is projected (lig_project_fwd_view) into its
-    slice of concatenated per-Gaussian arrays; one batched prefix sum,
-    binning (lig_bin_batch: a single stable sort, tile keys offset per view)
-    and forward (lig_raster_fwd_batch) then render every view.  A view's tile
+    LIG_MAX_BATCH).  The views are projected into concatenated per-Gaussian
+    arrays (lig_views_project); one batched prefix sum, binning
+    (lig_bin_batch: tile keys offset per view) and forward (lig_views_raster,
+    each image its own allocation) then render every view.  A view's tile
     lists are exactly its single-view lists, so each [out_h, out_w, 3] image
     equals render_view's bit for bit.  Runs on the current stream; one host
     synchronisation (the intersection count sizes the sort)."""
@@ -102,26 +103,26 @@ def render_views(views, block: int = 16) -> List[torch.Tensor]:
     N = L.points
     f32 = dict(dtype=torch.float32, device=dev)
     xys, ext = torch.empty(max(N, 1), 2, **f32), torch.empty(max(N, 1), 2, **f32)
-    con, rgbs = torch.empty(max(N, 1), 3, **f32), torch.empty(max(N, 1), 3, **f32)
     cnt = torch.empty(max(N, 1), dtype=torch.int32, device=dev)
-    any_op = any(v[0].opacities is not None for v in views)
-    opac = torch.ones(max(N, 1), **f32) if any_op else None
+    rws = torch.empty(_lib.lib.lig_raster_workspace_bytes(_lib.LIG_F32, N), dtype=torch.uint8,
+                      device=dev)
     st = ops._stream(dev)
     p = ops._p
-    for k, (gs, h, w, origin, scale) in enumerate(views):
-        a, b = L.g_off[k], L.g_off[k + 1]
-        if b == a:
-            continue
-        # inputs held in locals: a converted copy must outlive the launch
-        o = None if gs.opacities is None else ops._c(gs.opacities, torch.float32)
-        in3, mu = ops._c(gs.chol, torch.float32), ops._c(gs.means, torch.float32)
-        ops.call("lig_project_fwd_view", _lib.LIG_F32, b - a, int(gs.cholesky), p(in3), p(mu),
-                 p(o), int(h), int(w), int(block), float(origin[0]), float(origin[1]),
-                 float(scale[0]), float(scale[1]), p(xys[a:b]), p(ext[a:b]), p(con[a:b]),
-                 p(cnt[a:b]), st)
-        rgbs[a:b].copy_(gs.rgbs)
-        if o is not None:
-            opac[a:b].copy_(o)
+    # the views' sets as fp32 rows on this device (held until the launch)
+    def rows(gs):
+        cast = lambda t: t.to(dev, torch.float32).contiguous()  # noqa: E731
+        op = gs.opacities
+        return (cast(gs.chol), cast(gs.means), None if op is None else cast(op.expand(gs.n)),
+                cast(gs.rgbs.expand(gs.n, 3)))
+
+    sets = [rows(v[0]) if v[0].n else (None,) * 4 for v in views]
+    ptrs = [(ctypes.c_void_p * L.n)(*map(p, col)) for col in zip(*sets)]
+    chol = (ctypes.c_int32 * L.n)(*(int(v[0].cholesky) for v in views))
+    origins = (ctypes.c_double * (2 * L.n))(*(float(v[3][k]) for v in views for k in (0, 1)))
+    scales = (ctypes.c_double * (2 * L.n))(*(float(v[4][k]) for v in views for k in (0, 1)))
+    ref = lambda a: ctypes.cast(a, ctypes.c_void_p)  # noqa: E731
+    ops.call("lig_views_project", *L.args(), L.block, *map(ref, ptrs), ref(chol), ref(origins),
+             ref(scales), p(rws), rws.numel(), p(xys), p(ext), p(cnt), st)
     cum = torch.empty(max(N, 1), dtype=torch.int32, device=dev)
     total = torch.zeros(1, dtype=torch.int32, device=dev)
     if N > 0:
@@ -136,15 +137,11 @@ def render_views(views, block: int = 16) -> List[torch.Tensor]:
     status = torch.empty(1, dtype=torch.int32, device=dev)
     ops.call("lig_bin_batch", _lib.LIG_F32, *L.args(), L.block, p(xys), p(ext), p(cum),
              p(total), cap, p(bws), bws.numel(), p(gids), p(bins), p(status), st)
-    rws = torch.empty(_lib.lib.lig_raster_workspace_bytes(_lib.LIG_F32, N), dtype=torch.uint8,
-                      device=dev)
-    img = torch.empty(max(L.pixels, 1), 3, **f32)
-    wsum = torch.empty(max(L.pixels, 1), **f32)
-    fin = torch.empty(max(L.pixels, 1), dtype=torch.int32, device=dev)
-    ops.call("lig_raster_fwd_batch", _lib.LIG_F32, *L.args(), L.block, p(gids), p(bins),
-             p(total), p(cum), p(xys), p(con), p(rgbs), p(opac), 0, None, p(rws), rws.numel(),
-             p(img), p(wsum), None, None, None, p(fin), st)
-    return [L.image(img, k).clone() for k in range(L.n)]
+    imgs = [torch.empty(int(v[1]), int(v[2]), 3, **f32) for v in views]
+    out = (ctypes.c_void_p * L.n)(*map(p, imgs))
+    ops.call("lig_views_raster", *L.args(), L.block, p(gids), p(bins), p(cum),
+             int(any(s[2] is not None for s in sets)), p(rws), rws.numel(), ref(out), st)
+    return imgs
 
 
 # ---------------------------------------------------------------- requests
