@@ -849,7 +849,8 @@ tile_sort_long_kernel(BatchGeo geo, const uint32_t *__restrict__ tcount,
 // While the tile counters fit an SM's shared memory (up to kHistMaxTiles), the
 // global atomics of count and scatter — what those kernels wait for: 6M slots
 // at 2048^2 / 1M Gaussians took 37 and 63 us, at any enumeration cost — become
-// shared-memory atomics.  CTA c of `parts` takes the c-th run of Gaussians:
+// shared-memory atomics.  CTA c of `parts` takes every parts-th 32 Gaussians from
+// the c-th on, so that images with more slots a Gaussian are shared by all:
 //   1. tile_hist_kernel: its slots' tile counts in shared memory, written as
 //      row c of hist [parts][tiles];
 //   2. hist_prefix_kernel: per tile the exclusive prefix over the rows (in
@@ -859,47 +860,44 @@ tile_sort_long_kernel(BatchGeo geo, const uint32_t *__restrict__ tcount,
 //      one shared atomic per slot;
 // then the per-tile sort as above.  Count, prefix and scatter against global
 // atomics: 512^2 / 50k 11.5 us against 23, 16 images of 1.1M Gaussians 56
-// against 99, 2048^2 / 1M 88 against 100, eight views of 500k 139 against 236;
-// what is left is the enumeration and the scattered 4-byte stores.  Slots past the capacity are dropped by
-// position (outputs are incomplete then, and flagged).
+// against 99, 2048^2 / 1M 88 against 100, eight views of 500k 121 against 236
+// (139 with one run of consecutive Gaussians per CTA: the larger views waited);
+// what is left is the enumeration and the scattered 4-byte stores.  Slots past
+// the capacity are dropped by position (outputs are incomplete then, and flagged).
 constexpr int kHistThreads = 1024;
 constexpr int kHistMaxTiles = 48 * 1024;  // 192 KB of counters
 constexpr int kHistTwoTiles = 24 * 1024;  // two CTAs' counters fit an SM up to here
 constexpr int kHistMaxParts = 2 * 148;
 
-// Rows of the histogram (CTAs): LIG_BIN_HIST_RUN Gaussians each, up to one per
+// Rows of the histogram (CTAs): at least LIG_BIN_HIST_RUN Gaussians each, up to one per
 // SM; two per SM from kHistTwoMinPoints Gaussians on, where the second CTA's
 // warps hide more of the enumeration than the longer prefix costs (eight
-// views, 4M Gaussians / 17k tiles: 174 -> 139 us; 2048^2 / 1M: 87 -> 88).
+// views, 4M Gaussians / 17k tiles: 174 -> 139 us, on runs; 2048^2 / 1M 88 with
+// one, 87 with two; 16 images of 1.1M Gaussians 57 and 55).
 constexpr int kHistTwoMinPoints = 2000000;
 inline int hist_parts(int n, size_t tiles) {
     const bool two = tiles <= kHistTwoTiles && n >= kHistTwoMinPoints;
     return std::min(std::max(n / LIG_BIN_HIST_RUN, 1), two ? kHistMaxParts : kHistMaxParts / 2);
 }
 
-// f(slot, tile key, sort value) for every slot of Gaussians [g0, g1), by the
-// CTA's warps.
+// f(slot, tile key, sort value) for every slot of the CTA's Gaussians.
 template <typename T, typename F>
-__device__ __forceinline__ void for_each_slot_of_run(int g0, int g1, const T *__restrict__ xys,
+__device__ __forceinline__ void for_each_slot_of_cta(int n, const T *__restrict__ xys,
                                                      const T *__restrict__ ext,
                                                      const int32_t *__restrict__ cum,
                                                      const BatchGeo &geo,
                                                      int32_t *__restrict__ status, F f) {
     const int lane = threadIdx.x & 31;
-    for (int64_t g = g0 + (int)(threadIdx.x >> 5) * 32; g < g1; g += blockDim.x) {
+    const int64_t chunk = (int64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+    for (int64_t g = chunk * 32; g < n; g += (int64_t)gridDim.x * blockDim.x) {
         SlotWarp sw;
-        if (!slot_warp<T>(g, g1, xys, ext, cum, geo, status, sw)) continue;
+        if (!slot_warp<T>(g, n, xys, ext, cum, geo, status, sw)) continue;
         for (int s0 = 0; s0 < sw.total; s0 += 32) {
             int slot;
             uint32_t key, val;
             if (slot_at(sw, s0 + lane, slot, key, val)) f(slot, key, val);
         }
     }
-}
-
-__device__ __forceinline__ void run_of_part(int n, int &g0, int &g1) {
-    g0 = (int)((int64_t)n * blockIdx.x / gridDim.x);
-    g1 = (int)((int64_t)n * (blockIdx.x + 1) / gridDim.x);
 }
 
 // clear: words cleared for the later kernels (the scan's state, the long-tile
@@ -917,9 +915,7 @@ tile_hist_kernel(int n, int tiles, const T *__restrict__ xys, const T *__restric
     }
     for (int t = threadIdx.x; t < tiles; t += blockDim.x) s_tile[t] = 0;
     __syncthreads();
-    int g0, g1;
-    run_of_part(n, g0, g1);
-    for_each_slot_of_run<T>(g0, g1, xys, ext, cum, geo, status,
+    for_each_slot_of_cta<T>(n, xys, ext, cum, geo, status,
                             [&](int, uint32_t key, uint32_t) { atomicAdd(&s_tile[key], 1u); });
     __syncthreads();
     uint32_t *row = hist + (size_t)blockIdx.x * tiles;
@@ -973,9 +969,7 @@ hist_scatter_kernel(int n, int tiles, const T *__restrict__ xys, const T *__rest
     for (int t = threadIdx.x; t < tiles; t += blockDim.x)
         s_tile[t] = tend[t] - tcount[t] + row[t];
     __syncthreads();
-    int g0, g1;
-    run_of_part(n, g0, g1);
-    for_each_slot_of_run<T>(g0, g1, xys, ext, cum, geo, nullptr,
+    for_each_slot_of_cta<T>(n, xys, ext, cum, geo, nullptr,
                             [&](int, uint32_t key, uint32_t val) {
                                 const uint32_t pos = atomicAdd(&s_tile[key], 1u);
                                 if (pos < (uint32_t)capacity) out[pos] = val;
@@ -1005,7 +999,7 @@ bin_small_kernel(int n, int tiles, const T *__restrict__ xys, const T *__restric
     }
     s_cnt[tid] = 0;
     __syncthreads();
-    for_each_slot_of_run<T>(0, n, xys, ext, cum, geo, status,
+    for_each_slot_of_cta<T>(n, xys, ext, cum, geo, status,
                             [&](int, uint32_t key, uint32_t) { atomicAdd(&s_cnt[key], 1u); });
     __syncthreads();
     const uint32_t c = s_cnt[tid];
@@ -1017,7 +1011,7 @@ bin_small_kernel(int n, int tiles, const T *__restrict__ xys, const T *__restric
         tile_bins[tid] = c ? make_int2(a, b) : make_int2(0, 0);
     }
     __syncthreads();
-    for_each_slot_of_run<T>(0, n, xys, ext, cum, geo, nullptr,
+    for_each_slot_of_cta<T>(n, xys, ext, cum, geo, nullptr,
                             [&](int, uint32_t key, uint32_t val) {
                                 const uint32_t pos = atomicAdd(&s_cur[key], 1u);
                                 if (pos < (uint32_t)capacity) vals[pos] = val;
