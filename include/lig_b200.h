@@ -493,12 +493,17 @@ int lig_adam_step_batch(int n_img, const int32_t *counts, float *params, const f
  * denominator on the device.  No reference counterpart (measurement aid). */
 int lig_probe_fp32(int blocks, int iters, float *out, void *stream);
 
-/* The fit engine's iteration behind the binning of a batch (fp32, Cholesky
- * parameters, no opacities), in two calls on one workspace:
+/* The fit engine's iteration of a batch (fp32, Cholesky parameters, no
+ * opacities), in three calls on one workspace:
+ *
+ * lig_fit_bin_batch: lig_project_fwd_batch of the flat buffer params [means 2N |
+ * cholesky 3N | rgb 3N], lig_cumsum_tiles and lig_bin_batch; leaves the raster
+ * records and cleared gradient sums in `workspace` (lig_raster_workspace_bytes)
+ * and tile_partials ready for the next calls.  xys and extents are written for
+ * the Gaussians with tiles (and each image's first) only.
  *
  * lig_fit_forward_batch: lig_raster_fwd_l2_batch (target fp32, or bytes with
- * target_u8) without final indices; leaves its records and cleared gradient
- * sums in `workspace` (lig_raster_workspace_bytes) for the second call, and
+ * target_u8) of those records without final indices, and
  * forms this step's Adam scalars in `scratch` (lig_adam_batch_scratch_bytes)
  * as lig_adam_step_batch does: steps[i] counts an applied step; with
  * LIG_STATUS_OVERFLOW in *status the step is skipped and *skipped counted.
@@ -506,13 +511,21 @@ int lig_probe_fp32(int blocks, int iters, float *out, void *stream);
  *
  * lig_fit_backward_batch: lig_raster_bwd_diff_batch on the same lists, workspace
  * and diff, lig_project_bwd_batch and the Adam update of the flat buffer
- * params [means 2N | cholesky 3N | rgb 3N] (grads laid out likewise, written
+ * params (grads laid out likewise, written
  * even when the update is skipped). */
+int lig_fit_bin_batch(int n_img, const int32_t *heights, const int32_t *widths,
+                      const int32_t *counts, int block_width, const float *params,
+                      void *workspace, size_t workspace_bytes, double *tile_partials, float *xys,
+                      float *extents, int32_t *num_tiles_hit, int32_t *cum_tiles_hit,
+                      int32_t *num_intersects, void *cumsum_workspace,
+                      size_t cumsum_workspace_bytes, int capacity, void *bin_workspace,
+                      size_t bin_workspace_bytes, int32_t *gaussian_ids_sorted,
+                      int32_t *tile_bins, int32_t *status, void *stream);
 int lig_fit_forward_batch(int n_img, const int32_t *heights, const int32_t *widths,
                           const int32_t *counts, int block_width, const int32_t *gaussian_ids_sorted,
                           const int32_t *tile_bins, const int32_t *num_intersects,
-                          const int32_t *cum_tiles_hit, const float *xys, const float *conics,
-                          const float *colors, const void *target, int target_u8, int persistent,
+                          const int32_t *cum_tiles_hit, const void *target, int target_u8,
+                          int persistent,
                           int32_t *work, void *workspace, size_t workspace_bytes,
                           double *tile_partials, float *diff, float *loss, float *per_image,
                           const int32_t *status, int32_t *steps, int32_t *skipped,

@@ -96,8 +96,10 @@ SIGNATURES = {
     "lig_project_fwd_view": (I, [I, I, I, P, P, P, I, I, I, D, D, D, D, P, P, P, P, P]),
     "lig_views_project": (I, [I, P, P, P, I, P, P, P, P, P, P, P, P, SZ, P, P, P, P]),
     "lig_views_raster": (I, [I, P, P, P, I, P, P, P, I, P, SZ, P, P]),
-    "lig_fit_forward_batch": (I, [I, P, P, P, I, P, P, P, P, P, P, P, P, I, I, P, P, SZ, P, P, P,
-                                  P, P, P, P, P, D, D, D, P, SZ, P]),
+    "lig_fit_bin_batch": (I, [I, P, P, P, I, P, P, SZ, P, P, P, P, P, P, P, SZ, I, P, SZ, P, P, P,
+                              P]),
+    "lig_fit_forward_batch": (I, [I, P, P, P, I, P, P, P, P, P, I, I, P, P, SZ, P, P, P, P, P, P,
+                                  P, P, D, D, D, P, SZ, P]),
     "lig_fit_backward_batch": (I, [I, P, P, P, I, P, P, P, P, P, P, I, P, P, SZ, P, P, P, P, D, D,
                                    D, P, P]),
     "lig_adam_step_batch": (I, [I, P, P, P, P, P, D, D, D, D, P, P, P, P, SZ, P]),

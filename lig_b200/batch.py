@@ -303,11 +303,15 @@ class BatchedFit:
         L = self.L
         st = self._stream()
         tgt = self.target if target is None else target
-        self._bin(st)
+        call("lig_fit_bin_batch", *L.args(), L.block, _p(self.flat), _p(self.r_ws),
+             self.r_ws.numel(), _p(self.partials), _p(self.xys), _p(self.ext), _p(self.cnt),
+             _p(self.cum), _p(self.total), _p(self.cs_ws), self.cs_ws.numel(), self.capacity,
+             _p(self.bin_ws), self.bin_ws.numel(), _p(self.gids), _p(self.bins), _p(self.status),
+             st)
         # no opacities: the backward reads no final indices, so the forward
         # neither tracks nor writes them; its records serve the backward
         call("lig_fit_forward_batch", *L.args(), L.block, _p(self.gids), _p(self.bins),
-             _p(self.total), _p(self.cum), _p(self.xys), _p(self.con), _p(self.rgbs), _p(tgt),
+             _p(self.total), _p(self.cum), _p(tgt),
              int(tgt.dtype == torch.uint8), int(self.persistent), _p(self.work), _p(self.r_ws),
              self.r_ws.numel(), _p(self.partials), _p(self.img), _p(self.loss),
              _p(self.per_image), _p(self.status), _p(self.steps), _p(self.skipped),

@@ -1111,7 +1111,7 @@ template <typename T>
 int run_bin_scatter(const BatchGeo &geo, const void *xys, const void *ext, const int32_t *cum,
                     const int32_t *d_total, int capacity, void *ws, size_t ws_bytes,
                     int32_t *gid_sorted, int32_t *tile_bins, int64_t *isect, int32_t *gids,
-                    int64_t *isect_sorted, int32_t *status, cudaStream_t s) {
+                    int64_t *isect_sorted, int32_t *status, cudaStream_t s, bool status_clear) {
     const int n = geo.total_points();
     const int T_ = geo.total_tiles();
     ScatterPlan p = make_scatter_plan(n, T_);
@@ -1131,7 +1131,7 @@ int run_bin_scatter(const BatchGeo &geo, const void *xys, const void *ext, const
         LIG_LAUNCH_CHECK();
         return LIG_OK;
     }
-    cudaMemsetAsync(status, 0, sizeof(int32_t), s);
+    if (!status_clear) cudaMemsetAsync(status, 0, sizeof(int32_t), s);
     if (n == 0 || capacity == 0) {
         cudaMemsetAsync(tile_bins, 0, sizeof(int32_t) * 2 * (size_t)T_, s);
         flag_overflow_kernel<<<1, 1, 0, s>>>(d_total, capacity, status);
@@ -1191,10 +1191,11 @@ template <typename T>
 int run_bin(const BatchGeo &geo, const void *xys, const void *ext, const int32_t *cum,
             const int32_t *d_total, int capacity, void *ws, size_t ws_bytes, int32_t *gid_sorted,
             int32_t *tile_bins, int64_t *isect, int32_t *gids, int64_t *isect_sorted,
-            int32_t *status, cudaStream_t s) {
+            int32_t *status, cudaStream_t s, bool status_clear = false) {
     if (LIG_BIN_SCATTER)
         return run_bin_scatter<T>(geo, xys, ext, cum, d_total, capacity, ws, ws_bytes,
-                                  gid_sorted, tile_bins, isect, gids, isect_sorted, status, s);
+                                  gid_sorted, tile_bins, isect, gids, isect_sorted, status, s,
+                                  status_clear);
     const int n = geo.total_points();
     const int T_ = geo.total_tiles();
     BinPlan p = make_plan(capacity, T_);
@@ -1272,6 +1273,16 @@ int run_bin(const BatchGeo &geo, const void *xys, const void *ext, const int32_t
     note_launches(isect_sorted ? 2 : 1);
     LIG_LAUNCH_CHECK();
     return LIG_OK;
+}
+
+int scan_and_bin(const BatchGeo &geo, const float *xys, const float *ext, const int32_t *counts,
+                 int32_t *cum, int32_t *total, void *scan_ws, int capacity, void *ws,
+                 size_t ws_bytes, int32_t *ids, int32_t *bins, int32_t *status, cudaStream_t s) {
+    const int rc = device_scan((const uint32_t *)counts, (uint32_t *)cum, geo.total_points(), true,
+                               (uint64_t *)scan_ws, total, s, /*zeroed=*/true);
+    if (rc) return rc;
+    return run_bin<float>(geo, xys, ext, cum, total, capacity, ws, ws_bytes, ids, bins, nullptr,
+                          nullptr, nullptr, status, s, /*status_clear=*/true);
 }
 
 }  // namespace lig

@@ -148,6 +148,12 @@ struct BatchGeo {
     }
 };
 
+// The inclusive scan of the counts and the binning (binning.cu), where the
+// caller's launch has cleared the scan's workspace and *status.
+int scan_and_bin(const BatchGeo &geo, const float *xys, const float *ext, const int32_t *counts,
+                 int32_t *cum, int32_t *total, void *scan_ws, int capacity, void *ws,
+                 size_t ws_bytes, int32_t *ids, int32_t *bins, int32_t *status, cudaStream_t s);
+
 // Process-wide count of kernel launches issued by this library.
 void note_launches(int n);
 

@@ -139,6 +139,13 @@ __device__ __forceinline__ bool tame_cotangent(T a, T b, T c, T d) {
     return fabs(a) < (T)kTameCot && fabs(b) < (T)kTameCot && fabs(c) < (T)kTameCot &&
            fabs(d) < (T)kTameCot;
 }
+__device__ __forceinline__ void publish_alpha_cut() {  // first warp of the grid
+    if (blockIdx.x == 0 && threadIdx.x < 32) {
+        const uint32_t cut = alpha_cut_search();
+        if (threadIdx.x == 0) g_alpha_cut = cut;
+    }
+}
+
 // Completes a record whose inputs are set: the culling data, and with HALF the
 // halved conic.
 template <typename T, bool HALF, bool TAME>
@@ -180,10 +187,7 @@ __global__ void pack_kernel(int n, const T *__restrict__ xys, const T *__restric
                             Rec<T> *__restrict__ recs, T *__restrict__ zero, int zero_stride,
                             uint32_t *__restrict__ ticket) {
     if (ticket && blockIdx.x == 0 && threadIdx.x == 32) *ticket = 0;
-    if (sizeof(T) == 4 && blockIdx.x == 0 && threadIdx.x < 32) {
-        const uint32_t cut = alpha_cut_search();
-        if (threadIdx.x == 0) g_alpha_cut = cut;
-    }
+    if (sizeof(T) == 4) publish_alpha_cut();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     if (zero) {
@@ -205,11 +209,56 @@ __global__ void pack_kernel(int n, const T *__restrict__ xys, const T *__restric
     recs[i] = r;
 }
 
-// The views of a batch of decodes, each with its own set and transform:
-// projection (as project_kernel's) and the forward's records in one launch, one
-// CTA per 256 Gaussians of one view.  A Gaussian outside its view costs its
-// input and a zero count: nothing reads its other outputs, except those of each
-// view's first, which phantom slots name (slot_id in binning.cu).
+// Projection (as project_fwd_kernel's) and the forward's record of Gaussian k of
+// a set, number i of the batch, in image im.  A Gaussian outside its image
+// leaves a zero count only: nothing reads its other outputs, except those of
+// each image's first, which phantom slots name (slot_id in binning.cu).
+template <bool VIEW>
+__device__ __forceinline__ void project_rec(const BatchGeo &geo, int im, int i, int k, bool chol,
+                                            const float *in3, const float *means, float o,
+                                            const float *rgb, const View<float> &view,
+                                            float *__restrict__ xys, float *__restrict__ extents,
+                                            int32_t *__restrict__ counts,
+                                            Rec<float> *__restrict__ recs) {
+    float cx, cy, cz;
+    input_cov<float, VIEW>(chol, in3, k, cx, cy, cz, view);
+    float mx = means[2 * k], my = means[2 * k + 1];
+    if constexpr (VIEW) {
+        mx = (mx - view.ox) * view.sx;
+        my = (my - view.oy) * view.sy;
+    }
+    Rec<float> r;
+    float ex = 0, ey = 0;
+    r.a = r.b = r.c = 0;
+    const bool ok = cov2d_bounds(cx, cy, cz, o, r.a, r.b, r.c, ex, ey);
+    int32_t area = 0;
+    if (ok) {
+        int x0, y0, x1, y1;
+        tile_bbox(mx, my, ex, ey, (unsigned)geo.tbx[im], (unsigned)geo.tby(im), (unsigned)geo.B, x0,
+                  y0, x1, y1);
+        area = (int32_t)((unsigned)(x1 - x0) * (unsigned)(y1 - y0));
+    } else {
+        r.a = r.b = r.c = 0;
+    }
+    const bool hit = area > 0;
+    counts[i] = hit ? area : 0;
+    if (!hit && i != geo.g_off[im]) return;
+    r.x = hit ? mx : 0.f;
+    r.y = hit ? my : 0.f;
+    xys[2 * i] = r.x;
+    xys[2 * i + 1] = r.y;
+    extents[2 * i] = hit ? ex : 0.f;
+    extents[2 * i + 1] = hit ? ey : 0.f;
+    r.o = o;
+    r.r = rgb[3 * k];
+    r.g = rgb[3 * k + 1];
+    r.bl = rgb[3 * k + 2];
+    finish_rec<float, true, false>(r);
+    recs[i] = r;
+}
+
+// The views of a batch of decodes, each with its own set and transform, in one
+// launch, one CTA per 256 Gaussians of one view.
 // Bound by the records' fp64 and the reads of every Gaussian.  Eight views of
 // 500k Gaussians: 71 us, against 44 for eight projections, 51 for the colours'
 // copies and 54 for packing every record.
@@ -227,49 +276,40 @@ __global__ void __launch_bounds__(256)
 project_views_kernel(const BatchGeo geo, const ViewSets sets, float *__restrict__ xys,
                      float *__restrict__ extents, int32_t *__restrict__ counts,
                      Rec<float> *__restrict__ recs) {
-    if (blockIdx.x == 0 && threadIdx.x < 32) {
-        const uint32_t cut = alpha_cut_search();
-        if (threadIdx.x == 0) g_alpha_cut = cut;
-    }
+    publish_alpha_cut();
     const int im = BatchGeo::find(sets.block_off, geo.n_img, blockIdx.x);
     const int k = (blockIdx.x - sets.block_off[im]) * blockDim.x + threadIdx.x;
     const int i = geo.g_off[im] + k;
     if (i >= geo.g_off[im + 1]) return;
     const ViewSet &s = sets.v[im];
     const View<float> view{s.ox, s.oy, s.sx, s.sy, true};
-    float cx, cy, cz;
-    input_cov<float, true>(s.chol != 0, s.in3, k, cx, cy, cz, view);
-    const float o = s.opac ? s.opac[k] : 1.f;
-    const float mx = (s.means[2 * k] - view.ox) * view.sx;
-    const float my = (s.means[2 * k + 1] - view.oy) * view.sy;
-    Rec<float> r;
-    float ex = 0, ey = 0;
-    r.a = r.b = r.c = 0;
-    const bool ok = cov2d_bounds(cx, cy, cz, o, r.a, r.b, r.c, ex, ey);
-    int32_t area = 0;
-    if (ok) {
-        int x0, y0, x1, y1;
-        tile_bbox(mx, my, ex, ey, (unsigned)geo.tbx[im], (unsigned)geo.tby(im), (unsigned)geo.B, x0,
-                  y0, x1, y1);
-        area = (int32_t)((unsigned)(x1 - x0) * (unsigned)(y1 - y0));
-    } else {
-        r.a = r.b = r.c = 0;
+    project_rec<true>(geo, im, i, k, s.chol != 0, s.in3, s.means, s.opac ? s.opac[k] : 1.f, s.rgb,
+                      view, xys, extents, counts, recs);
+}
+
+// The fit step's first kernel: projection and records, the backward's gradient
+// sums cleared, and the words that the scan, the binning and the loss launch
+// start from.
+// HBM-bound.  8192^2 / 2M: 51 us (132 B a Gaussian: 40), against 18 + 37 for
+// projection and packing; 512^2 / 50k: the step 104 -> 96 us, three launches fewer.
+__global__ void __launch_bounds__(256)
+fit_project_kernel(const BatchGeo geo, int n, const float *__restrict__ params,
+                   float *__restrict__ xys, float *__restrict__ extents,
+                   int32_t *__restrict__ counts, Rec<float> *__restrict__ recs,
+                   float4 *__restrict__ sums, uint32_t *__restrict__ scan_state, int n_state,
+                   int32_t *__restrict__ status, uint32_t *__restrict__ ticket) {
+    publish_alpha_cut();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n_state) scan_state[i] = 0;
+    if (i == 0) {
+        *status = 0;
+        *ticket = 0;
     }
-    const bool hit = area > 0;
-    counts[i] = hit ? area : 0;
-    if (!hit && k != 0) return;
-    r.x = hit ? mx : 0.f;
-    r.y = hit ? my : 0.f;
-    xys[2 * i] = r.x;
-    xys[2 * i + 1] = r.y;
-    extents[2 * i] = hit ? ex : 0.f;
-    extents[2 * i + 1] = hit ? ey : 0.f;
-    r.o = o;
-    r.r = s.rgb[3 * k];
-    r.g = s.rgb[3 * k + 1];
-    r.bl = s.rgb[3 * k + 2];
-    finish_rec<float, true, false>(r);
-    recs[i] = r;
+    if (i >= n) return;
+    sums[2 * (size_t)i] = sums[2 * (size_t)i + 1] = make_float4(0.f, 0.f, 0.f, 0.f);
+    project_rec<false>(geo, geo.image_of_gauss(i), i, i, true, params + 2 * (size_t)n, params, 1.f,
+                       params + 5 * (size_t)n, View<float>{0, 0, 1, 1, false}, xys, extents,
+                       counts, recs);
 }
 
 // ---------------------------------------------------------------- regions
@@ -2531,17 +2571,19 @@ int raster_fwd(const BatchGeo &geo, TileWalk walk, const int32_t *ids, const int
                const void *op, void *ws, size_t ws_bytes, void *img, void *wsum, void *dx,
                void *dy, void *dxy, int32_t *fin, cudaStream_t s,
                L2Fwd<T> l2 = L2Fwd<T>{nullptr, nullptr}, L2Out<T> l2o = L2Out<T>{},
-               T *clear_grads = nullptr, AdamPro pro = AdamPro{}) {
+               bool have_recs = false, AdamPro pro = AdamPro{}) {
     const int n = geo.total_points();
     const bool ga = dx != nullptr;
     const bool fused = l2.target || l2.target_u8;
     // the sum forward reads the halved conic (see sigma_half)
-    // (clear_grads: the fit step's backward reuses the records; its [N][8]
-    // accumulators are cleared in the same pass)
+    // (have_recs: the fit step's fit_project_kernel has written the records and
+    // cleared the ticket)
     double *chunk_sum = l2.tile_partial + geo.total_tiles();
     uint32_t *ticket = fused ? loss_ticket(l2.tile_partial, geo.total_tiles()) : nullptr;
-    int rc = pack<T>(n, xys, con, col, op, ws, ws_bytes, s, !ga, clear_grads, 8, ga, ticket);
-    if (rc) return rc;
+    if (!have_recs) {
+        const int rc = pack<T>(n, xys, con, col, op, ws, ws_bytes, s, !ga, nullptr, 0, ga, ticket);
+        if (rc) return rc;
+    }
     if constexpr (sizeof(T) == 4) {
         if (ga)
             return raster_fwd_ga(geo, walk, ids, bins, d_total, ws, op != nullptr, (float *)img,
@@ -3321,15 +3363,15 @@ extern "C" int lig_raster_bwd_diff_batch(int dtype, int n_img, const int32_t *he
 }
 
 // ------------------------------------------------------------------ fit step
-// The fit engine's iteration behind the binning, with what its four separate
-// calls repeat taken out: the forward's records serve the backward (one pack),
-// the loss launch forms Adam's scalars and mirrors the skip count, and one
+// The fit engine's iteration, with what its seven separate calls repeat taken
+// out: the projection writes the forward's records, which serve the backward,
+// and clears what the later launches start from; the loss launch forms Adam's scalars and mirrors the skip count, and one
 // kernel takes the backward's packed sums through the projection backward and
 // Adam.  64 B of parameters and gradients, 128 B of moments and the 32 B sums
 // move once per Gaussian; before, v_xy, v_conic and the gradients were written
-// and read again between five launches.  Iteration: 512^2 / 50k 121 -> 106 us (15
-// launches instead of 21), 16 images 875 -> 832, 2048^2 / 1M 1497 -> 1460, 8192^2 /
-// 2M 3736 -> 3670.
+// and read again between five launches.  Iteration: 512^2 / 50k 121 -> 96 us (12
+// launches instead of 21), 16 images 875 -> 847, 2048^2 / 1M 1497 -> 1458, 8192^2 /
+// 2M 3736 -> 3662.
 namespace lig {
 __global__ void __launch_bounds__(256)
 fit_update_kernel(const BatchGeo geo, int n, const float4 *__restrict__ packed,
@@ -3372,11 +3414,47 @@ fit_update_kernel(const BatchGeo geo, int n, const float4 *__restrict__ packed,
 }
 }  // namespace lig
 
+extern "C" int lig_fit_bin_batch(int n_img, const int32_t *heights, const int32_t *widths,
+                                 const int32_t *counts, int B, const float *params, void *ws,
+                                 size_t ws_bytes, double *tile_partials, float *xys,
+                                 float *extents, int32_t *num_tiles_hit, int32_t *cum,
+                                 int32_t *d_total, void *cum_ws, size_t cum_ws_bytes, int capacity,
+                                 void *bin_ws, size_t bin_ws_bytes, int32_t *ids, int32_t *bins,
+                                 int32_t *status, void *stream) {
+    BatchGeo geo;
+    if (!batch_geo(n_img, heights, widths, counts, B, geo)) return LIG_ERR_INVALID;
+    const int n = geo.total_points();
+    if (capacity < 0 || !ws || !tile_partials || !d_total || !bins || !status ||
+        (capacity > 0 && (!ids || !bin_ws)) ||
+        (n > 0 && (!params || !xys || !extents || !num_tiles_hit || !cum || !cum_ws)) ||
+        (reinterpret_cast<uintptr_t>(ws) & 15) != 0 ||      // 16-byte records
+        (reinterpret_cast<uintptr_t>(cum_ws) & 7) != 0)
+        return LIG_ERR_INVALID;
+    const size_t goff = bwd_grad_offset<float>(n);
+    if (ws_bytes < goff + sizeof(float) * 8 * (size_t)n ||
+        (n > 0 && cum_ws_bytes < lig_cumsum_workspace_bytes(n)))
+        return LIG_ERR_WORKSPACE;
+    cudaStream_t s = (cudaStream_t)stream;
+    uint32_t *ticket = loss_ticket(tile_partials, geo.total_tiles());
+    if (n == 0) {
+        cudaMemsetAsync(ticket, 0, sizeof(*ticket), s);
+        cudaMemsetAsync(status, 0, sizeof(*status), s);
+    } else {
+        fit_project_kernel<<<(n + 255) / 256, 256, 0, s>>>(
+            geo, n, params, xys, extents, num_tiles_hit, (Rec<float> *)ws,
+            (float4 *)((char *)ws + goff), (uint32_t *)cum_ws,
+            (int)(lig_cumsum_workspace_bytes(n) / sizeof(uint32_t)), status, ticket);
+        note_launches(1);
+        LIG_LAUNCH_CHECK();
+    }
+    return scan_and_bin(geo, xys, extents, num_tiles_hit, cum, d_total, cum_ws, capacity, bin_ws,
+                        bin_ws_bytes, ids, bins, status, s);
+}
+
 extern "C" int lig_fit_forward_batch(int n_img, const int32_t *heights, const int32_t *widths,
                                      const int32_t *counts, int B, const int32_t *ids,
                                      const int32_t *bins, const int32_t *d_total,
-                                     const int32_t *cum, const float *xys, const float *con,
-                                     const float *col, const void *target, int target_u8,
+                                     const int32_t *cum, const void *target, int target_u8,
                                      int persistent, int32_t *work, void *ws, size_t ws_bytes,
                                      double *tile_partials, float *diff, float *loss,
                                      float *per_image, const int32_t *status, int32_t *steps,
@@ -3388,7 +3466,7 @@ extern "C" int lig_fit_forward_batch(int n_img, const int32_t *heights, const in
     const int n = geo.total_points();
     if (!bins || !d_total || !target || !ws || !tile_partials || !diff || !loss || !status ||
         !steps || !skipped || !skipped_host || !scratch || (persistent && !work) ||
-        (n > 0 && (!xys || !con || !col || !cum)))
+        (n > 0 && !cum))
         return LIG_ERR_INVALID;
     const size_t goff = bwd_grad_offset<float>(n);
     if (ws_bytes < goff + sizeof(float) * 8 * (size_t)n ||
@@ -3398,9 +3476,9 @@ extern "C" int lig_fit_forward_batch(int n_img, const int32_t *heights, const in
         target_u8 ? L2Fwd<float>{nullptr, tile_partials, (const uint8_t *)target}
                   : L2Fwd<float>{(const float *)target, tile_partials};
     TileWalk walk{n > 0 ? cum : nullptr, persistent ? work : nullptr};
-    return raster_fwd<float>(geo, walk, ids, bins, d_total, xys, con, col, nullptr, ws, goff, diff,
-                             nullptr, nullptr, nullptr, nullptr, nullptr, (cudaStream_t)stream, l2,
-                             L2Out<float>{loss, per_image}, (float *)((char *)ws + goff),
+    return raster_fwd<float>(geo, walk, ids, bins, d_total, nullptr, nullptr, nullptr, nullptr, ws,
+                             goff, diff, nullptr, nullptr, nullptr, nullptr, nullptr,
+                             (cudaStream_t)stream, l2, L2Out<float>{loss, per_image}, true,
                              AdamPro{status, steps, skipped, skipped_host, lr, beta1, beta2,
                                      (AdamScalars *)scratch});
 }

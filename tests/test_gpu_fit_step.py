@@ -1,4 +1,4 @@
-"""The fit engine's two fused calls against the separate entry points they
+"""The fit engine's three fused calls against the separate entry points they
 replace: gradients, loss, parameters, moments, step counts; the skipped step of
 an overflowed binning; fp32 and 8-bit targets; the persistent walk; an image
 without Gaussians; one and many loss chunks per image.
@@ -65,6 +65,11 @@ def test_fused_step_matches_separate_calls(shapes, counts, u8, persistent):
         a.step()
         _separate_step(b)
         torch.cuda.synchronize()
+        assert torch.equal(a.cnt, b.cnt) and torch.equal(a.cum, b.cum)
+        seen = a.cnt > 0
+        assert torch.equal(a.xys[seen], b.xys[seen]) and torch.equal(a.ext[seen], b.ext[seen])
+        assert torch.equal(a.bins, b.bins)
+        assert torch.equal(a.gids[:int(a.total)], b.gids[:int(b.total)])
         assert torch.equal(a.img, b.img)
         assert torch.allclose(a.per_image, b.per_image, rtol=1e-6)
         assert torch.allclose(a.loss, b.loss, rtol=1e-6)
