@@ -254,34 +254,29 @@ __device__ __forceinline__ int32_t slot_id(uint32_t v, const BatchGeo &geo) {
 // bbox of width 1 and row stride -1, so its key stays on the first tile.
 struct SlotWarp {
     int64_t g0;
+    int g;  // this lane's Gaussian
     int incl, excl, slot_base, bw, stride, total;
     uint32_t base, magic;
 };
 
-// g0: the warp's first Gaussian; n: end of its range.  False when the warp has
-// no slots (a view's Gaussians are mostly outside it: those cost one load).
+// Fills in the warp's slots from each lane's Gaussian (ascending over the
+// lanes, lane 0 valid), its count and its first slot.
 template <typename T>
-__device__ __forceinline__ bool slot_warp(int64_t g0, int n, const T *__restrict__ xys,
-                                          const T *__restrict__ extents,
-                                          const int32_t *__restrict__ cum, const BatchGeo &geo,
-                                          int32_t *__restrict__ status, SlotWarp &sw) {
+__device__ __forceinline__ void slot_lanes(int g, bool valid, int cnt, int start,
+                                           const T *__restrict__ xys,
+                                           const T *__restrict__ extents, const BatchGeo &geo,
+                                           int32_t *__restrict__ status, SlotWarp &sw) {
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
-    sw.g0 = g0;
-    if (g0 >= n) return false;
-    const int g = (int)(g0 + lane);
-    const int last = g < n ? cum[g] : 0;
-    int start = __shfl_up_sync(FULL, last, 1);
-    if (lane == 0) start = g0 > 0 ? cum[g0 - 1] : 0;
-    const int cnt = g < n ? last - start : 0;
-    if (!__any_sync(FULL, cnt != 0)) return false;
+    sw.g = g;
     sw.bw = 1;
     sw.stride = -1;
     sw.base = 0;
     sw.magic = 0;
-    if (g < n) {
+    const int g0 = __shfl_sync(FULL, g, 0);
+    if (valid) {
         // the image of the warp's first Gaussian, then this lane's
-        int im = geo.image_of_gauss((int)g0);
+        int im = geo.image_of_gauss(g0);
         while (im + 1 < geo.n_img && g >= geo.g_off[im + 1]) ++im;
         const int tbx = geo.tbx[im];
         sw.base = (uint32_t)geo.tile_off[im];
@@ -315,6 +310,26 @@ __device__ __forceinline__ bool slot_warp(int64_t g0, int n, const T *__restrict
     sw.total = __shfl_sync(FULL, incl, 31);
     sw.excl = incl - cnt;
     sw.slot_base = start - sw.excl;
+}
+
+// g0: the warp's first Gaussian; n: end of its range.  False when the warp has
+// no slots (a view's Gaussians are mostly outside it: those cost one load).
+template <typename T>
+__device__ __forceinline__ bool slot_warp(int64_t g0, int n, const T *__restrict__ xys,
+                                          const T *__restrict__ extents,
+                                          const int32_t *__restrict__ cum, const BatchGeo &geo,
+                                          int32_t *__restrict__ status, SlotWarp &sw) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    sw.g0 = g0;
+    if (g0 >= n) return false;
+    const int g = (int)(g0 + lane);
+    const int last = g < n ? cum[g] : 0;
+    int start = __shfl_up_sync(FULL, last, 1);
+    if (lane == 0) start = g0 > 0 ? cum[g0 - 1] : 0;
+    const int cnt = g < n ? last - start : 0;
+    if (!__any_sync(FULL, cnt != 0)) return false;
+    slot_lanes<T>(g, g < n, cnt, start, xys, extents, geo, status, sw);
     return true;
 }
 
@@ -324,7 +339,9 @@ __device__ __forceinline__ int64_t warp_first_gauss() {  // one warp per 32 Gaus
 
 // Flattened slot sl of the warp (all lanes call it together): false when sl
 // is past the warp's slots; otherwise the slot number, tile key and sort
-// value (2 g + phantom).
+// value (2 g + phantom).  LIST: the lanes' Gaussians are not consecutive; no
+// slot numbers.
+template <bool LIST = false>
 __device__ __forceinline__ bool slot_at(const SlotWarp &sw, int sl, int &slot, uint32_t &key,
                                         uint32_t &val) {
     const unsigned FULL = 0xffffffffu;
@@ -335,7 +352,7 @@ __device__ __forceinline__ bool slot_at(const SlotWarp &sw, int sl, int &slot, u
         if (v <= sl) lo += step;
     }
     const int o_excl = __shfl_sync(FULL, sw.excl, lo);
-    const int o_sb = __shfl_sync(FULL, sw.slot_base, lo);
+    const int o_sb = __shfl_sync(FULL, LIST ? sw.g : sw.slot_base, lo);
     const uint32_t o_base = __shfl_sync(FULL, sw.base, lo);
     const int o_bw = __shfl_sync(FULL, sw.bw, lo);
     const int o_stride = __shfl_sync(FULL, sw.stride, lo);
@@ -348,7 +365,7 @@ __device__ __forceinline__ bool slot_at(const SlotWarp &sw, int sl, int &slot, u
     else if (o_magic) q = __umulhi(j, o_magic);
     else q = j / (uint32_t)o_bw;
     key = o_base + j + q * (uint32_t)o_stride;
-    val = ((uint32_t)(sw.g0 + lo) << 1) | (o_stride < 0 ? kPhantom : 0u);
+    val = (LIST ? (uint32_t)o_sb << 1 : (uint32_t)(sw.g0 + lo) << 1) | (o_stride < 0 ? kPhantom : 0u);
     return true;
 }
 
@@ -860,7 +877,7 @@ tile_sort_long_kernel(BatchGeo geo, const uint32_t *__restrict__ tcount,
 //      one shared atomic per slot;
 // then the per-tile sort as above.  Count, prefix and scatter against global
 // atomics: 512^2 / 50k 11.5 us against 23, 16 images of 1.1M Gaussians 56
-// against 99, 2048^2 / 1M 88 against 100, eight views of 500k 121 against 236
+// against 99, 2048^2 / 1M 88 against 100, eight views of 500k 96 against 236
 // (139 with one run of consecutive Gaussians per CTA: the larger views waited);
 // what is left is the enumeration and the scattered 4-byte stores.  Slots past
 // the capacity are dropped by position (outputs are incomplete then, and flagged).
@@ -880,22 +897,61 @@ inline int hist_parts(int n, size_t tiles) {
     return std::min(std::max(n / LIG_BIN_HIST_RUN, 1), two ? kHistMaxParts : kHistMaxParts / 2);
 }
 
-// f(slot, tile key, sort value) for every slot of the CTA's Gaussians.
+// f(tile key, sort value) for every slot of the CTA's Gaussians.  Of 32
+// Gaussians with fewer than kQueueBelow visible a warp queues the visible ones,
+// and enumerates the queue 32 at a time: those outside their view cost a load and
+// a vote (eight views of 500k: count and scatter 39 + 46 us, 53 + 57 without the
+// queue).  Mostly visible ones are enumerated in place (all through the queue:
+// 2048^2 / 1M 88 us instead of 83).
+constexpr int kQueueBelow = 24;
 template <typename T, typename F>
 __device__ __forceinline__ void for_each_slot_of_cta(int n, const T *__restrict__ xys,
                                                      const T *__restrict__ ext,
                                                      const int32_t *__restrict__ cum,
                                                      const BatchGeo &geo,
                                                      int32_t *__restrict__ status, F f) {
+    __shared__ int s_queue[kHistThreads / 32][64];
+    const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
+    int *q = s_queue[threadIdx.x >> 5];
+    int nq = 0;  // queued Gaussians, below 32 between trips
     const int64_t chunk = (int64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
-    for (int64_t g = chunk * 32; g < n; g += (int64_t)gridDim.x * blockDim.x) {
+    for (int64_t g0 = chunk * 32;; g0 += (int64_t)gridDim.x * blockDim.x) {
+        int g = (int)(g0 + lane), cnt = 0;
+        bool valid = false;
+        if (g0 < n) {
+            valid = g0 + lane < n;
+            const int last = valid ? cum[g] : 0;
+            int start = __shfl_up_sync(FULL, last, 1);
+            if (lane == 0) start = g0 > 0 ? cum[g0 - 1] : 0;
+            cnt = valid ? last - start : 0;
+            const unsigned vis = __ballot_sync(FULL, cnt != 0);
+            if (__popc(vis) < kQueueBelow) {
+                if (cnt != 0) q[nq + __popc(vis & ((1u << lane) - 1u))] = g;
+                nq += __popc(vis);
+                __syncwarp();
+                if (nq < 32) continue;
+                valid = false;
+            }
+        } else if (nq == 0) {
+            break;
+        }
+        if (!__any_sync(FULL, valid)) {  // from the queue
+            valid = lane < nq;
+            g = valid ? q[lane] : 0;
+            const int rest = q[32 + lane];
+            __syncwarp();
+            q[lane] = rest;
+            nq = max(nq - 32, 0);
+            __syncwarp();
+            cnt = valid ? cum[g] - (g > 0 ? cum[g - 1] : 0) : 0;
+        }
         SlotWarp sw;
-        if (!slot_warp<T>(g, n, xys, ext, cum, geo, status, sw)) continue;
+        slot_lanes<T>(g, valid, cnt, 0, xys, ext, geo, status, sw);
         for (int s0 = 0; s0 < sw.total; s0 += 32) {
             int slot;
             uint32_t key, val;
-            if (slot_at(sw, s0 + lane, slot, key, val)) f(slot, key, val);
+            if (slot_at<true>(sw, s0 + lane, slot, key, val)) f(key, val);
         }
     }
 }
@@ -916,7 +972,7 @@ tile_hist_kernel(int n, int tiles, const T *__restrict__ xys, const T *__restric
     for (int t = threadIdx.x; t < tiles; t += blockDim.x) s_tile[t] = 0;
     __syncthreads();
     for_each_slot_of_cta<T>(n, xys, ext, cum, geo, status,
-                            [&](int, uint32_t key, uint32_t) { atomicAdd(&s_tile[key], 1u); });
+                            [&](uint32_t key, uint32_t) { atomicAdd(&s_tile[key], 1u); });
     __syncthreads();
     uint32_t *row = hist + (size_t)blockIdx.x * tiles;
     for (int t = threadIdx.x; t < tiles; t += blockDim.x) row[t] = s_tile[t];
@@ -970,7 +1026,7 @@ hist_scatter_kernel(int n, int tiles, const T *__restrict__ xys, const T *__rest
         s_tile[t] = tend[t] - tcount[t] + row[t];
     __syncthreads();
     for_each_slot_of_cta<T>(n, xys, ext, cum, geo, nullptr,
-                            [&](int, uint32_t key, uint32_t val) {
+                            [&](uint32_t key, uint32_t val) {
                                 const uint32_t pos = atomicAdd(&s_tile[key], 1u);
                                 if (pos < (uint32_t)capacity) out[pos] = val;
                             });
@@ -1000,7 +1056,7 @@ bin_small_kernel(int n, int tiles, const T *__restrict__ xys, const T *__restric
     s_cnt[tid] = 0;
     __syncthreads();
     for_each_slot_of_cta<T>(n, xys, ext, cum, geo, status,
-                            [&](int, uint32_t key, uint32_t) { atomicAdd(&s_cnt[key], 1u); });
+                            [&](uint32_t key, uint32_t) { atomicAdd(&s_cnt[key], 1u); });
     __syncthreads();
     const uint32_t c = s_cnt[tid];
     uint32_t total;
@@ -1012,7 +1068,7 @@ bin_small_kernel(int n, int tiles, const T *__restrict__ xys, const T *__restric
     }
     __syncthreads();
     for_each_slot_of_cta<T>(n, xys, ext, cum, geo, nullptr,
-                            [&](int, uint32_t key, uint32_t val) {
+                            [&](uint32_t key, uint32_t val) {
                                 const uint32_t pos = atomicAdd(&s_cur[key], 1u);
                                 if (pos < (uint32_t)capacity) vals[pos] = val;
                             });

@@ -3,24 +3,24 @@
 // Work decomposition (B200): one CTA per tile (or per work item of a
 // batch's flattened (image, tile) list); the tile is split into <= 32
 // regions of 32 lanes and warp w owns region w: 8x8 pixels with two pixels
-// per lane in the sum forward, 8x4 pixels in the gradient-aware forward and
-// the sum backward, the reference's warp in the gradient-aware backward,
+// per lane in the sum forward (8x16 with four for many tiles) and, as a pair,
+// in the gradient-aware forward; 8x4, 8x8 or 8x16 in the sum backward by tile
+// count and density; the reference's warp in the gradient-aware backward,
 // whose v_xy_abs is |sum over that warp| per Gaussian
 // (csrc/gradient_aware_rasterizer.cu:317-341).
 //
-// Gaussian data: a pack kernel writes one 16-byte-aligned 48-byte record per
+// Gaussian data: a pack kernel (or the projection of the fit step and of decode
+// batches) writes one 16-byte-aligned 48-byte record per
 // Gaussian (mean, conic, opacity, colour, cull half-widths, sigma
-// threshold).  The tile's sorted id list is consumed in batches of blockDim
-// Gaussians: each thread parks one record in shared memory (fetched into
-// registers while the previous batch was processed) together with that
-// Gaussian's region mask.
+// threshold).  Forwards: each warp streams the tile's sorted id list in chunks
+// of 32 records through shared memory, the next chunk in registers meanwhile.
+// Backwards: the CTA stages batches of blockDim records.
 //
-// Culling: a warp runs only the Gaussians whose mask has its region bit
+// Culling: a warp runs only the Gaussians that can reach its region
 // (forward: one ballot per 32 Gaussians, then the set bits in ascending, i.e.
-// list, order; backward: a compacted per-warp list).  The mask comes from a
+// list, order; backward: a compacted per-warp list).  The test is a
 // conservative box around the Gaussian's alpha >= 1/255 ellipse, built with
-// margin (see pack_kernel), refined in the backward by an exact
-// ellipse-over-rectangle test, so every skipped pixel would have failed the
+// margin (see finish_rec), refined by an exact ellipse-over-rectangle test, so every skipped pixel would have failed the
 // reference's own `alpha < 1/255` test (csrc/forward.cu:258): results are
 // unchanged.
 //
@@ -139,6 +139,7 @@ __device__ __forceinline__ bool tame_cotangent(T a, T b, T c, T d) {
     return fabs(a) < (T)kTameCot && fabs(b) < (T)kTameCot && fabs(c) < (T)kTameCot &&
            fabs(d) < (T)kTameCot;
 }
+
 __device__ __forceinline__ void publish_alpha_cut() {  // first warp of the grid
     if (blockIdx.x == 0 && threadIdx.x < 32) {
         const uint32_t cut = alpha_cut_search();
@@ -429,7 +430,7 @@ __device__ __forceinline__ T sigma_min_rect(T a, T b, T c, T dx0, T dx1, T dy0, 
 
 // Region mask of one Gaussian for the tile at pixel origin (tx0, ty0): the
 // regions whose pixel-centre rectangle meets the Gaussian's cull box and, on
-// it, reaches sigma <= thr (see pack_kernel: every pixel with sigma > thr
+// it, reaches sigma <= thr (see finish_rec: every pixel with sigma > thr
 // fails the reference's own alpha >= 1/255 test).  Records without culling
 // data (wx < 0) touch every region.
 // ELLIPSE = false stops at the box test.  HALF: the record carries the

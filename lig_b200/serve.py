@@ -7,7 +7,7 @@ This module serves both kinds of work at once:
 
 * **Render requests** decode a crop of a resident set at a scale: the view
   transform means' = (means - origin) * s, L' = s L is folded into the
-  projection (lig_project_fwd_view), then binning and the forward rasterizer
+  projection, then binning and the forward rasterizer
   produce the [h, w, 3] image in HBM.  The renders queued when the render
   worker is free are decoded together (continuous batching): one batched
   binning and one batched forward launch for all of them (render_views),

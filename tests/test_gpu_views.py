@@ -61,3 +61,14 @@ def test_views_tile_sizes(block, big):
     args = (h, w, (7.0, 9.0), (2.0, 3.0))
     got = render_views([(gs, *args), (gs, 20, 30, (1.0, 1.0), (1.0, 1.0))], block)[0]
     assert torch.equal(got, render_view(gs, *args, block)[0])
+
+
+@pytest.mark.parametrize("h,w", [(200, 30), (900, 900), (1990, 2010)])
+def test_views_of_a_partly_visible_set(h, w):
+    """From 2049 Gaussians on the counting kernels queue the visible ones: few,
+    a fifth and all of the set, beside a small view of another set."""
+    gs, other = _set(60000, 2048, 9), _set(2500, 100, 10)
+    args = (h, w, (20.0, 31.0), (1.0, 1.0))
+    got = render_views([(gs, *args), (other, 50, 60, (0.0, 0.0), (1.0, 1.0)), (gs, *args)])
+    want = render_view(gs, *args)[0]
+    assert torch.equal(got[0], want) and torch.equal(got[2], want)
