@@ -2491,8 +2491,13 @@ int pack(int n, const void *xys, const void *con, const void *col, const void *o
 #define LIG_RASTER_CARVEOUT -1  // shared-memory carveout percent; -1: driver default
 #endif
 
+// Opts a kernel into its dynamic shared memory, once per device and size.  A
+// launch is given 48 KB unasked, its static shared memory included: a kernel
+// that comes within kStaticSmem of that asks too.
+constexpr size_t kDefaultSmem = 48 * 1024, kStaticSmem = 4 * 1024;
 inline bool set_dyn_smem(const void *fn, size_t bytes) {
-    if (bytes <= 48 * 1024 && LIG_RASTER_CARVEOUT < 0) return true;
+    const bool ask = bytes > kDefaultSmem - kStaticSmem;
+    if (!ask && LIG_RASTER_CARVEOUT < 0) return true;
     static std::mutex mu;
     static std::vector<std::tuple<const void *, int, size_t>> done;
     int dev = 0;
@@ -2500,7 +2505,7 @@ inline bool set_dyn_smem(const void *fn, size_t bytes) {
     std::lock_guard<std::mutex> lock(mu);
     for (auto &e : done)
         if (std::get<0>(e) == fn && std::get<1>(e) == dev && std::get<2>(e) >= bytes) return true;
-    if (bytes > 48 * 1024 &&
+    if (ask &&
         cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) !=
             cudaSuccess)
         return false;
