@@ -1199,7 +1199,7 @@ int run_bin_scatter(const BatchGeo &geo, const void *xys, const void *ext, const
     // slot-order kernels)
     const bool hist_path = T_ <= kHistMaxTiles && !isect && ws_bytes >= p.total_hist;
     if (hist_path) {
-        if (!hist_smem_opt_in<T>()) return LIG_ERR_LAUNCH;
+        if (!hist_smem_opt_in<T>()) return launch_refused();
         uint32_t *hist = (uint32_t *)(base + p.off_hist);
         const int parts = hist_parts(n, (size_t)T_);
         const size_t sm = sizeof(uint32_t) * (size_t)T_;
@@ -1295,13 +1295,13 @@ int run_bin(const BatchGeo &geo, const void *xys, const void *ext, const int32_t
         static std::mutex mu;
         static size_t opted[128] = {};
         int dev = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 128) return LIG_ERR_LAUNCH;
+        if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 128) return launch_refused();
         std::lock_guard<std::mutex> lock(mu);
         if (opted[dev] < dsm) {
             if (cudaFuncSetAttribute(radix_downsweep_kernel,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)dsm) != cudaSuccess)
-                return LIG_ERR_LAUNCH;
+                return launch_refused();
             opted[dev] = dsm;
         }
     }

@@ -159,6 +159,16 @@ void note_launches(int n);
 
 }  // namespace lig
 
+namespace lig {
+// A launch that the runtime refused before it was made (shared memory beyond an
+// SM's, say): the runtime's error goes with the status, so that the caller's
+// next check of its own work does not meet it.
+inline int launch_refused() {
+    (void)cudaGetLastError();
+    return LIG_ERR_LAUNCH;
+}
+}  // namespace lig
+
 // Host-side launch check: every entry point returns a LIG_* status.
 #define LIG_LAUNCH_CHECK()                                            \
     do {                                                              \

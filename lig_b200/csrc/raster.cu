@@ -2560,7 +2560,7 @@ inline int raster_fwd_ga(const BatchGeo &geo, TileWalk walk, const int32_t *ids,
     int grid = geo.total_tiles();
     if (walk.work) {
         const int pg = persistent_grid((const void *)fn, nt, sm);
-        if (pg <= 0) return LIG_ERR_LAUNCH;
+        if (pg <= 0) return launch_refused();
         grid = grid < pg ? grid : pg;
         cudaMemsetAsync(walk.work, 0, sizeof(int), s);
     }
@@ -2638,11 +2638,11 @@ int raster_fwd(const BatchGeo &geo, TileWalk walk, const int32_t *ids, const int
     } else {
         fn = ppl4 ? pick(std::integral_constant<int, 4>{}) : pick(std::integral_constant<int, 2>{});
     }
-    if (!set_dyn_smem((const void *)fn, sm)) return LIG_ERR_LAUNCH;
+    if (!set_dyn_smem((const void *)fn, sm)) return launch_refused();
     int grid = geo.total_tiles();
     if (walk.work) {
         const int pg = persistent_grid((const void *)fn, nt, sm);
-        if (pg <= 0) return LIG_ERR_LAUNCH;
+        if (pg <= 0) return launch_refused();
         grid = grid < pg ? grid : pg;
         cudaMemsetAsync(walk.work, 0, sizeof(int), s);
     }
@@ -2679,7 +2679,7 @@ inline int raster_bwd_ga(const BatchGeo &geo, TileWalk walk, const int32_t *ids,
     int grid = geo.total_tiles();
     if (walk.work) {
         const int pg = persistent_grid((const void *)fn, nt, 0);
-        if (pg <= 0) return LIG_ERR_LAUNCH;
+        if (pg <= 0) return launch_refused();
         grid = grid < pg ? grid : pg;
         cudaMemsetAsync(walk.work, 0, sizeof(int), s);
     }
@@ -2794,11 +2794,11 @@ int raster_bwd(const BatchGeo &geo, TileWalk walk, const int32_t *ids, const int
                  : lean_abs ? raster_bwd_kernel<T, false, true, 64, M16, true, 16>
                             : raster_bwd_kernel<T, false, true, 64, M16, false, 16>;
     }
-    if (!set_dyn_smem((const void *)fn, sm)) return LIG_ERR_LAUNCH;
+    if (!set_dyn_smem((const void *)fn, sm)) return launch_refused();
     int grid = geo.total_tiles();
     if (walk.work) {
         const int pg = persistent_grid((const void *)fn, nt, sm);
-        if (pg <= 0) return LIG_ERR_LAUNCH;
+        if (pg <= 0) return launch_refused();
         grid = grid < pg ? grid : pg;
         cudaMemsetAsync(walk.work, 0, sizeof(int), s);
     }
@@ -3139,7 +3139,7 @@ extern "C" int lig_views_raster(int n_img, const int32_t *heights, const int32_t
                                  : raster_views_kernel<2, 512, 2, O>);
     };
     auto fn = with_opacities ? pick(std::true_type{}) : pick(std::false_type{});
-    if (!set_dyn_smem((const void *)fn, sm)) return LIG_ERR_LAUNCH;
+    if (!set_dyn_smem((const void *)fn, sm)) return launch_refused();
     fn<<<geo.total_tiles(), nt, sm, (cudaStream_t)stream>>>(
         geo, cum, ids, (const int2 *)bins, (const Rec<float> *)ws, out);
     note_launches(1);
