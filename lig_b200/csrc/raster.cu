@@ -87,6 +87,12 @@ __device__ __forceinline__ uint32_t alpha_cut_search() {
 // value) and read by the rasterizer launched after it on the same stream.
 __device__ uint32_t g_alpha_cut;
 
+// A backward's cut: its clamp is the caller's, and below 1/255 every pixel fails
+// (no sigma lies below a cut of 0).
+__device__ __forceinline__ uint32_t backward_cut(float clamp) {
+    return clamp < 1.f / 255.f ? 0u : g_alpha_cut;
+}
+
 // The fused fit step's optimiser scalars (out null: not wanted).
 // skipped_host: pinned host copy of *skipped.
 struct AdamPro {
@@ -1675,7 +1681,7 @@ __device__ __forceinline__ void bwd_tile(const TileCtx &tc, int tile,
     // masks: the warps test the box and ellipse themselves)
     constexpr bool kBulk = kPairs && LIG_RASTER_BWD_BULK;
     constexpr bool kCut = kPairs && !GEN && LIG_RASTER_BWD_CUT;
-    [[maybe_unused]] const uint32_t cut = kCut ? g_alpha_cut : 0u;
+    [[maybe_unused]] const uint32_t cut = kCut ? backward_cut(clamp) : 0u;
     static_assert(RR == 4 || kPairs, "taller regions are walked by the pair form only");
     static_assert(RR == 4 || RR == 8 || RR == 16, "region rows");
     constexpr int kRows = RR;  // pair entries per region: kRows * 4
@@ -2307,7 +2313,7 @@ raster_bwd_ga_kernel(const BatchGeo geo, const int32_t *__restrict__ cum, int *w
     }
     __syncthreads();
     const int n_tiles = geo.total_tiles();
-    const uint32_t cut = OP ? 0u : g_alpha_cut;
+    const uint32_t cut = OP ? 0u : backward_cut(clamp);
     const GaPix *my_pix = s_pix + w * 16;
     uint16_t *my_list = s_list[w];
     for (int tile = next_tile(work, s_slot, true); tile < n_tiles;
