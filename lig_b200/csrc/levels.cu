@@ -138,7 +138,7 @@ resid_normalise_kernel(int64_t n, const float *__restrict__ gt, const float *__r
 // together.  The rows' taps and weights come from a table the CTA fills once:
 // the float / integer conversions run at a quarter of the other operations'
 // rate and cost more than the memory traffic when every value makes its own.
-// Off: unsigned type of a byte offset into prev.
+// Off: unsigned type of the byte offsets from a CTA's first row, and into prev.
 // 4095x4093 from 2047x2046 (69 us of traffic): 92 us, against 115 with one
 // pixel a thread and a 64-bit division each, 131 with the conversions per value
 // and 146 with four flat values a thread.  Issue-bound (75% of the slots).
@@ -156,7 +156,7 @@ compose_kernel(int ph, int pw, const float *__restrict__ prev, int H, int W,
                float hi_h, int clamp_render, int clamp_out, float *__restrict__ out) {
     __shared__ RowTap<Off> s_row[kComposeRows];
     const int64_t pitch = 3 * (int64_t)W;
-    const uint32_t q = blockIdx.x * kLevelThreads + threadIdx.x;
+    const Off q = (Off)blockIdx.x * kLevelThreads + threadIdx.x;
     const int r0 = blockIdx.y * kComposeRows, nr = min(kComposeRows, H - r0);
     // the half-pixel source index and weights written as the bilinear
     // definition states them (src = s (d + 0.5) - 0.5, negative -> 0;
@@ -173,7 +173,7 @@ compose_kernel(int ph, int pw, const float *__restrict__ prev, int H, int W,
     }
     const float lo = mm ? mm[0] : lo_h, hi = mm ? mm[1] : hi_h;
     const float rng = __fsub_rn(hi, lo);
-    const uint32_t x = q / 3u, c = q - 3u * x;
+    const Off x = q / 3u, c = q - 3u * x;
     float lx0 = 0.f, lx1 = 0.f;
     Off oa = 0, ob = 0;
     if constexpr (RESIZE) {
@@ -273,11 +273,12 @@ extern "C" int lig_level_compose(int prev_h, int prev_w, const float *prev, int 
     const bool resize = prev && !(prev_h == H && prev_w == W);
     const dim3 grid((unsigned)((3 * (int64_t)W + kLevelThreads - 1) / kLevelThreads),
                     (H + kComposeRows - 1) / kComposeRows);
-    const bool small = 12 * (int64_t)prev_h * prev_w <= 0xffffffffll &&
-                       12 * (int64_t)W * kComposeRows <= 0xffffffffll;
-    auto k = !resize ? compose_kernel<false, uint32_t>
-             : small ? compose_kernel<true, uint32_t>
-                     : compose_kernel<true, uint64_t>;
+    // 32-bit byte offsets while a CTA's rows (and prev, which a resize gathers
+    // from anywhere) lie within 4 GiB
+    const bool small = 12 * (int64_t)W * kComposeRows <= 0xffffffffll &&
+                       (!resize || 12 * (int64_t)prev_h * prev_w <= 0xffffffffll);
+    auto k = resize ? (small ? compose_kernel<true, uint32_t> : compose_kernel<true, uint64_t>)
+                    : (small ? compose_kernel<false, uint32_t> : compose_kernel<false, uint64_t>);
     k<<<grid, kLevelThreads, 0, s>>>(prev_h, prev_w, prev, H, W, render, minmax, (float)store_min,
                                      (float)store_max, clamp_render, clamp_out, out);
     note_launches(1);
