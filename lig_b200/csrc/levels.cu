@@ -157,7 +157,10 @@ compose_kernel(int ph, int pw, const float *__restrict__ prev, int H, int W,
     __shared__ RowTap<Off> s_row[kComposeRows];
     const int64_t pitch = 3 * (int64_t)W;
     const Off q = (Off)blockIdx.x * kLevelThreads + threadIdx.x;
-    const int r0 = blockIdx.y * kComposeRows, nr = min(kComposeRows, H - r0);
+    // (the row blocks run over y and z of the grid: one dimension holds 65535)
+    const int64_t rb = (int64_t)blockIdx.z * gridDim.y + blockIdx.y;
+    if (rb * kComposeRows >= H) return;
+    const int r0 = (int)rb * kComposeRows, nr = min(kComposeRows, H - r0);
     // the half-pixel source index and weights written as the bilinear
     // definition states them (src = s (d + 0.5) - 0.5, negative -> 0;
     // lambda1 = src - floor, lambda0 = 1 - lambda1), so that the
@@ -271,8 +274,10 @@ extern "C" int lig_level_compose(int prev_h, int prev_w, const float *prev, int 
         return LIG_ERR_INVALID;
     cudaStream_t s = (cudaStream_t)stream;
     const bool resize = prev && !(prev_h == H && prev_w == W);
+    const int64_t row_blocks = ((int64_t)H + kComposeRows - 1) / kComposeRows;
+    const unsigned gz = (unsigned)((row_blocks + 65534) / 65535);
     const dim3 grid((unsigned)((3 * (int64_t)W + kLevelThreads - 1) / kLevelThreads),
-                    (H + kComposeRows - 1) / kComposeRows);
+                    (unsigned)((row_blocks + gz - 1) / gz), gz);
     // 32-bit byte offsets while a CTA's rows (and prev, which a resize gathers
     // from anywhere) lie within 4 GiB
     const bool small = 12 * (int64_t)W * kComposeRows <= 0xffffffffll &&
