@@ -142,37 +142,53 @@ resid_normalise_kernel(int64_t n, const float *__restrict__ gt, const float *__r
 // 4095x4093 from 2047x2046 (69 us of traffic): 92 us, against 115 with one
 // pixel a thread and a 64-bit division each, 131 with the conversions per value
 // and 146 with four flat values a thread.  Issue-bound (75% of the slots).
+// Images of up to kNarrowValues values a row: a CTA is CW = 32 columns (16 or 4,
+// if those hold a row) by several groups of sixteen rows, so that few threads
+// lie past the row's end (100000x5: 9.0 us with 32, 15 with 256).
 constexpr int kComposeRows = 16, kComposeBatch = 4;  // 32 rows 95 us, batches of 2 / 8 98 / 104
+constexpr int kNarrowValues = 128;
+// Small images: groups of four rows where sixteen would leave fewer than two CTAs
+// per SM (512^2 5.3 us instead of 6.2; 767x1023, four CTAs, 7.1 with sixteen and 8.3).
+constexpr int kComposeFewRows = 4, kComposeFewCtas = 2;
 
 template <typename Off> struct RowTap {
     Off a, b;        // byte offsets of the upper and lower row of prev
     float ly0, ly1;  // their weights
 };
 
-template <bool RESIZE, typename Off>
+template <bool RESIZE, typename Off, int CW = kLevelThreads>
 __global__ void __launch_bounds__(kLevelThreads)
-compose_kernel(int ph, int pw, const float *__restrict__ prev, int H, int W,
+compose_kernel(int rows, int ph, int pw, const float *__restrict__ prev, int H, int W,
                const float *__restrict__ render, const float *__restrict__ mm, float lo_h,
                float hi_h, int clamp_render, int clamp_out, float *__restrict__ out) {
-    __shared__ RowTap<Off> s_row[kComposeRows];
+    constexpr int kGroups = kLevelThreads / CW;
+    __shared__ RowTap<Off> s_rows[kGroups][kComposeRows];
+    const int tx = threadIdx.x % CW, ty = threadIdx.x / CW;
+    RowTap<Off> *s_row = s_rows[ty];
     const int64_t pitch = 3 * (int64_t)W;
-    const Off q = (Off)blockIdx.x * kLevelThreads + threadIdx.x;
+    const Off q = (Off)blockIdx.x * CW + tx;
     // (the row blocks run over y and z of the grid: one dimension holds 65535)
     const int64_t rb = (int64_t)blockIdx.z * gridDim.y + blockIdx.y;
-    if (rb * kComposeRows >= H) return;
-    const int r0 = (int)rb * kComposeRows, nr = min(kComposeRows, H - r0);
+    if (rb * (rows * kGroups) >= H) return;
+    const int64_t first = rb * (rows * kGroups) + ty * rows;
+    const int r0 = (int)(first < H ? first : H), nr = min(rows, H - r0);
     // the half-pixel source index and weights written as the bilinear
     // definition states them (src = s (d + 0.5) - 0.5, negative -> 0;
     // lambda1 = src - floor, lambda0 = 1 - lambda1), so that the
     // compiler contracts them as it does torch's upsample kernel
-    if (RESIZE && threadIdx.x < nr) {
+    auto tap = [&](int k) {
         const float sh = __fdiv_rn((float)ph, (float)H);
-        float ry = sh * ((float)(r0 + threadIdx.x) + 0.5f) - 0.5f;
+        float ry = sh * ((float)(r0 + k) + 0.5f) - 0.5f;
         ry = ry < 0.f ? 0.f : ry;
         const int y0 = (int)ry, y1 = y0 + (y0 < ph - 1 ? 1 : 0);
         const float ly1 = ry - (float)y0;
         const Off p = (Off)pw * 12u;
-        s_row[threadIdx.x] = RowTap<Off>{(Off)y0 * p, (Off)y1 * p, 1.f - ly1, ly1};
+        s_row[k] = RowTap<Off>{(Off)y0 * p, (Off)y1 * p, 1.f - ly1, ly1};
+    };
+    if constexpr (RESIZE) {
+        if (tx < nr) tap(tx);
+        if constexpr (CW < kComposeRows)
+            for (int k = tx + CW; k < nr; k += CW) tap(k);
     }
     const float lo = mm ? mm[0] : lo_h, hi = mm ? mm[1] : hi_h;
     const float rng = __fsub_rn(hi, lo);
@@ -199,7 +215,7 @@ compose_kernel(int ph, int pw, const float *__restrict__ prev, int H, int W,
     if (!RESIZE && prev) prv = prev + r0 * pitch;
     float *dst = out + r0 * pitch;
     const Off row = (Off)(pitch * 4);
-    auto rows = [&](int k0, auto full_tag) {  // FULL: the whole batch lies inside
+    auto walk = [&](int k0, auto full_tag) {  // FULL: the whole batch lies inside
         constexpr bool FULL = decltype(full_tag)::value;
         float v[kComposeBatch], t[kComposeBatch][4];
 #pragma unroll
@@ -235,8 +251,8 @@ compose_kernel(int ph, int pw, const float *__restrict__ prev, int H, int W,
         }
     };
     int k0 = 0;
-    for (; k0 + kComposeBatch <= nr; k0 += kComposeBatch) rows(k0, std::true_type{});
-    if (k0 < nr) rows(k0, std::false_type{});
+    for (; k0 + kComposeBatch <= nr; k0 += kComposeBatch) walk(k0, std::true_type{});
+    if (k0 < nr) walk(k0, std::false_type{});
 }
 
 inline int level_blocks(int64_t n) {
@@ -274,18 +290,34 @@ extern "C" int lig_level_compose(int prev_h, int prev_w, const float *prev, int 
         return LIG_ERR_INVALID;
     cudaStream_t s = (cudaStream_t)stream;
     const bool resize = prev && !(prev_h == H && prev_w == W);
-    const int64_t row_blocks = ((int64_t)H + kComposeRows - 1) / kComposeRows;
+    const bool narrow = 3 * (int64_t)W <= kNarrowValues;
+    const int cw = !narrow ? kLevelThreads : W <= 1 ? 4 : W <= 5 ? 16 : 32;
+    const int64_t cols = (3 * (int64_t)W + cw - 1) / cw;
+    const int groups = kLevelThreads / cw;
+    const int rows = cols * ((H + (int64_t)groups * kComposeRows - 1) / (groups * kComposeRows)) <
+                             148 * kComposeFewCtas ? kComposeFewRows : kComposeRows;
+    const int64_t row_blocks = ((int64_t)H + rows * groups - 1) / (rows * groups);
     const unsigned gz = (unsigned)((row_blocks + 65534) / 65535);
-    const dim3 grid((unsigned)((3 * (int64_t)W + kLevelThreads - 1) / kLevelThreads),
-                    (unsigned)((row_blocks + gz - 1) / gz), gz);
+    const dim3 grid((unsigned)cols, (unsigned)((row_blocks + gz - 1) / gz), gz);
     // 32-bit byte offsets while a CTA's rows (and prev, which a resize gathers
     // from anywhere) lie within 4 GiB
     const bool small = 12 * (int64_t)W * kComposeRows <= 0xffffffffll &&
                        (!resize || 12 * (int64_t)prev_h * prev_w <= 0xffffffffll);
-    auto k = resize ? (small ? compose_kernel<true, uint32_t> : compose_kernel<true, uint64_t>)
-                    : (small ? compose_kernel<false, uint32_t> : compose_kernel<false, uint64_t>);
-    k<<<grid, kLevelThreads, 0, s>>>(prev_h, prev_w, prev, H, W, render, minmax, (float)store_min,
-                                     (float)store_max, clamp_render, clamp_out, out);
+    auto pick = [&](auto off, auto w) {
+        using Off = decltype(off);
+        constexpr int CW = decltype(w)::value;
+        return resize ? compose_kernel<true, Off, CW> : compose_kernel<false, Off, CW>;
+    };
+    auto width = [&](auto off) {
+        return cw == 4    ? pick(off, std::integral_constant<int, 4>{})
+               : cw == 16 ? pick(off, std::integral_constant<int, 16>{})
+               : cw == 32 ? pick(off, std::integral_constant<int, 32>{})
+                          : pick(off, std::integral_constant<int, kLevelThreads>{});
+    };
+    auto k = small ? width(uint32_t{}) : width(uint64_t{});
+    k<<<grid, kLevelThreads, 0, s>>>(rows, prev_h, prev_w, prev, H, W, render, minmax,
+                                     (float)store_min, (float)store_max, clamp_render, clamp_out,
+                                     out);
     note_launches(1);
     LIG_LAUNCH_CHECK();
     return LIG_OK;
