@@ -36,6 +36,7 @@ import json
 import collections
 import math
 import os
+import weakref
 from dataclasses import dataclass
 from typing import Dict, List, Optional, Sequence
 
@@ -129,6 +130,27 @@ class BatchStats:
     capacity: int = 0
 
 
+_HELD: collections.deque = collections.deque()  # words that could not be released yet
+
+
+def _release_host_word(word, source, streams):
+    """A dropped fit may leave steps in flight that still write its pinned word.
+    A copy behind them on each stream they ran on tells the pinned-memory
+    allocator, which hands the block out again once those copies are done.  (A
+    stream under capture would take the copy into its graph: the word is then
+    held until the next fit goes.)"""
+    todo = [(word, source, s) for s in streams]
+    while _HELD:
+        todo.append(_HELD.popleft())
+    with torch.inference_mode():
+        for item in todo:
+            with torch.cuda.stream(item[2]):
+                if torch.cuda.is_current_stream_capturing():
+                    _HELD.append(item)
+                else:
+                    item[0].copy_(item[1], non_blocking=True)
+
+
 class BatchedFit:
     """Fits one Gaussian set per target image, all images per launch.
 
@@ -214,6 +236,11 @@ class BatchedFit:
         self.adam_scratch = torch.empty(_lib.lib.lig_adam_batch_scratch_bytes(L.n),
                                         dtype=torch.uint8, **kw)
         self.host_skipped = torch.zeros(1, dtype=i32, pin_memory=True)
+        # the steps write this word from the device, which the pinned-memory
+        # allocator does not see: see _release_host_word
+        self._streams: set = set()
+        weakref.finalize(self, _release_host_word, self.host_skipped, self.skipped,
+                         self._streams).atexit = False
         self.capacity = 0
         self.gids = None
         self.bin_ws = None
@@ -302,6 +329,8 @@ class BatchedFit:
         target: the concatenated [pixels, 3] target (default self.target)."""
         L = self.L
         st = self._stream()
+        if not torch.cuda.is_current_stream_capturing():
+            self._streams.add(torch.cuda.current_stream(self.dev))
         tgt = self.target if target is None else target
         call("lig_fit_bin_batch", *L.args(), L.block, _p(self.flat), _p(self.r_ws),
              self.r_ws.numel(), _p(self.partials), _p(self.xys), _p(self.ext), _p(self.cnt),
@@ -379,6 +408,7 @@ class BatchedFit:
             g = self._graphs[key] = self._capture(t)
             self.graph = g
         if g is not None:
+            self._streams.add(torch.cuda.current_stream(self.dev))
             g.replay()
         else:
             self._enqueue_step(t)
