@@ -240,10 +240,25 @@ bin_raster_fwd(const Tensor &xys0, const Tensor &ext0, const Tensor &counts, con
     const auto stream = c10::cuda::getCurrentCUDAStream(xys.get_device());
     C10_CUDA_CHECK(cudaMemcpyAsync(slot.data_ptr(), total.data_ptr(), sizeof(int32_t),
                                    cudaMemcpyDeviceToHost, stream));
-    at::cuda::CUDAEvent arrived;
-    arrived.record(stream);
+    // (also when a later call throws: the slot is the thread's, and free again
+    // once this function is left)
+    struct Arrival {
+        at::cuda::CUDAEvent event;
+        bool waited = false;
+        void wait() {
+            waited = true;
+            event.synchronize();
+        }
+        ~Arrival() {
+            try {
+                if (!waited) wait();
+            } catch (...) {  // the CUDA error is the caller's next one
+            }
+        }
+    } arrived;
+    arrived.event.record(stream);
     auto wait = [&]() -> int64_t {
-        arrived.synchronize();
+        arrived.wait();
         return *slot.data_ptr<int32_t>();
     };
     const bool guess = capacity >= 0;

@@ -267,11 +267,14 @@ def bin_gaussians(xys, extents, num_tiles_hit, img_h, img_w, block, want_keys=Fa
         cap = m
     else:
         cap = _guess(hint)
-    res = _run_bin(xys, extents, cum, total, img_h, img_w, block, cap, want_keys)
-    b = Binning(-1, total, cap, cum, *res)
-    extra = after_enqueue(b) if after_enqueue is not None else None
+    try:
+        res = _run_bin(xys, extents, cum, total, img_h, img_w, block, cap, want_keys)
+        b = Binning(-1, total, cap, cum, *res)
+        extra = after_enqueue(b) if after_enqueue is not None else None
+    finally:  # the slot is the thread's: the copy arrives before it is left
+        if hint is not None:
+            ev.synchronize()
     if hint is not None:
-        ev.synchronize()
         m = int(host.item())
         if m > cap:  # speculation failed: redo with the exact count
             res = _run_bin(xys, extents, cum, total, img_h, img_w, block, m, want_keys)
