@@ -397,10 +397,11 @@ class BatchedFit:
         host synchronisation unless a capacity overflow is being recovered.
         target (optional): fit against this [pixels, 3] buffer instead of the
         constructor's targets, read in place; one captured graph is kept per
-        target buffer (a caller alternating two upload buffers replays two
+        target buffer and type (a caller alternating two upload buffers replays two
         graphs, no copies)."""
         t = self._target_arg(target)
-        key = 0 if t is None else t.data_ptr()
+        # (a graph reads its target's address as its target's type)
+        key = 0 if t is None else (t.data_ptr(), t.dtype)
         g = self._graphs.get(key)
         if g is None and self.use_graph and self.stats.iters >= 2:
             if len(self._graphs) >= 4:
