@@ -87,6 +87,7 @@ class KernelTimer:
     def __enter__(self):
         global _TIMER
         self.events = []
+        self._starts = threading.local()  # a thread's call under way
         _TIMER = self.events
         _host.set_observer(self._observe)
         return self
@@ -101,10 +102,11 @@ class KernelTimer:
         """Calls made by the native operators: before (0) and after (1)."""
         ev = torch.cuda.Event(enable_timing=True)
         ev.record()
-        if end:
-            self.events.append((name, self._start, ev))
-        else:
-            self._start = ev
+        if not end:
+            self._starts.event = ev
+        elif getattr(self._starts, "event", None) is not None:  # begun inside the timer
+            self.events.append((name, self._starts.event, ev))
+            self._starts.event = None
 
     def summary(self):
         torch.cuda.synchronize()
