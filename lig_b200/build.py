@@ -26,6 +26,7 @@ CSRC = os.path.join(PKG, "csrc")
 HOST_SRC = os.path.join(CSRC, "host.cpp")
 HOST_LIB = os.path.join(PKG, "_host.so")
 BUILD = os.path.join(PKG, "_build")
+HOST_STAMP = os.path.join(BUILD, "host.stamp")  # what _host.so was built against
 LIB = os.path.join(PKG, "liblig_b200.so")
 INCLUDE = os.path.join(os.path.dirname(PKG), "include")
 
@@ -64,12 +65,28 @@ def _compile(src: str, extra) -> str:
     return obj
 
 
+def _run_host(cmd) -> None:
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"g++ failed for {HOST_SRC}:\n{r.stdout}\n{r.stderr}")
+
+
 def _build_host() -> None:
     """Compile the native half of ops.py (a Python module on torch's headers,
-    linked against the CUDA library beside it)."""
+    linked against the CUDA library beside it), unless it is newer than its
+    source and was built against this Python and this torch."""
     import sysconfig
 
     import torch
+
+    against = f"python {sys.version}\ntorch {torch.__version__}\n"
+    try:
+        with open(HOST_STAMP) as f:
+            same = f.read() == against
+    except OSError:
+        same = False
+    if same and not _stale(HOST_LIB, [HOST_SRC, os.path.join(INCLUDE, "lig_b200.h")]):
+        return
     from torch.utils import cpp_extension as tx
 
     cuda = os.path.dirname(os.path.dirname(nvcc()))
@@ -82,9 +99,9 @@ def _build_host() -> None:
            "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python",
            "-L", os.path.join(cuda, "lib64"), "-lcudart", "-Wl,-rpath,$ORIGIN",
            f"-Wl,-rpath,{lib}"]
-    r = subprocess.run(cmd, capture_output=True, text=True)
-    if r.returncode != 0:
-        raise RuntimeError(f"g++ failed for {HOST_SRC}:\n{r.stdout}\n{r.stderr}")
+    _run_host(cmd)
+    with open(HOST_STAMP, "w") as f:
+        f.write(against)
 
 
 def build(verbose: bool = False, extra=()) -> str:
@@ -98,8 +115,7 @@ def build(verbose: bool = False, extra=()) -> str:
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
-    if _stale(HOST_LIB, [HOST_SRC, os.path.join(INCLUDE, "lig_b200.h")]):
-        _build_host()
+    _build_host()
     if verbose:
         print(f"built {LIB}, {HOST_LIB}")
     return LIB
