@@ -34,6 +34,7 @@ from __future__ import annotations
 import ctypes
 import json
 import collections
+import functools
 import math
 import os
 import weakref
@@ -227,9 +228,6 @@ class BatchedFit:
                                     dtype=torch.float64, **kw)
         self.r_ws = torch.empty(_lib.lib.lig_raster_workspace_bytes(_lib.LIG_F32, N),
                                 dtype=torch.uint8, **kw)
-        self.v_xy = torch.empty(N, 2, dtype=f32, **kw)
-        self.v_abs = torch.empty(N, 2, dtype=f32, **kw)
-        self.v_con = torch.empty(N, 3, dtype=f32, **kw)
         self.one = torch.ones((), dtype=f32, **kw)
         self.work = torch.zeros(1, dtype=i32, **kw)
         self.skipped = torch.zeros(1, dtype=i32, **kw)
@@ -250,6 +248,20 @@ class BatchedFit:
         self._size_capacity(self._count_intersections())
 
     # ------------------------------------------------------------ helpers
+    # gradient rows of the separate backward calls; the step keeps the packed
+    # sums, so these 28 bytes a Gaussian are allocated when they are asked for
+    @functools.cached_property
+    def v_xy(self):
+        return torch.empty(self.L.points, 2, dtype=torch.float32, device=self.dev)
+
+    @functools.cached_property
+    def v_abs(self):
+        return torch.empty(self.L.points, 2, dtype=torch.float32, device=self.dev)
+
+    @functools.cached_property
+    def v_con(self):
+        return torch.empty(self.L.points, 3, dtype=torch.float32, device=self.dev)
+
     def _segments(self, flat, i):
         """Image i's (means, cholesky, rgb) views in a flat [8N] buffer."""
         return tuple(self.L.points_of(v, i) for v in self._views(flat))
