@@ -57,6 +57,7 @@ __device__ __forceinline__ void hermite(T t, T (&w)[4]) {
 struct UpMap {
     int mode, dst_n, src_n, roi_n;
     double lo;
+    int flip = 0;  // backward: walk the output indices from the last one down
 };
 
 // Source coordinate of output index d (float arithmetic for T=float).
@@ -83,14 +84,6 @@ __device__ __forceinline__ void coord(const UpMap &m, int d, int &i0, int &i1, T
     i1 = max(0, min(f + 1, m.src_n - 1));
     i0 = max(0, min(f, m.src_n - 1));
     hermite<T>(t, w);
-}
-
-template <typename T>
-__device__ __forceinline__ void coord_idx(const UpMap &m, int d, int &i0, int &i1) {
-    T s = src_coord<T>(m, d);
-    int f = (int)Math<T>::floor_(s);
-    i1 = max(0, min(f + 1, m.src_n - 1));
-    i0 = max(0, min(f, m.src_n - 1));
 }
 
 // ---------------------------------------------------------------- forward
@@ -185,14 +178,29 @@ upscale_fwd_kernel(UpMap mx, UpMap my, int src_w, int rows, const T *__restrict_
 constexpr int kBwdRowChunk = 32;  // output rows whose weights are staged at a time
 constexpr int kBwdMaxRows = 32;   // texel rows a CTA walks (32 to 128 measured alike)
 
+// A reversed ROI (roi_n < 0) maps output indices down the source; the backward
+// (its FLIP instantiation) then numbers them from the last one, so that its maps
+// always ascend.
+template <bool FLIP> __device__ __forceinline__ int walk_index(const UpMap &m, int d) {
+    return FLIP && m.flip ? m.dst_n - 1 - d : d;
+}
+
+template <typename T, bool FLIP>
+__device__ __forceinline__ void coord_idx(const UpMap &m, int d, int &i0, int &i1) {
+    T s = src_coord<T>(m, walk_index<FLIP>(m, d));
+    int f = (int)Math<T>::floor_(s);
+    i1 = max(0, min(f + 1, m.src_n - 1));
+    i0 = max(0, min(f, m.src_n - 1));
+}
+
 // First output index in [0, dst_n] whose left (RIGHT: right) corner is >= s.
-// The map is monotone: from the inverse map's estimate a few steps find the
+// The map ascends: from the inverse map's estimate a few steps find the
 // index; a degenerate map, or an estimate further off, takes the binary search.
-template <typename T, bool RIGHT>
+template <typename T, bool FLIP, bool RIGHT>
 __device__ __forceinline__ int first_ge(const UpMap &m, int s) {
     auto ge = [&](int d) {
         int a, b;
-        coord_idx<T>(m, d, a, b);
+        coord_idx<T, FLIP>(m, d, a, b);
         return (RIGHT ? b : a) >= s;
     };
     const int n = m.dst_n;
@@ -220,9 +228,9 @@ __device__ __forceinline__ int first_ge(const UpMap &m, int s) {
 
 // Weights of output index d, with a clamped cell (both corners the same
 // texel) folded into its first corner.
-template <typename T>
+template <typename T, bool FLIP>
 __device__ __forceinline__ void folded(const UpMap &m, int d, int &i0, int &i1, T (&w)[4]) {
-    coord<T>(m, d, i0, i1, w);
+    coord<T>(m, walk_index<FLIP>(m, d), i0, i1, w);
     if (i0 == i1) {
         w[0] += w[1];
         w[2] += w[3];
@@ -240,8 +248,8 @@ __device__ __forceinline__ void folded(const UpMap &m, int d, int &i0, int &i1, 
 // took 140 us at 2047x1535 -> 3070x2302, against 89).
 template <typename T>
 struct BwdWalk {
-    const T *g;          // this thread's first output column, output row 0
-    int64_t g_pitch;
+    const T *g;          // this thread's first output column, first row of the walk
+    int64_t g_pitch;     // to the walk's next row
     T *gf, *gfx, *gfy, *gfxy;
     int64_t o_pitch;     // values of a texel row
     bool active;
@@ -277,7 +285,8 @@ struct BwdWalk {
     }
 };
 
-template <typename T, int C>
+// FLIP: a reversed ROI, in x or y (mx.flip, my.flip)
+template <typename T, int C, bool FLIP>
 __global__ void __launch_bounds__(kUpThreads)
 upscale_bwd_kernel(UpMap mx, UpMap my, int src_w, int src_h, int rows, const T *__restrict__ g,
                    T *__restrict__ gf, T *__restrict__ gfx, T *__restrict__ gfy,
@@ -288,22 +297,26 @@ upscale_bwd_kernel(UpMap mx, UpMap my, int src_w, int src_h, int rows, const T *
     const int tid = threadIdx.x, dst_w = mx.dst_n;
     const int64_t q = (int64_t)blockIdx.x * kUpThreads + tid;
     const int sy0 = blockIdx.y * rows, sy1 = min(sy0 + rows, src_h) - 1;
-    if (tid == 0) s_rng[0] = first_ge<T, true>(my, sy0);
-    else if (tid == 32) s_rng[1] = first_ge<T, false>(my, sy1 + 1) - 1;
+    if (tid == 0) s_rng[0] = first_ge<T, FLIP, true>(my, sy0);
+    else if (tid == 32) s_rng[1] = first_ge<T, FLIP, false>(my, sy1 + 1) - 1;
     // this thread's texel column x: output columns [ia, im) have it as their
     // right corner, [im, ib) as their left one
     const int x = (int)min(q / C, (int64_t)src_w - 1), ch = (int)(q % C);
-    const int ia = first_ge<T, true>(mx, x), im = first_ge<T, false>(mx, x),
-              ib = first_ge<T, false>(mx, x + 1);
+    const int ia = first_ge<T, FLIP, true>(mx, x), im = first_ge<T, FLIP, false>(mx, x),
+              ib = first_ge<T, FLIP, false>(mx, x + 1);
     const int n = ib - ia;
     __syncthreads();
     const int j_lo = s_rng[0], j_hi = s_rng[1];
-    BwdWalk<T> B{g + (int64_t)ia * C + ch, (int64_t)dst_w * C, gf, gfx, gfy, gfxy,
-                 (int64_t)src_w * C, q < (int64_t)src_w * C, sy0, sy1, sy0 - 1, {}, {}};
+    const int CS = FLIP && mx.flip ? -C : C;  // to the walk's next column
+    const int64_t pitch = (int64_t)dst_w * C;
+    const T *g0 = g + (int64_t)walk_index<FLIP>(mx, ia) * C + ch +
+                  (FLIP && my.flip ? (my.dst_n - 1) * pitch : 0);
+    BwdWalk<T> B{g0, FLIP && my.flip ? -pitch : pitch, gf, gfx, gfy, gfxy, (int64_t)src_w * C,
+                 q < (int64_t)src_w * C, sy0, sy1, sy0 - 1, {}, {}};
     auto weights = [&](int i, T &wv, T &wd) {  // of output column ia + i
         int x0, x1;
         T w[4];
-        folded<T>(mx, ia + i, x0, x1, w);
+        folded<T, FLIP>(mx, ia + i, x0, x1, w);
         wv = ia + i < im ? w[1] : w[0];
         wd = ia + i < im ? w[3] : w[2];
     };
@@ -322,7 +335,7 @@ upscale_bwd_kernel(UpMap mx, UpMap my, int src_w, int src_h, int rows, const T *
         for (int jb = j_lo; jb <= j_hi; jb += kBwdRowChunk) {
             const int nj = min(kBwdRowChunk, j_hi - jb + 1);
             __syncthreads();
-            if (tid < nj) folded<T>(my, jb + tid, s_y[tid].x, s_y[tid].y, s_cy[tid].w);
+            if (tid < nj) folded<T, FLIP>(my, jb + tid, s_y[tid].x, s_y[tid].y, s_cy[tid].w);
             __syncthreads();
             const T *gp = B.g + jb * B.g_pitch;
             if constexpr (NT > 0) {
@@ -331,8 +344,8 @@ upscale_bwd_kernel(UpMap mx, UpMap my, int src_w, int src_h, int rows, const T *
                     T v[2][NT];
 #pragma unroll
                     for (int k = 0; k < NT; ++k) {
-                        v[0][k] = FULL || k < n ? gp[k * C] : (T)0;
-                        v[1][k] = (FULL || k < n) && two ? gp[B.g_pitch + k * C] : (T)0;
+                        v[0][k] = FULL || k < n ? gp[k * CS] : (T)0;
+                        v[1][k] = (FULL || k < n) && two ? gp[B.g_pitch + k * CS] : (T)0;
                     }
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
@@ -352,7 +365,7 @@ upscale_bwd_kernel(UpMap mx, UpMap my, int src_w, int src_h, int rows, const T *
                     for (int i = 0; i < n; ++i) {
                         T a, b;
                         weights(i, a, b);
-                        const T gv = gp[(int64_t)i * C];
+                        const T gv = gp[(int64_t)i * CS];
                         uv += gv * a;
                         ud += gv * b;
                     }
@@ -410,12 +423,14 @@ int upscale_bwd(int mode, int src_h, int src_w, int dst_h, int dst_w, double x1,
                 cudaStream_t s) {
     UpMap mx{mode, dst_w, src_w, (int)((T)x2 - (T)x1), (double)(T)x1};
     UpMap my{mode, dst_h, src_h, (int)((T)y2 - (T)y1), (double)(T)y1};
+    mx.flip = mode == 0 && mx.roi_n < 0;
+    my.flip = mode == 0 && my.roi_n < 0;
     const int64_t row = (int64_t)src_w * C;
     const int rows = up_rows(row, src_h, kBwdMaxRows);
     const dim3 grid((unsigned)((row + kUpThreads - 1) / kUpThreads), (src_h + rows - 1) / rows);
-    upscale_bwd_kernel<T, C><<<grid, kUpThreads, 0, s>>>(mx, my, src_w, src_h, rows,
-                                                         (const T *)g, (T *)gf, (T *)gfx,
-                                                         (T *)gfy, (T *)gfxy);
+    auto k = mx.flip || my.flip ? upscale_bwd_kernel<T, C, true> : upscale_bwd_kernel<T, C, false>;
+    k<<<grid, kUpThreads, 0, s>>>(mx, my, src_w, src_h, rows, (const T *)g, (T *)gf, (T *)gfx,
+                                  (T *)gfy, (T *)gfxy);
     note_launches(1);
     LIG_LAUNCH_CHECK();
     return LIG_OK;
