@@ -29,6 +29,7 @@
 // (csrc/gradient_aware_upscaler.cu:313-370).  2047x1535 -> 3070x2302: 328 us
 // (8x16 texels per CTA, patch staged in shared memory) -> 89; 512^2 -> 1024^2:
 // 39 -> 12.  Bound by load latency (half the warps resident at 64 registers).
+// Upscaling by more than four: upscale_bwd_wide_kernel.
 #include <type_traits>
 
 #include "common.cuh"
@@ -193,18 +194,18 @@ __device__ __forceinline__ void coord_idx(const UpMap &m, int d, int &i0, int &i
     i0 = max(0, min(f, m.src_n - 1));
 }
 
-// First output index in [0, dst_n] whose left (RIGHT: right) corner is >= s.
+// First output index in [0, dst_n] whose left (right: right) corner is >= s.
 // The map ascends: from the inverse map's estimate a few steps find the
 // index; a degenerate map, or an estimate further off, takes the binary search.
-template <typename T, bool FLIP, bool RIGHT>
-__device__ __forceinline__ int first_ge(const UpMap &m, int s) {
+template <typename T, bool FLIP>
+__device__ __forceinline__ int first_ge(const UpMap &m, int s, bool right) {
     auto ge = [&](int d) {
         int a, b;
         coord_idx<T, FLIP>(m, d, a, b);
-        return (RIGHT ? b : a) >= s;
+        return (right ? b : a) >= s;
     };
     const int n = m.dst_n;
-    const T x = (T)(RIGHT ? s - 1 : s);
+    const T x = (T)(right ? s - 1 : s);
     const T est = m.mode == 0 ? (x - (T)m.lo + (T)0.5) * (T)n / (T)m.roi_n - (T)0.5
                               : x * (T)(n - 1) / (T)max(m.src_n - 1, 1);
     if (m.mode != 0 || m.roi_n > 0) {
@@ -297,13 +298,13 @@ upscale_bwd_kernel(UpMap mx, UpMap my, int src_w, int src_h, int rows, const T *
     const int tid = threadIdx.x, dst_w = mx.dst_n;
     const int64_t q = (int64_t)blockIdx.x * kUpThreads + tid;
     const int sy0 = blockIdx.y * rows, sy1 = min(sy0 + rows, src_h) - 1;
-    if (tid == 0) s_rng[0] = first_ge<T, FLIP, true>(my, sy0);
-    else if (tid == 32) s_rng[1] = first_ge<T, FLIP, false>(my, sy1 + 1) - 1;
+    if (tid == 0) s_rng[0] = first_ge<T, FLIP>(my, sy0, true);
+    else if (tid == 32) s_rng[1] = first_ge<T, FLIP>(my, sy1 + 1, false) - 1;
     // this thread's texel column x: output columns [ia, im) have it as their
     // right corner, [im, ib) as their left one
     const int x = (int)min(q / C, (int64_t)src_w - 1), ch = (int)(q % C);
-    const int ia = first_ge<T, FLIP, true>(mx, x), im = first_ge<T, FLIP, false>(mx, x),
-              ib = first_ge<T, FLIP, false>(mx, x + 1);
+    const int ia = first_ge<T, FLIP>(mx, x, true), im = first_ge<T, FLIP>(mx, x, false),
+              ib = first_ge<T, FLIP>(mx, x + 1, false);
     const int n = ib - ia;
     __syncthreads();
     const int j_lo = s_rng[0], j_hi = s_rng[1];
@@ -389,6 +390,178 @@ upscale_bwd_kernel(UpMap mx, UpMap my, int src_w, int src_h, int rows, const T *
     }
 }
 
+// Strong upscaling, more than kBwdColumns output columns a texel: a warp takes a
+// texel column.  Its lanes share the column's output values (contiguous in a
+// row: ten columns of three channels, or 32 of one, at a time), K to a lane,
+// with weights in registers; a lane sums its own share over the rows, and the
+// lanes' sums meet when the walk leaves a texel row.  More than K columns a
+// lane: further walks, which add to the texels.
+// With one thread a value (upscale_bwd_kernel) every value of such a column
+// recomputes its weights in each row, and small sources leave the chip idle.
+// us with a patch staged per block of texels / one thread a value / this:
+// 128^2 x 8 55 / 111 / 19, 512^2 x 8 488 / 221 / 165, 128^2 x 32 1190 / 2137 /
+// 164, 64^2 x 64 5310 / 7700 / 230; a 64^2 crop of 1024^2 to 512^2 60 / 88 / 37.
+// Up to kWideColumns columns and from kWideTexels texels on one thread a value
+// stays ahead: 500^2 x 5 143 / 92 / 98, 1000^2 x 6.5 949 / 468 / 506 (400^2 x 5 97 /
+// 64 / 63, 1000^2 x 7 1081 / 535 / 531).  Bound by issue (a row's sums, 20 of 30
+// lanes at 8x) and the rows' loads.
+constexpr int kWideWarps = 8, kBwdColumns = 8, kWideColumns = 13, kWideTexels = 200000;
+
+template <int C, typename T> __device__ __forceinline__ T sum_slots(T t) {
+    const unsigned FULL = 0xffffffffu;
+    if constexpr (C == 1) {
+#pragma unroll
+        for (int o = 16; o >= 1; o >>= 1) t += __shfl_xor_sync(FULL, t, o);
+        return t;
+    } else {  // ten slots of three lanes; lanes 0..2 have the sums
+        t += __shfl_down_sync(FULL, t, 15);
+        const T fifth = __shfl_down_sync(FULL, t, 12);
+        t += __shfl_down_sync(FULL, t, 6);
+        t += __shfl_down_sync(FULL, t, 3);
+        return t + fifth;
+    }
+}
+
+template <typename T, int C, bool FLIP, int K>
+__global__ void __launch_bounds__(32 * kWideWarps)
+upscale_bwd_wide_kernel(UpMap mx, UpMap my, int src_w, int src_h, int rows,
+                        const T *__restrict__ g, T *__restrict__ gf, T *__restrict__ gfx,
+                        T *__restrict__ gfy, T *__restrict__ gfxy) {
+    constexpr int SLOTS = 32 / C, U = K == 4 ? 2 : 4;  // U: rows loaded together
+    static_assert(C == 1 || C == 3, "channels");
+    __shared__ int2 s_y[kWideWarps][32];
+    __shared__ W4<T> s_cy[kWideWarps][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, dst_w = mx.dst_n;
+    const int x = blockIdx.x * kWideWarps + w;
+    const int sy0 = blockIdx.y * rows, sy1 = min(sy0 + rows, src_h) - 1;
+    // lanes 0, 1: the texel rows' output rows [j_lo, j_hi); lanes 2..4: columns
+    // [ia, im) have the texel as their right corner, [im, ib) as their left
+    const int at = lane == 0 ? sy0 : lane == 1 ? sy1 + 1 : lane < 4 ? x : x + 1;
+    const int found = first_ge<T, FLIP>(lane < 2 ? my : mx, at, lane == 0 || lane == 2);
+    const unsigned ALL = 0xffffffffu;
+    const int j_lo = __shfl_sync(ALL, found, 0), j_hi = __shfl_sync(ALL, found, 1);
+    const int ia = __shfl_sync(ALL, found, 2), im = __shfl_sync(ALL, found, 3),
+              ib = __shfl_sync(ALL, found, 4);
+    const int64_t o_pitch = (int64_t)src_w * C;
+    if (!__syncthreads_or(x < src_w && ia < ib && j_lo < j_hi)) {
+        // the crop has no outputs near these texels
+        const int first = blockIdx.x * kWideWarps, n = min(kWideWarps, src_w - first) * C;
+        for (int i = threadIdx.x; i < n * (sy1 - sy0 + 1); i += blockDim.x) {
+            const int64_t o = (sy0 + i / n) * o_pitch + first * C + i % n;
+            gf[o] = gfx[o] = gfy[o] = gfxy[o] = (T)0;
+        }
+        return;
+    }
+    if (x >= src_w) return;  // (no CTA barriers below)
+    const int slot = lane / C, ch = lane % C;
+    const int64_t pitch = (int64_t)dst_w * C, down = FLIP && my.flip ? -pitch : pitch;
+    const T *g0 = g + (FLIP && my.flip ? (my.dst_n - 1) * pitch : 0) + ch;
+    const int64_t o_at = (int64_t)x * C + ch;
+    int c0 = ia;
+    do {
+        T wv[K], wd[K];
+        const T *gk[K];
+        bool on[K];
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            const int c = c0 + slot + k * SLOTS;
+            on[k] = slot < SLOTS && c < ib;
+            wv[k] = wd[k] = (T)0;
+            gk[k] = g0 + (int64_t)walk_index<FLIP>(mx, on[k] ? c : ia) * C;
+            if (on[k]) {
+                int x0, x1;
+                T cw[4];
+                folded<T, FLIP>(mx, c, x0, x1, cw);
+                wv[k] = c < im ? cw[1] : cw[0];
+                wd[k] = c < im ? cw[3] : cw[2];
+            }
+        }
+        T acc0[4] = {}, acc1[4] = {};
+        int cur = sy0 - 1;  // acc0 belongs to texel row cur, acc1 to the next
+        auto flush = [&]() {
+            if (cur >= sy0 && cur <= sy1) {
+                T t[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) t[k] = sum_slots<C>(acc0[k]);
+                if (slot == 0) {
+                    const int64_t o = cur * o_pitch + o_at;
+                    const bool add = c0 > ia;
+                    gf[o] = add ? gf[o] + t[0] : t[0];
+                    gfx[o] = add ? gfx[o] + t[1] : t[1];
+                    gfy[o] = add ? gfy[o] + t[2] : t[2];
+                    gfxy[o] = add ? gfxy[o] + t[3] : t[3];
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                acc0[k] = acc1[k];
+                acc1[k] = (T)0;
+            }
+            ++cur;
+        };
+        for (int jb = j_lo; jb < j_hi; jb += 32) {
+            const int nj = min(32, j_hi - jb);
+            __syncwarp();
+            if (lane < nj) folded<T, FLIP>(my, jb + lane, s_y[w][lane].x, s_y[w][lane].y, s_cy[w][lane].w);
+            __syncwarp();
+            for (int j = 0; j < nj; j += U) {
+                T v[U][K];
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+#pragma unroll
+                    for (int k = 0; k < K; ++k)
+                        v[u][k] = on[k] && j + u < nj ? gk[k][(jb + j + u) * down] : (T)0;
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    if (j + u >= nj) break;
+                    const int2 y = s_y[w][j + u];
+                    const W4<T> cy = s_cy[w][j + u];
+                    T uv = 0, ud = 0;
+#pragma unroll
+                    for (int k = 0; k < K; ++k) {
+                        uv += v[u][k] * wv[k];
+                        ud += v[u][k] * wd[k];
+                    }
+                    while (cur < y.x) flush();  // y is the same for the whole warp
+                    acc0[0] += uv * cy.w[0];
+                    acc0[1] += ud * cy.w[0];
+                    acc0[2] += uv * cy.w[2];
+                    acc0[3] += ud * cy.w[2];
+                    if (y.y != y.x) {
+                        acc1[0] += uv * cy.w[1];
+                        acc1[1] += ud * cy.w[1];
+                        acc1[2] += uv * cy.w[3];
+                        acc1[3] += ud * cy.w[3];
+                    }
+                }
+            }
+        }
+        while (cur <= sy1) flush();
+        c0 += SLOTS * K;
+    } while (c0 < ib);
+}
+
+// Output columns of a texel away from the borders, at most.
+inline int64_t columns_per_texel(const UpMap &m) {
+    const int64_t out = m.mode == 0 ? m.dst_n : m.dst_n - 1;
+    const int64_t src = m.mode == 0 ? (m.roi_n < 0 ? -(int64_t)m.roi_n : m.roi_n) : m.src_n - 1;
+    return src > 0 ? (2 * out + src - 1) / src : m.dst_n;
+}
+
+template <typename T, int C, bool FLIP>
+void upscale_bwd_wide(UpMap mx, UpMap my, int64_t columns, int src_h, int src_w, const T *g, T *gf,
+                      T *gfx, T *gfy, T *gfxy, cudaStream_t s) {
+    constexpr int SLOTS = 32 / C;
+    int rows = 8;  // texel rows a warp walks: the most that leave 32 warps per SM
+    while (rows > 1 && (int64_t)src_w * ((src_h + rows - 1) / rows) < 148 * 32) rows >>= 1;
+    while ((src_h + rows - 1) / rows > 65535) rows <<= 1;  // (the grid's limit)
+    const dim3 grid((src_w + kWideWarps - 1) / kWideWarps, (src_h + rows - 1) / rows);
+    auto k = columns <= SLOTS       ? upscale_bwd_wide_kernel<T, C, FLIP, 1>
+             : columns <= 2 * SLOTS ? upscale_bwd_wide_kernel<T, C, FLIP, 2>
+                                   : upscale_bwd_wide_kernel<T, C, FLIP, 4>;
+    k<<<grid, 32 * kWideWarps, 0, s>>>(mx, my, src_w, src_h, rows, g, gf, gfx, gfy, gfxy);
+}
+
 // Output (forward) or texel (backward) rows a CTA walks: the most, up to
 // `most`, that leave at least 16 CTAs per SM.
 inline int up_rows(int64_t row_values, int n_rows, int most) {
@@ -425,6 +598,15 @@ int upscale_bwd(int mode, int src_h, int src_w, int dst_h, int dst_w, double x1,
     UpMap my{mode, dst_h, src_h, (int)((T)y2 - (T)y1), (double)(T)y1};
     mx.flip = mode == 0 && mx.roi_n < 0;
     my.flip = mode == 0 && my.roi_n < 0;
+    const int64_t columns = columns_per_texel(mx);
+    if (columns > kBwdColumns &&
+        (columns > kWideColumns || (int64_t)src_h * src_w < kWideTexels)) {
+        auto wide = mx.flip || my.flip ? upscale_bwd_wide<T, C, true> : upscale_bwd_wide<T, C, false>;
+        wide(mx, my, columns, src_h, src_w, (const T *)g, (T *)gf, (T *)gfx, (T *)gfy, (T *)gfxy, s);
+        note_launches(1);
+        LIG_LAUNCH_CHECK();
+        return LIG_OK;
+    }
     const int64_t row = (int64_t)src_w * C;
     const int rows = up_rows(row, src_h, kBwdMaxRows);
     const dim3 grid((unsigned)((row + kUpThreads - 1) / kUpThreads), (src_h + rows - 1) / rows);
