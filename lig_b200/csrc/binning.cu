@@ -9,8 +9,8 @@
 //
 // Ordering (default, LIG_BIN_SCATTER): per-tile counters, their scan, a scatter
 // of every slot into its tile's range and a per-tile sort by Gaussian index —
-// in one CTA for small problems, on shared-memory counters while the tiles fit
-// them, on global atomics beyond (see "scatter binning" and the two sections
+// in one CTA for small problems, on shared-memory counters where many slots meet
+// in few tiles, on global atomics elsewhere (see "scatter binning" and the two sections
 // after it); workspace: two counters per tile, the scan state, the long-tile
 // list and, for the shared counters, their histogram.  Alternative kept for comparison: keys are 32-bit tile
 // ids (the reference's int64 (tile << 32) | depth keys carry depth 0, so only
@@ -863,11 +863,11 @@ tile_sort_long_kernel(BatchGeo geo, const uint32_t *__restrict__ tcount,
 }
 
 // ---------------------------------------------- binning on shared counters
-// While the tile counters fit an SM's shared memory (up to kHistMaxTiles), the
-// global atomics of count and scatter — what those kernels wait for: 6M slots
-// at 2048^2 / 1M Gaussians took 37 and 63 us, at any enumeration cost — become
-// shared-memory atomics.  CTA c of `parts` takes every parts-th 32 Gaussians from
-// the c-th on, so that images with more slots a Gaussian are shared by all:
+// Where many slots meet in few tiles (hist_pays), the global atomics of count and
+// scatter — what those kernels wait for: 6M slots at 2048^2 / 1M Gaussians took
+// 37 and 63 us, at any enumeration cost — become shared-memory atomics.  CTA c
+// of `parts` takes every parts-th 32 Gaussians from the c-th on, so that images
+// with more slots a Gaussian are shared by all:
 //   1. tile_hist_kernel: its slots' tile counts in shared memory, written as
 //      row c of hist [parts][tiles];
 //   2. hist_prefix_kernel: per tile the exclusive prefix over the rows (in
@@ -882,19 +882,34 @@ tile_sort_long_kernel(BatchGeo geo, const uint32_t *__restrict__ tcount,
 // what is left is the enumeration and the scattered 4-byte stores.  Slots past
 // the capacity are dropped by position (outputs are incomplete then, and flagged).
 constexpr int kHistThreads = 1024;
-constexpr int kHistMaxTiles = 48 * 1024;  // 192 KB of counters
-constexpr int kHistTwoTiles = 24 * 1024;  // two CTAs' counters fit an SM up to here
+constexpr int kHistMaxTiles = 24 * 1024;  // 96 KB of counters: two CTAs an SM
 constexpr int kHistMaxParts = 2 * 148;
 
 // Rows of the histogram (CTAs): at least LIG_BIN_HIST_RUN Gaussians each, up to one per
 // SM; two per SM from kHistTwoMinPoints Gaussians on, where the second CTA's
-// warps hide more of the enumeration than the longer prefix costs (eight
-// views, 4M Gaussians / 17k tiles: 174 -> 139 us, on runs; 2048^2 / 1M 88 with
-// one, 87 with two; 16 images of 1.1M Gaussians 57 and 55).
+// warps hide more of the enumeration than the longer prefix costs.  The whole
+// binning with one / two: 16384 tiles, 2M Gaussians 131 / 125 us, 4M 277 / 247 (a
+// tenth of them visible 95 / 89), 1M 81 / 82, 600k 64 / 67; 22500 tiles, 2M 130 /
+// 127, 1M 86 / 90; 4096 tiles, 2M 240 / 227, 1M 88 / 83, 300k 54 / 52.
 constexpr int kHistTwoMinPoints = 2000000;
-inline int hist_parts(int n, size_t tiles) {
-    const bool two = tiles <= kHistTwoTiles && n >= kHistTwoMinPoints;
-    return std::min(std::max(n / LIG_BIN_HIST_RUN, 1), two ? kHistMaxParts : kHistMaxParts / 2);
+inline int hist_parts(int n) {
+    return std::min(std::max(n / LIG_BIN_HIST_RUN, 1),
+                    n >= kHistTwoMinPoints ? kHistMaxParts : kHistMaxParts / 2);
+}
+
+// Whether the shared counters pay.  Their histogram costs parts * tiles words four
+// times over, whatever the slots; each slot's atomic costs less, the more so the
+// fewer the tiles it contends for.  capacity stands for the slots (callers allow
+// for 13 to 25% more than there are).  The whole binning, global / shared, by
+// slots a tile: 16384 tiles: 36 43 / 47 us, 72 62 / 64, 119 82 / 81, 149 90 / 82,
+// 238 141 / 125; 22500: 87 85 / 86, 109 88 / 80; 9216: 21 33 / 35, 64 45 / 43, 132 68 /
+// 55; 4096: 10 27 / 33, 48 35 / 32, 99 40 / 35; 1024: 19 27 / 29, 57 31 / 29; 32900: 124
+// 123 / 119, 178 174 / 183; 47000: 87 113 / 124, 262 333 / 361.  From kHistTwoMinPoints
+// on the shared route also enumerates invisible Gaussians faster: 16384 tiles, a
+// tenth of 2M visible, 50 slots a tile 67 / 67; of 4M, 100 109 / 89.
+inline bool hist_pays(int n, int64_t capacity, int64_t tiles) {
+    const int64_t per_tile = n >= kHistTwoMinPoints ? 50 : std::max<int64_t>(64, tiles / 160);
+    return tiles <= kHistMaxTiles && capacity >= per_tile * tiles;
 }
 
 // f(tile key, sort value) for every slot of the CTA's Gaussians.  Of 32
@@ -1129,7 +1144,7 @@ struct ScatterPlan {
     size_t off_count, off_part, off_long, off_cursor, off_hist, total, total_hist;
 };
 
-inline ScatterPlan make_scatter_plan(int n, int num_tiles) {
+inline ScatterPlan make_scatter_plan(int n, int capacity, int num_tiles) {
     ScatterPlan p{};
     size_t t = (size_t)(num_tiles > 0 ? num_tiles : 1);
     size_t off = 0;
@@ -1139,7 +1154,7 @@ inline ScatterPlan make_scatter_plan(int n, int num_tiles) {
     p.off_cursor = off; off = align_up(off + 4 * t);
     p.total = off;
     p.off_hist = off;
-    p.total_hist = t <= kHistMaxTiles ? align_up(off + 4 * t * hist_parts(n, t)) : off;
+    p.total_hist = hist_pays(n, capacity, (int64_t)t) ? align_up(off + 4 * t * hist_parts(n)) : off;
     return p;
 }
 
@@ -1170,7 +1185,7 @@ int run_bin_scatter(const BatchGeo &geo, const void *xys, const void *ext, const
                     int64_t *isect_sorted, int32_t *status, cudaStream_t s, bool status_clear) {
     const int n = geo.total_points();
     const int T_ = geo.total_tiles();
-    ScatterPlan p = make_scatter_plan(n, T_);
+    ScatterPlan p = make_scatter_plan(n, capacity, T_);
     if (ws_bytes < p.total) return LIG_ERR_WORKSPACE;
     char *base = (char *)ws;
     uint32_t *tcount = (uint32_t *)(base + p.off_count);
@@ -1195,13 +1210,13 @@ int run_bin_scatter(const BatchGeo &geo, const void *xys, const void *ext, const
         LIG_LAUNCH_CHECK();
         return LIG_OK;
     }
-    // shared counters while they fit (the emission-order outputs keep the
-    // slot-order kernels)
-    const bool hist_path = T_ <= kHistMaxTiles && !isect && ws_bytes >= p.total_hist;
+    // (the emission-order outputs keep the slot-order kernels, and a workspace
+    // without the histogram the global counters)
+    const bool hist_path = hist_pays(n, capacity, T_) && !isect && ws_bytes >= p.total_hist;
     if (hist_path) {
         if (!hist_smem_opt_in<T>()) return launch_refused();
         uint32_t *hist = (uint32_t *)(base + p.off_hist);
-        const int parts = hist_parts(n, (size_t)T_);
+        const int parts = hist_parts(n);
         const size_t sm = sizeof(uint32_t) * (size_t)T_;
         const int n_clear = (int)((p.off_long + sizeof(int32_t) - p.off_part) / sizeof(uint32_t));
         tile_hist_kernel<T><<<parts, kHistThreads, sm, s>>>(n, T_, (const T *)xys, (const T *)ext,
@@ -1369,7 +1384,7 @@ extern "C" int lig_cumsum_tiles(int n, const int32_t *counts, int32_t *cum, int3
 }
 
 extern "C" size_t lig_bin_workspace_bytes(int n, int capacity, int num_tiles) {
-    if (LIG_BIN_SCATTER) return make_scatter_plan(n, num_tiles).total_hist;
+    if (LIG_BIN_SCATTER) return make_scatter_plan(n, capacity, num_tiles).total_hist;
     return make_plan(capacity, num_tiles).total;
 }
 
