@@ -87,12 +87,6 @@ __device__ __forceinline__ uint32_t alpha_cut_search() {
 // value) and read by the rasterizer launched after it on the same stream.
 __device__ uint32_t g_alpha_cut;
 
-// A backward's cut: its clamp is the caller's, and below 1/255 every pixel fails
-// (no sigma lies below a cut of 0).
-__device__ __forceinline__ uint32_t backward_cut(float clamp) {
-    return clamp < 1.f / 255.f ? 0u : g_alpha_cut;
-}
-
 // The fused fit step's optimiser scalars (out null: not wanted).
 // skipped_host: pinned host copy of *skipped.
 struct AdamPro {
@@ -1681,7 +1675,7 @@ __device__ __forceinline__ void bwd_tile(const TileCtx &tc, int tile,
     // masks: the warps test the box and ellipse themselves)
     constexpr bool kBulk = kPairs && LIG_RASTER_BWD_BULK;
     constexpr bool kCut = kPairs && !GEN && LIG_RASTER_BWD_CUT;
-    [[maybe_unused]] const uint32_t cut = kCut ? backward_cut(clamp) : 0u;
+    [[maybe_unused]] const uint32_t cut = kCut ? g_alpha_cut : 0u;
     static_assert(RR == 4 || kPairs, "taller regions are walked by the pair form only");
     static_assert(RR == 4 || RR == 8 || RR == 16, "region rows");
     constexpr int kRows = RR;  // pair entries per region: kRows * 4
@@ -2313,7 +2307,7 @@ raster_bwd_ga_kernel(const BatchGeo geo, const int32_t *__restrict__ cum, int *w
     }
     __syncthreads();
     const int n_tiles = geo.total_tiles();
-    const uint32_t cut = OP ? 0u : backward_cut(clamp);
+    const uint32_t cut = OP ? 0u : g_alpha_cut;
     const GaPix *my_pix = s_pix + w * 16;
     uint16_t *my_list = s_list[w];
     for (int tile = next_tile(work, s_slot, true); tile < n_tiles;
@@ -2737,13 +2731,25 @@ int raster_bwd(const BatchGeo &geo, TileWalk walk, const int32_t *ids, const int
     if (rc) return rc;
     const T cl = (T)(clamp > 0 ? clamp : (ga ? 0.999 : 0.99));
     Grads<T> g{(T *)v_xy, (T *)v_abs, (T *)v_con, (T *)v_rgb, (T *)v_op};
+    auto unpack = [&]() {
+        if (n > 0 && lean) unpack_lean_grads_kernel<T><<<(n + 255) / 256, 256, 0, s>>>(n, packed, g);
+        else if (n > 0) unpack_grads_kernel<T><<<(n + 255) / 256, 256, 0, s>>>(n, packed, g);
+        note_launches(n > 0 ? 1 : 0);
+    };
+    // min(clamp, exp(-sigma)) < 1/255 at every pixel: the cleared sums are the
+    // gradients (the walks' alpha cut stands for the rule from 1/255 on)
+    if (!prepacked && cl < (T)1 / (T)255) {
+        unpack();
+        LIG_LAUNCH_CHECK();
+        return LIG_OK;
+    }
     if constexpr (sizeof(T) == 4) {
         if (ga_pairs) {
             rc = raster_bwd_ga(geo, walk, ids, bins, d_total, ws, op || v_op, cot, (const T *)v_dx,
                                (const T *)v_dy, (const T *)v_dxy, cl, packed, s);
             if (rc) return rc;
-            if (n > 0) unpack_grads_kernel<T><<<(n + 255) / 256, 256, 0, s>>>(n, packed, g);
-            note_launches(n > 0 ? 2 : 1);
+            note_launches(1);
+            unpack();
             LIG_LAUNCH_CHECK();
             return LIG_OK;
         }
@@ -2812,14 +2818,8 @@ int raster_bwd(const BatchGeo &geo, TileWalk walk, const int32_t *ids, const int
                             (const Rec<T> *)ws, fin, cot, ga ? (const T *)v_dx : nullptr,
                             ga ? (const T *)v_dy : nullptr, ga ? (const T *)v_dxy : nullptr, cl,
                             packed);
-    if (prepacked) {
-        note_launches(1);
-        LIG_LAUNCH_CHECK();
-        return LIG_OK;
-    }
-    if (n > 0 && lean) unpack_lean_grads_kernel<T><<<(n + 255) / 256, 256, 0, s>>>(n, packed, g);
-    else if (n > 0) unpack_grads_kernel<T><<<(n + 255) / 256, 256, 0, s>>>(n, packed, g);
-    note_launches(n > 0 ? 2 : 1);
+    note_launches(1);
+    if (!prepacked) unpack();
     LIG_LAUNCH_CHECK();
     return LIG_OK;
 }
