@@ -260,11 +260,11 @@ struct SlotWarp {
 };
 
 // Fills in the warp's slots from each lane's Gaussian (ascending over the
-// lanes, lane 0 valid), its count and its first slot.
-template <typename T>
-__device__ __forceinline__ void slot_lanes(int g, bool valid, int cnt, int start,
-                                           const T *__restrict__ xys,
-                                           const T *__restrict__ extents, const BatchGeo &geo,
+// lanes, lane 0 valid), its count, its first slot and its extent (read for a
+// count above 0 only).  LIST: from a CTA's queue; one image search per warp.
+template <typename T, bool LIST>
+__device__ __forceinline__ void slot_lanes(int g, bool valid, int cnt, int start, T ex, T ey,
+                                           const T *__restrict__ xys, const BatchGeo &geo,
                                            int32_t *__restrict__ status, SlotWarp &sw) {
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
@@ -273,15 +273,18 @@ __device__ __forceinline__ void slot_lanes(int g, bool valid, int cnt, int start
     sw.stride = -1;
     sw.base = 0;
     sw.magic = 0;
-    const int g0 = __shfl_sync(FULL, g, 0);
+    [[maybe_unused]] const int g0 = LIST ? __shfl_sync(FULL, g, 0) : 0;
     if (valid) {
-        // the image of the warp's first Gaussian, then this lane's
-        int im = geo.image_of_gauss(g0);
-        while (im + 1 < geo.n_img && g >= geo.g_off[im + 1]) ++im;
+        int im;
+        if constexpr (LIST) {  // the image of the warp's first Gaussian, then this lane's
+            im = geo.image_of_gauss(g0);
+            while (im + 1 < geo.n_img && g >= geo.g_off[im + 1]) ++im;
+        } else {
+            im = geo.image_of_gauss(g);
+        }
         const int tbx = geo.tbx[im];
         sw.base = (uint32_t)geo.tile_off[im];
         if (cnt > 0) {
-            const T ex = extents[2 * g], ey = extents[2 * g + 1];
             if (!(ex <= (T)0 || ey <= (T)0)) {
                 int x0, y0, x1, y1;
                 tile_bbox(xys[2 * g], xys[2 * g + 1], ex, ey, tbx, geo.tby(im), geo.B, x0, y0, x1,
@@ -312,24 +315,24 @@ __device__ __forceinline__ void slot_lanes(int g, bool valid, int cnt, int start
     sw.slot_base = start - sw.excl;
 }
 
-// g0: the warp's first Gaussian; n: end of its range.  False when the warp has
-// no slots (a view's Gaussians are mostly outside it: those cost one load).
+// g0: the warp's first Gaussian; n: end of its range.  Every load is on its way at
+// once, for Gaussians without slots too: leaving early for warps without any, and
+// a neighbour's count by shuffle, made the global-atomic kernels 1 to 5% slower
+// (3000x3400 / 2M 127.3 us of binning, 125.2 so; 8192^2 / 4M, 5% of them visible,
+// 137 and 132).
 template <typename T>
 __device__ __forceinline__ bool slot_warp(int64_t g0, int n, const T *__restrict__ xys,
                                           const T *__restrict__ extents,
                                           const int32_t *__restrict__ cum, const BatchGeo &geo,
                                           int32_t *__restrict__ status, SlotWarp &sw) {
-    const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     sw.g0 = g0;
     if (g0 >= n) return false;
     const int g = (int)(g0 + lane);
     const int last = g < n ? cum[g] : 0;
-    int start = __shfl_up_sync(FULL, last, 1);
-    if (lane == 0) start = g0 > 0 ? cum[g0 - 1] : 0;
-    const int cnt = g < n ? last - start : 0;
-    if (!__any_sync(FULL, cnt != 0)) return false;
-    slot_lanes<T>(g, g < n, cnt, start, xys, extents, geo, status, sw);
+    const int start = g < n && g > 0 ? cum[g - 1] : 0;
+    const T ex = g < n ? extents[2 * g] : (T)0, ey = g < n ? extents[2 * g + 1] : (T)0;
+    slot_lanes<T, false>(g, g < n, g < n ? last - start : 0, start, ex, ey, xys, geo, status, sw);
     return true;
 }
 
@@ -961,8 +964,9 @@ __device__ __forceinline__ void for_each_slot_of_cta(int n, const T *__restrict_
             __syncwarp();
             cnt = valid ? cum[g] - (g > 0 ? cum[g - 1] : 0) : 0;
         }
+        const T ex = cnt > 0 ? ext[2 * g] : (T)0, ey = cnt > 0 ? ext[2 * g + 1] : (T)0;
         SlotWarp sw;
-        slot_lanes<T>(g, valid, cnt, 0, xys, ext, geo, status, sw);
+        slot_lanes<T, true>(g, valid, cnt, 0, ex, ey, xys, geo, status, sw);
         for (int s0 = 0; s0 < sw.total; s0 += 32) {
             int slot;
             uint32_t key, val;
