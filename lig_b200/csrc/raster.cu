@@ -2615,16 +2615,19 @@ int raster_fwd(const BatchGeo &geo, TileWalk walk, const int32_t *ids, const int
         // registers), 1436 with 14; with weight sums and indices eight views
         // 401 with 14, 412 with 16 (spilling); 8x8 regions, 512^2 / 50k 26.8
         // with 9, 27.8 with 8, 27.4 with 10 (767x1023 with opacities 63 / 65 / 69)
-        constexpr int kMinB = P == 4 ? (S ? 14 : 16) : 9;
+        // (double: 6; 512^2 / 20k 48.6 us with 6, 49.4 with 8, 51.6 with 9)
+        constexpr int kMinB = P == 4 ? (S ? 14 : 16) : sizeof(T) == 8 ? 6 : 9;
         return nt <= kMaxT ? raster_fwd_kernel<T, false, P, kMaxT, kMinB, O, F, S>
                            : raster_fwd_kernel<T, false, P, 512, 2, O, F, S>;
     };
     auto pick = [&](auto ppl) -> K {
         using std::false_type;
         using std::true_type;
+        // (double takes the walk with opacities, 1 where there are none: 512^2 / 20k
+        // 45.7 us, 48.6 without the product)
         if (!fused)
-            return op ? sum(ppl, true_type{}, true_type{}, true_type{})
-                      : sum(ppl, false_type{}, true_type{}, true_type{});
+            return op || sizeof(T) == 8 ? sum(ppl, true_type{}, true_type{}, true_type{})
+                                        : sum(ppl, false_type{}, true_type{}, true_type{});
         return op    ? sum(ppl, true_type{}, true_type{}, false_type{})
                : fin ? sum(ppl, false_type{}, true_type{}, false_type{})
                      : sum(ppl, false_type{}, false_type{}, false_type{});
