@@ -2763,8 +2763,10 @@ int raster_bwd(const BatchGeo &geo, TileWalk walk, const int32_t *ids, const int
     // (8x8 tiles fill half of an 8x16 region: 2048^2 / 150k 185 us with 8x8
     // regions, 275 with 8x16)
     const int rr_auto = density <= LIG_RASTER_BWD_R16_MAX_DENSITY && geo.B > 8 ? 16 : 8;
+    // (tiles of up to 4 rows fill a quarter of an 8x8 region: general walk, 4x4 tiles at
+    // 512^2 / 20k 45 us with 8x4 regions, 66 with 8x8)
     const int rr = (LIG_RASTER_BWD_RROWS != 4 && sizeof(T) == 4 && LIG_RASTER_BWD_F2 &&
-                    !ga && large && geo.B <= 16)
+                    !ga && large && geo.B <= 16 && !(gen && geo.B <= 4))
                        ? (LIG_RASTER_BWD_RROWS ? LIG_RASTER_BWD_RROWS : rr_auto)
                        : 4;
     const int nt = 32 * Regions::make(ga ? 2 : (rr == 8 ? 1 : rr == 16 ? 3 : 0), geo.B).count;
