@@ -2590,8 +2590,11 @@ int raster_fwd(const BatchGeo &geo, TileWalk walk, const int32_t *ids, const int
         const int rc = pack<T>(n, xys, con, col, op, ws, ws_bytes, s, !ga, nullptr, 0, ga, ticket);
         if (rc) return rc;
     }
+    // float, gradient-aware: the pair walk on 8x8 regions, but for tiles that fill
+    // those by a half or two thirds where 8x4 regions hold twice or a fifth more
+    // (one pixel a lane / pairs: 4x4 tiles, 512^2 / 20k 36 / 43 us, 20x20 35 / 37)
     if constexpr (sizeof(T) == 4) {
-        if (ga)
+        if (ga && !(geo.B <= 4 || (geo.B > 16 && geo.B <= 20)))
             return raster_fwd_ga(geo, walk, ids, bins, d_total, ws, op != nullptr, (float *)img,
                                  (float *)wsum, (float *)dx, (float *)dy, (float *)dxy, fin, s);
     }
@@ -2633,11 +2636,8 @@ int raster_fwd(const BatchGeo &geo, TileWalk walk, const int32_t *ids, const int
                      : sum(ppl, false_type{}, false_type{}, false_type{});
     };
     K fn;
-    if (ga) {  // (double: float has its own kernel above)
-        if constexpr (sizeof(T) == 4) return LIG_ERR_INVALID;
-        else
-            fn = small ? raster_fwd_kernel<T, true, 1, 256, FM>
-                       : raster_fwd_kernel<T, true, 1, 1024, 1>;
+    if (ga) {
+        fn = small ? raster_fwd_kernel<T, true, 1, 256, FM> : raster_fwd_kernel<T, true, 1, 1024, 1>;
     } else {
         fn = ppl4 ? pick(std::integral_constant<int, 4>{}) : pick(std::integral_constant<int, 2>{});
     }
