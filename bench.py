@@ -56,16 +56,19 @@ FLOP_PER_EVAL = {"lig_raster_fwd": 20.0, "lig_raster_bwd": 40.0, "lig_raster_bwd
                  "lig_raster_fwd_l2": 20.0, "lig_raster_bwd_diff": 40.0,
                  "lig_raster_fwd_l2_batch": 20.0, "lig_raster_fwd_l2_u8_batch": 20.0,
                  "lig_raster_bwd_diff_batch": 40.0, "lig_fit_forward_batch": 20.0,
-                 # (with the projection backward and Adam in the same call)
                  "lig_fit_backward_batch": 40.0}
-# DRAM bytes (read + write) per launch measured by an ncu capture of the same
-# kernels on the 2048^2 / 125k-Gaussian step (same density); traffic grows
-# with pixels and Gaussians, so a size-S launch is scaled by (S / 2048)^2.
+# DRAM bytes (read + write) per launch from one-kernel ncu captures on the
+# 2048^2 / 125k-Gaussian step (same density; profiles/kernels_by_case.md);
+# traffic grows with pixels and Gaussians, so a size-S launch is scaled by
+# (S / 2048)^2.  The fit calls: the rasterizer's capture, and in the backward the
+# update kernel's too.
 DRAM_BYTES_2048 = {"lig_raster_fwd_l2_u8_batch": 21.7e6 + 15.3e6,
                    "lig_raster_bwd_diff_batch": 63.4e6 + 1.0e6,
-                   "lig_fit_forward_batch": 21.7e6 + 15.3e6,
-                   # the rasterizer's bytes and the update kernel's 256 B a Gaussian
-                   "lig_fit_backward_batch": 63.4e6 + 1.0e6 + 256 * 125e3}
+                   "lig_fit_forward_batch": 21.6e6 + 2.1e6,
+                   "lig_fit_backward_batch": 63.4e6 + 0.8e6 + 16.0e6}
+CALL_NOTE = {"lig_fit_forward_batch": "; the call's time includes the loss launch",
+             "lig_fit_backward_batch": "; the call's time includes the update kernel (projection "
+                                       "backward and Adam), whose operations are not counted"}
 CLOCK_FIELDS = ("index,clocks.sm,clocks.max.sm,power.draw,clocks_event_reasons.active,"
                 "clocks_event_reasons.hw_slowdown,clocks_event_reasons.hw_thermal_slowdown,"
                 "clocks_event_reasons.sw_thermal_slowdown,clocks_event_reasons.sw_power_cap")
@@ -406,11 +409,12 @@ def run_lig(args, rank, world, local_rank):
             traffic = DRAM_BYTES_2048[dom] * (size / 2048) ** 2
         roof = {"bound": "fp32", "achieved": achieved, "peak": fp32_peak / 1e12,
                 "unit": "TFLOP/s", "frac": achieved * 1e12 / fp32_peak, "traffic": traffic,
-                "traffic_note": "ncu dram bytes of the 2048^2 capture x (size/2048)^2",
+                "traffic_note": "ncu dram bytes of the 2048^2 captures x (size/2048)^2",
                 "kernel": dom, "per_launch_units": evals,
                 "note": "algorithmic = reference Gaussian-pixel evaluations x FLOP/eval "
                         f"({FLOP_PER_EVAL[dom]:.0f}); peak = FP32 FMA probe measured on this "
-                        "device (a SIMT-bound kernel: neither HBM nor tensor cores bound it)"}
+                        "device (a SIMT-bound kernel: neither HBM nor tensor cores bound it)"
+                        + CALL_NOTE.get(dom, "")}
     else:
         roof = {"bound": "hbm", "achieved": None, "peak": None, "unit": "GB/s", "frac": None,
                 "traffic": None, "kernel": dom}
