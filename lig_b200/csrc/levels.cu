@@ -27,6 +27,10 @@ constexpr int kLevelThreads = 256;
 // Elementwise passes: 6 CTAs per SM, 4 vectors in flight per thread (4095x4093:
 // minmax / normalise 75 / 84 us; 8 CTAs 75 / 87, 4 79 / 95, 2 in flight 74 / 99).
 constexpr int kLevelCtas = 6, kLevelUnroll = 4;
+// One value at a time (misaligned arrays): 16 CTAs from kScalarMany values on
+// (normalise, 6 / 16: 1023^2 6.0 / 6.9 us, 2048^2 37 / 32, 4095^2 150 / 125).
+constexpr int kScalarCtas = 16;
+constexpr int64_t kScalarMany = 6000000;
 
 __device__ __forceinline__ float atomic_min_f(float *a, float v) {
     // order-preserving int mapping of finite floats
@@ -255,9 +259,9 @@ compose_kernel(int rows, int ph, int pw, const float *__restrict__ prev, int H, 
     if (k0 < nr) walk(k0, std::false_type{});
 }
 
-inline int level_blocks(int64_t n) {
+inline int level_blocks(int64_t n, int ctas) {
     int64_t b = (n + kLevelThreads - 1) / kLevelThreads;
-    const int64_t cap = 148 * kLevelCtas;
+    const int64_t cap = 148 * ctas;
     return (int)(b < 1 ? 1 : (b > cap ? cap : b));
 }
 
@@ -272,7 +276,8 @@ extern "C" int lig_level_residual(int64_t n, const float *gt, const float *up, f
     minmax_init_kernel<<<1, 1, 0, s>>>(minmax);
     const bool vec = ((reinterpret_cast<uintptr_t>(gt) | reinterpret_cast<uintptr_t>(up) |
                        reinterpret_cast<uintptr_t>(out)) & 15) == 0;
-    const int blocks = level_blocks(vec ? (n + 3) / 4 : n);
+    const int blocks = level_blocks(vec ? (n + 3) / 4 : n,
+                                    vec || n < kScalarMany ? kLevelCtas : kScalarCtas);
     auto minmax_k = vec ? resid_minmax_kernel<true> : resid_minmax_kernel<false>;
     auto norm_k = vec ? resid_normalise_kernel<true> : resid_normalise_kernel<false>;
     minmax_k<<<blocks, kLevelThreads, 0, s>>>(n, gt, up, minmax);
