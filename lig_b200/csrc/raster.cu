@@ -2722,15 +2722,18 @@ int raster_bwd(const BatchGeo &geo, TileWalk walk, const int32_t *ids, const int
     // float gradient-aware: 16x16 and 8x8 tiles, whose reference warps are
     // blocks of pixels
     const bool ga_pairs = ga && sizeof(T) == 4 && cot.v_img && (geo.B == 16 || geo.B == 8);
-    // float sum backward with opacities or a wsum cotangent: the pair walk too
-    const bool gen = !ga && !lean && !lean_abs && sizeof(T) == 4;
+    // float sum backward with opacities or a wsum cotangent: the pair walk too, but for
+    // 2x2 tiles, which fill an eighth of its 8x4 regions (300x333 / 8k: 49 us a call,
+    // 46 with the scalar walk, which skips the pixels outside; 3x3 33, 38 scalar)
+    const bool general = !ga && !lean && !lean_abs;
+    const bool gen = general && sizeof(T) == 4 && geo.B > 2;
     // records (halved conic for the pair walks), and the packed gradients cleared
     // in the same pass; prepacked (lean): the forward left both in ws, and the
     // gradients stay packed
     int rc = LIG_OK;
     if (!prepacked)
-        rc = pack<T>(n, xys, con, col, op, ws, goff, s, !ga && sizeof(T) == 4, packed, stride,
-                     ga_pairs || gen);
+        rc = pack<T>(n, xys, con, col, op, ws, goff, s,
+                     sizeof(T) == 4 && (lean || lean_abs || gen), packed, stride, ga_pairs || gen);
     if (rc) return rc;
     const T cl = (T)(clamp > 0 ? clamp : (ga ? 0.999 : 0.99));
     Grads<T> g{(T *)v_xy, (T *)v_abs, (T *)v_con, (T *)v_rgb, (T *)v_op};
@@ -2766,7 +2769,7 @@ int raster_bwd(const BatchGeo &geo, TileWalk walk, const int32_t *ids, const int
     // (tiles of up to 4 rows fill a quarter of an 8x8 region: general walk, 4x4 tiles at
     // 512^2 / 20k 45 us with 8x4 regions, 66 with 8x8)
     const int rr = (LIG_RASTER_BWD_RROWS != 4 && sizeof(T) == 4 && LIG_RASTER_BWD_F2 &&
-                    !ga && large && geo.B <= 16 && !(gen && geo.B <= 4))
+                    !ga && large && geo.B <= 16 && !(general && geo.B <= 4))
                        ? (LIG_RASTER_BWD_RROWS ? LIG_RASTER_BWD_RROWS : rr_auto)
                        : 4;
     const int nt = 32 * Regions::make(ga ? 2 : (rr == 8 ? 1 : rr == 16 ? 3 : 0), geo.B).count;
@@ -2793,6 +2796,8 @@ int raster_bwd(const BatchGeo &geo, TileWalk walk, const int32_t *ids, const int
             fn = !small  ? raster_bwd_kernel<T, false, true, 1024, 1, true>
                  : large ? raster_bwd_kernel<T, false, true, 256, kMinL, true>
                          : raster_bwd_kernel<T, false, true, 256, kMin, true>;
+        else if (!gen)
+            fn = raster_bwd_kernel<T, false, false, 256, LIG_RASTER_BWD_MINB>;
         else
             fn = !small  ? raster_bwd_kernel<T, false, true, 1024, 1, true, 4, true>
                          : raster_bwd_kernel<T, false, true, 256, LIG_RASTER_GEN_MINB, true, 4, true>;
