@@ -5,8 +5,8 @@
 // At small images these paths are bound by the host: in Python each entry
 // point cost 20-40 us of allocations, pointer conversions and stream lookups
 // beside its launches.  Project + rasterize at 64x80 / 400 Gaussians: 164 us
-// from Python, 83 from here (35 us of device work in 14 launches); a training
-// iteration at 512^2 / 50k: 555 -> 347.  Every function runs without the GIL;
+// from Python in 14 launches, 83 from here; 60 now in 6 launches (25 us of device
+// work).  A training iteration at 512^2 / 50k: 555 -> 347.  Every function runs without the GIL;
 // nothing is kept between calls.
 #include <ATen/ATen.h>
 #include <ATen/cuda/CUDAEvent.h>

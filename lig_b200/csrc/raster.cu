@@ -864,10 +864,11 @@ __device__ __forceinline__ void fwd_tile(const TileCtx &tc, int tile, const int3
 #endif
 // Region rows by density (Gaussians per pixel): taller regions save per-pair
 // work, but evaluate more pixels a pair cannot reach, which costs more when
-// the tile lists are long.  Measured (lean backward, 16x16 tiles): at 0.03
-// Gaussians per pixel (8192^2, 2M) 8x16 2.05 ms, 8x8 2.18, 8x4 2.79; at 0.06
-// (4096^2, 1M) 8x16 0.99, 8x8 0.89; at 0.12 (4096^2, 2M) 1.86 / 1.63 / 1.67;
-// at 0.24 (2048^2, 1M) 0.94 / 0.79 / 0.81.  The crossover is near 0.04.
+// the tile lists are long.  Whole calls on 16x16 tiles with 8x16 / 8x8 regions, us:
+// lean walk at 0.03 Gaussians per pixel (8192^2, 2M) 1940 / 2092, at 0.04 (4096^2)
+// 643 / 613, 0.06 937 / 818, 0.24 (2048^2, 1M) 896 / 722; general walk 2551 / 3013,
+// 816 / 922, 1225 / 1169, 1163 / 940.  The crossover is near 0.036 for the lean walks
+// and 0.046 for the general one; the line lies between.
 #ifndef LIG_RASTER_BWD_R16_MAX_DENSITY
 #define LIG_RASTER_BWD_R16_MAX_DENSITY 0.04
 #endif
@@ -992,8 +993,8 @@ raster_views_kernel(const BatchGeo geo, const int32_t *__restrict__ cum,
 // the test adds zeros, so the walk has no branches.  A chunk with a record
 // that could make those zeros NaN (no culling data under TAME packing) takes a
 // scalar walk that skips failing pixels.
-// Bound by the math pipes and issue together (70% of the issue slots; a packed
-// operation takes two cycles of the FMA pipe, so packing saves issue slots
+// Bound by the FMA pipe and issue together (66% of the cycles and of the slots; a
+// packed operation takes two cycles of the FMA pipe, so packing saves issue slots
 // only).  2048^2 / 1M Gaussians: 973 us, against 1265 with one pixel a lane in
 // 8x4 regions (scalar, skipping); 8x16 regions with two pairs a lane: 1120 (fewer operations a
 // pixel, more pixels out of reach).
@@ -2121,8 +2122,8 @@ raster_bwd_kernel(const BatchGeo geo, const int32_t *__restrict__ cum, int *work
 // come from row sums.
 // Entries after a pixel's final index are not cut off: they fail the alpha
 // test here exactly as they did in the forward.
-// Bound by the FMA pipe (a packed operation takes two cycles of it; 70% busy at
-// 61% of the issue slots).  2047x1535 / 190k Gaussians: 518 us, against 1171
+// Bound by the FMA pipe (a packed operation takes two cycles of it; 62% busy at
+// 61% of the issue slots) and the latency of its dependent chains (36% of the warps).  2047x1535 / 190k Gaussians: 518 us, against 1171
 // for the scalar walk over the expanded formulas; 512^2 / 50k with opacities:
 // 67 against 131.
 struct alignas(16) GaPix {  // pixels (row, c) and (row, c + W/2)
