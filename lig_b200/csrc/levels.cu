@@ -190,11 +190,13 @@ compose_flat_kernel(int64_t n, const float *__restrict__ prev, const float *__re
 // 4095x4093 from 2047x2046 (69 us of traffic): 92 us, against 115 with one
 // pixel a thread and a 64-bit division each, 131 with the conversions per value
 // and 146 with four flat values a thread.  Issue-bound (75% of the slots).
-// Images of up to kNarrowValues values a row: a CTA is CW = 32 columns (16 or 4,
-// if those hold a row) by several groups of sixteen rows, so that few threads
-// lie past the row's end (100000x5: 9.0 us with 32, 15 with 256).
+// Images of up to kNarrowValues values a row: a CTA is a whole row by as many
+// groups of sixteen rows as it has threads for, so that few threads idle; the
+// groups' rows alternate, so that a warp's loads lie side by side: 1000000x1 8.8 us
+// and 100000x5 5.6 (8.4 and 5.5 with one pixel a thread, 82 and 15 with CTAs of 256
+// columns).
 constexpr int kComposeRows = 16, kComposeBatch = 4;  // 32 rows 95 us, batches of 2 / 8 98 / 104
-constexpr int kNarrowValues = 128;
+constexpr int kNarrowValues = 128, kNarrowGroups = kLevelThreads / 3;
 // Small images: groups of four rows where sixteen would leave fewer than two CTAs
 // per SM (512^2 5.3 us instead of 6.2; 767x1023, four CTAs, 7.1 with sixteen and 8.3).
 constexpr int kComposeFewRows = 4, kComposeFewCtas = 2;
@@ -204,22 +206,23 @@ template <typename Off> struct RowTap {
     float ly0, ly1;  // their weights
 };
 
-template <typename Off, int CW>
+// NARROW: cw columns (a whole row) by kLevelThreads / cw groups, else one group.
+template <typename Off, bool NARROW>
 __global__ void __launch_bounds__(kLevelThreads)
-compose_kernel(int rows, int ph, int pw, const float *__restrict__ prev, int H, int W,
+compose_kernel(int rows, int cw, int ph, int pw, const float *__restrict__ prev, int H, int W,
                const float *__restrict__ render, const float *__restrict__ mm, float lo_h,
                float hi_h, int clamp_render, int clamp_out, float *__restrict__ out) {
-    constexpr int kGroups = kLevelThreads / CW;
-    __shared__ RowTap<Off> s_rows[kGroups][kComposeRows];
-    const int tx = threadIdx.x % CW, ty = threadIdx.x / CW;
-    RowTap<Off> *s_row = s_rows[ty];
+    __shared__ RowTap<Off> s_row[kComposeRows * (NARROW ? kNarrowGroups : 1)];
+    const int tid = threadIdx.x, groups = NARROW ? kLevelThreads / cw : 1;
+    const int ty = NARROW ? tid / cw : 0, tx = NARROW ? tid - ty * cw : tid;
     const int64_t pitch = 3 * (int64_t)W;
-    const Off q = (Off)blockIdx.x * CW + tx;
+    const Off q = NARROW ? (Off)tx : (Off)blockIdx.x * kLevelThreads + tx;
     // (the row blocks run over y and z of the grid: one dimension holds 65535)
-    const int64_t rb = (int64_t)blockIdx.z * gridDim.y + blockIdx.y;
-    if (rb * (rows * kGroups) >= H) return;
-    const int64_t first = rb * (rows * kGroups) + ty * rows;
-    const int r0 = (int)(first < H ? first : H), nr = min(rows, H - r0);
+    const int64_t rb = ((int64_t)blockIdx.z * gridDim.y + blockIdx.y) * (rows * groups);
+    if (rb >= H) return;
+    // the CTA's rows r0 .. r0 + n_rows - 1; group ty takes every groups-th
+    const int r0 = (int)rb, n_rows = min(rows * groups, H - r0);
+    const int nr = (n_rows - ty + groups - 1) / groups;
     // the half-pixel source index and weights written as the bilinear
     // definition states them (src = s (d + 0.5) - 0.5, negative -> 0;
     // lambda1 = src - floor, lambda0 = 1 - lambda1), so that the
@@ -233,9 +236,9 @@ compose_kernel(int rows, int ph, int pw, const float *__restrict__ prev, int H, 
         const Off p = (Off)pw * 12u;
         s_row[k] = RowTap<Off>{(Off)y0 * p, (Off)y1 * p, 1.f - ly1, ly1};
     };
-    if (tx < nr) tap(tx);
-    if constexpr (CW < kComposeRows)
-        for (int k = tx + CW; k < nr; k += CW) tap(k);
+    if (tid < n_rows) tap(tid);
+    if constexpr (NARROW)
+        for (int k = tid + kLevelThreads; k < n_rows; k += kLevelThreads) tap(k);
     const ComposeOp op(mm, lo_h, hi_h, clamp_render, clamp_out);
     const Off x = q / 3u, c = q - 3u * x;
     const float sw = __fdiv_rn((float)pw, (float)W);
@@ -245,14 +248,14 @@ compose_kernel(int rows, int ph, int pw, const float *__restrict__ prev, int H, 
     const float lx1 = rx - (float)x0, lx0 = 1.f - lx1;
     const Off oa = ((Off)3 * (Off)x0 + c) * 4u, ob = oa + (x0 < pw - 1 ? 12u : 0u);
     __syncthreads();
-    if (q >= pitch) return;
+    if (NARROW ? ty >= groups : q >= pitch) return;
     auto at = [](const float *p, Off o) {
         return *reinterpret_cast<const float *>(reinterpret_cast<const char *>(p) + o);
     };
     // this CTA's rows: one base per array, offsets in bytes
-    const float *rend = render + r0 * pitch;
-    float *dst = out + r0 * pitch;
-    const Off row = (Off)(pitch * 4);
+    const float *rend = render + (r0 + ty) * pitch;
+    float *dst = out + (r0 + ty) * pitch;
+    const Off row = (Off)(pitch * 4 * groups);
     auto walk = [&](int k0, auto full_tag) {  // FULL: the whole batch lies inside
         constexpr bool FULL = decltype(full_tag)::value;
         float v[kComposeBatch], t[kComposeBatch][4];
@@ -261,7 +264,7 @@ compose_kernel(int rows, int ph, int pw, const float *__restrict__ prev, int H, 
             if (!FULL && k0 + k >= nr) break;
             const Off o = (Off)(k0 + k) * row + (Off)q * 4u;
             v[k] = at(rend, o);
-            const RowTap<Off> r = s_row[k0 + k];
+            const RowTap<Off> r = s_row[(k0 + k) * groups + ty];
             t[k][0] = at(prev, r.a + oa);
             t[k][1] = at(prev, r.a + ob);
             t[k][2] = at(prev, r.b + oa);
@@ -270,7 +273,8 @@ compose_kernel(int rows, int ph, int pw, const float *__restrict__ prev, int H, 
 #pragma unroll
         for (int k = 0; k < kComposeBatch; ++k) {
             if (!FULL && k0 + k >= nr) break;
-            const float ly0 = s_row[k0 + k].ly0, ly1 = s_row[k0 + k].ly1;
+            const RowTap<Off> &rw = s_row[(k0 + k) * groups + ty];
+            const float ly0 = rw.ly0, ly1 = rw.ly1;
             const float base =
                 ly0 * (lx0 * t[k][0] + lx1 * t[k][1]) + ly1 * (lx0 * t[k][2] + lx1 * t[k][3]);
             *reinterpret_cast<float *>(reinterpret_cast<char *>(dst) + (Off)(k0 + k) * row +
@@ -329,9 +333,8 @@ extern "C" int lig_level_compose(int prev_h, int prev_w, const float *prev, int 
         return LIG_OK;
     }
     const bool narrow = 3 * (int64_t)W <= kNarrowValues;
-    const int cw = !narrow ? kLevelThreads : W <= 1 ? 4 : W <= 5 ? 16 : 32;
-    const int64_t cols = (3 * (int64_t)W + cw - 1) / cw;
-    const int groups = kLevelThreads / cw;
+    const int cw = narrow ? 3 * W : kLevelThreads, groups = kLevelThreads / cw;
+    const int64_t cols = narrow ? 1 : (3 * (int64_t)W + cw - 1) / cw;
     const int rows = cols * ((H + (int64_t)groups * kComposeRows - 1) / (groups * kComposeRows)) <
                              148 * kComposeFewCtas ? kComposeFewRows : kComposeRows;
     const int64_t row_blocks = ((int64_t)H + rows * groups - 1) / (rows * groups);
@@ -340,17 +343,9 @@ extern "C" int lig_level_compose(int prev_h, int prev_w, const float *prev, int 
     // 32-bit byte offsets while a CTA's rows, and prev, lie within 4 GiB
     const bool small = 12 * (int64_t)W * kComposeRows <= 0xffffffffll &&
                        12 * (int64_t)prev_h * prev_w <= 0xffffffffll;
-    auto pick = [](auto off, auto w) {
-        return compose_kernel<decltype(off), decltype(w)::value>;
-    };
-    auto width = [&](auto off) {
-        return cw == 4    ? pick(off, std::integral_constant<int, 4>{})
-               : cw == 16 ? pick(off, std::integral_constant<int, 16>{})
-               : cw == 32 ? pick(off, std::integral_constant<int, 32>{})
-                          : pick(off, std::integral_constant<int, kLevelThreads>{});
-    };
-    auto k = small ? width(uint32_t{}) : width(uint64_t{});
-    k<<<grid, kLevelThreads, 0, s>>>(rows, prev_h, prev_w, prev, H, W, render, minmax,
+    auto k = small ? (narrow ? compose_kernel<uint32_t, true> : compose_kernel<uint32_t, false>)
+                   : (narrow ? compose_kernel<uint64_t, true> : compose_kernel<uint64_t, false>);
+    k<<<grid, kLevelThreads, 0, s>>>(rows, cw, prev_h, prev_w, prev, H, W, render, minmax,
                                      (float)store_min, (float)store_max, clamp_render, clamp_out,
                                      out);
     note_launches(1);
